@@ -13,6 +13,7 @@
 #include "context.hpp"
 #include "dugma.h"
 #include "dugma_mex.hpp"
+#include "spatial.cuh"
 
 namespace dugma {
 
@@ -311,8 +312,9 @@ static int mapped_fetch(Context& c, int nv, double* dst)
 
 // sigma at a pose without copies or memsets: the pose goes to the search prologue by value (it
 // also zeroes the error word), and the result with the error word behind it comes back through
-// the mapped pinned staging, or by copies when it is not mapped.  o = (exact, quantised) sigma.
-static int sigma_call(Context& c, const double* R, const double* t, double o[2])
+// the mapped pinned staging, or by copies when it is not mapped.  o = (exact when asked for, quantised)
+// sigma.
+static int sigma_call(Context& c, const double* R, const double* t, bool exact, double o[2])
 {
     pack_pose(c, R, t, 1.0, c.host);
     PoseBlock pb;
@@ -320,6 +322,7 @@ static int sigma_call(Context& c, const double* R, const double* t, double o[2])
     SigmaOpts so;
     so.pose_value = &pb;
     so.reset_err = true;
+    so.exact = exact;
     so.host_out = c.host_dev ? c.host_dev + 64 : nullptr;
     DUGMA_RET(launch_sigma(c, c.pose, c.out, c.stream, 0, -1, so));
     if (!so.host_out) return fetch(c, c.out, 2, o);
@@ -434,6 +437,13 @@ int dugma_init(const double* X, const double* X_C, const double* Y, const double
     // One device arena holds every per-context buffer.  Its scratch region first receives
     // the FP64 host inputs during init and afterwards the kernels' partial sums.
     const int NS = D == 3 ? 6 : 3;
+    // grid of the spatial order: up to ~100K points 4 bits per axis in 3D, 6 in 2D (4096 cells, one step of
+    // the scan; the splits refine it), finer beyond
+    const bool fine = std::max(N, M) > 131072;
+    c->cell_bits = D == 3 ? (fine ? 5 : 4) : (fine ? 7 : 6);
+    c->cells = 1 << (D * c->cell_bits);
+    const int nxt = (N + kTile - 1) / kTile, nyt = (M + kTile - 1) / kTile;
+    const int nxs = (nxt + kSuper - 1) / kSuper, nys = (nyt + kSuper - 1) / kSuper;
     const size_t staging = sizeof(double) * ((size_t)N * D * (D + 1) + (size_t)M * D * (D + 1));
     const size_t scratch_bytes = std::max(staging, (size_t)4 << 20);
     struct Slot {
@@ -451,7 +461,16 @@ int dugma_init(const double* X, const double* X_C, const double* Y, const double
         {(void**)&c->yp32, sizeof(float4) * c->M_pad},  {(void**)&c->dmin, sizeof(float) * N},
         {(void**)&c->pose, sizeof(double) * kPoseDoubles * 2}, {(void**)&c->out, sizeof(double) * 64},
         {(void**)&c->poses, sizeof(double) * kPoseDoubles * kMaxPoses},
-        {(void**)&c->err, sizeof(int) * 4},             {(void**)&c->counter, sizeof(int) * 8},
+        {(void**)&c->err, sizeof(int) * 4},
+        {(void**)&c->counter, sizeof(int) * (kCounters + 2 * (size_t)c->cells)},
+        {(void**)&c->init_L, sizeof(float) * ((size_t)N + M)},
+        {(void**)&c->init_part, sizeof(double) * 2 * kInitParts * 5},
+        {(void**)&c->init_place, sizeof(int2) * ((size_t)N + M)},
+        {(void**)&c->xpt, sizeof(SortedPoint) * N},     {(void**)&c->ypt, sizeof(SortedPoint) * M},
+        {(void**)&c->xtile, sizeof(Bound) * nxt},       {(void**)&c->ytile, sizeof(Bound) * nyt},
+        {(void**)&c->xsub, sizeof(Bound) * 4 * nxt},    {(void**)&c->ysub, sizeof(Bound) * 4 * nyt},
+        {(void**)&c->xsuper, sizeof(Bound) * nxs},      {(void**)&c->ysuper, sizeof(Bound) * nys},
+        {(void**)&c->ysphere, sizeof(float4) * (nyt + nys)},
         {(void**)&c->mom, sizeof(double) * kMomSlots},        {(void**)&c->arena_scratch, scratch_bytes},
     };
     auto up = [](size_t v) { return (v + 255) / 256 * 256; };
@@ -464,6 +483,7 @@ int dugma_init(const double* X, const double* X_C, const double* Y, const double
         *s.p = static_cast<char*>(c->arena) + off;
         off += up(s.bytes);
     }
+    c->hist = c->counter + kCounters;
     c->scratch = c->arena_scratch;
     c->scratch_bytes = c->arena_scratch_bytes = scratch_bytes;
     c->host = pinned_acquire();
@@ -519,7 +539,7 @@ int dugma_update_sig(float* Ptr[6], const double* R, const double* t, const doub
     GET_CTX(c, Ptr);
     if (!check_sizes(*c, N, M, D)) return set_error(DUGMA_ERR_ARG, "update_sig: N, M, D differ from init");
     double o[2];
-    DUGMA_RET(sigma_call(*c, R, t, o));
+    DUGMA_RET(sigma_call(*c, R, t, false, o));
     sig[0] = (float)o[1];
     return DUGMA_OK;
 }
@@ -529,7 +549,7 @@ int dugma_sigma(float* Ptr[6], const double* R, const double* t, double* sig)
     if (!R || !t || !sig) return set_error(DUGMA_ERR_ARG, "sigma: null argument");
     GET_CTX(c, Ptr);
     double o[2];
-    DUGMA_RET(sigma_call(*c, R, t, o));
+    DUGMA_RET(sigma_call(*c, R, t, true, o));
     *sig = o[0];
     return DUGMA_OK;
 }
@@ -839,6 +859,7 @@ int dugma_set_shape(float* Ptr[6], int what, int ipt, int nt, int tj, int pack)
     for (const KernelShape& s : cand)
         if (s.same(want)) {
             shape_slot(*c, what) = s;
+            if (what == 2) c->nn_pinned = true;   // an all-pairs shape asked for: no pruned search
             return DUGMA_OK;
         }
     return set_error(DUGMA_ERR_ARG, "set_shape: (%d, %d, %d, %d) is not a compiled shape", ipt, nt, tj, pack);
@@ -980,6 +1001,7 @@ static int em_enqueue(Context& c, cudaStream_t s)
     SigmaOpts so;
     so.pose_src = c.host_dev;
     so.reset_err = true;
+    so.exact = false;
     so.pose_sig = c.pose;
     so.host_out = c.host_dev ? c.host_dev + 64 : nullptr;
     DUGMA_RET(launch_sigma(c, c.pose, c.out, s, 0, -1, so));

@@ -49,6 +49,14 @@ struct KernelShape {
     bool same(const KernelShape& o) const { return ipt == o.ipt && nt == o.nt && tj == o.tj && pack == o.pack; }
 };
 
+constexpr int kCounters = 8;      // ints of Context::counter
+constexpr int kInitParts = 256;   // most blocks per cloud of init's statistics
+constexpr int kInitOut = 10;      // scalars init hands to the host: log2 of the largest weights, the CONV
+                                  // scale, det <= 0 and indefinite counts, mean traces, mean squared radii
+
+struct SortedPoint;
+struct Bound;
+
 struct Context {
     int N = 0, M = 0, D = 0, dev = 0;
     int N_pad = 0, M_pad = 0;
@@ -63,6 +71,8 @@ struct Context {
     int x_indef = 0;                          // weighted sources whose sym(Sigma_x^-1) is not positive definite
     int y_indef = 0;                          // weighted targets whose sym(Sigma_y^-1) is not positive definite
     double Lmax_x = 0, Lmax_y = 0;
+    double trace_x = 0, trace_y = 0;          // mean covariance trace
+    double rho2_x = 0, rho2_y = 0;            // mean squared distance to the cloud's mean
     double cscale = 1.0;                      // CONV covariances are stored divided by this
     // per-evaluation records
     YRec* yrec = nullptr;
@@ -77,7 +87,19 @@ struct Context {
     double* poses = nullptr;                  // kMaxPoses x kPoseDoubles
     double* out = nullptr;                    // 64 doubles of results
     int* err = nullptr;                       // device error word
-    int* counter = nullptr;                   // work-queue counters (8)
+    int* counter = nullptr;                   // work-queue counters (kCounters: [0] items,
+                                              // [1] blocks done, [2, 3] sigma's integer sum), then hist
+    // the clouds in spatial order (spatial.cuh), made by init
+    int cell_bits = 0, cells = 0;             // grid bits per axis, cells
+    int* hist = nullptr;                      // 2 x cells
+    float* init_L = nullptr;                  // N + M (during init)
+    double* init_part = nullptr;              // 2 x kInitParts x 5 (during init)
+    int2* init_place = nullptr;               // N + M (during init)
+    SortedPoint *xpt = nullptr, *ypt = nullptr;
+    Bound *xtile = nullptr, *ytile = nullptr, *xsub = nullptr, *ysub = nullptr;
+    Bound *xsuper = nullptr, *ysuper = nullptr;
+    float4* ysphere = nullptr;                // the target tiles' and super tiles' spheres at a pose
+    bool nn_pinned = false;                   // a nearest-neighbour kernel shape was pinned: no pruning
     double* dedx = nullptr;                   // dE/dx rows (allocated on first request)
     double* mom = nullptr;                    // surrogate moments (512 doubles)
     double* mom_part = nullptr;               // per-block moment partials (with the 128-byte records)
@@ -155,8 +177,9 @@ int launch_pair_variant(Context& c, KernelFn fn, const KernelShape& sh, const vo
 // Nearest-neighbour prologue: only the target records of the search (c.yp32), y' = R y + t as the
 // full prologue rounds it.  The pose is *pv when given (then also written to pose_dev), else read
 // from pose_dev; reset_counter / reset_err (optional) are zeroed for the kernels that follow.
+// sorted: the records in spatial order with the targets' indices, and the tiles' spheres (c.ysphere).
 int launch_nn_prologue(Context& c, double* pose_dev, cudaStream_t s, const PoseBlock* pv, int* reset_counter,
-                       int* reset_err);
+                       int* reset_err, bool sorted);
 // One small kernel: the pose block from src (device-visible memory, e.g. the mapped pinned staging
 // a captured graph reads at each launch) into pose_dev, and the error word zeroed if reset_err.
 int launch_pose_in(Context& c, const double* src, double* pose_dev, cudaStream_t s, bool reset_err);
@@ -199,6 +222,7 @@ struct SigmaOpts {
     bool reset_err = false;                  // the first kernel zeroes the device error word
     double* host_out = nullptr;              // mapped pinned memory that also receives out_dev[0..1] and,
                                              // at [2], the error word
+    bool exact = true;                       // false: only out_dev[1] is wanted (the search sums it itself)
     double* pose_sig = nullptr;              // a device pose block whose sig receives out_dev[1]
 };
 // sigma: out_dev[0] = exact FP64 sigma, out_dev[1] = quantised (reference) sigma.  For a source

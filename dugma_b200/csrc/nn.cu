@@ -8,21 +8,18 @@
 // Target records hold two targets each, coordinates negated (d = x + (-y') is the same FP32
 // value), interleaved so that the search kernels evaluate both with f32x2 operations.
 //   the k smallest (d2, j) in lexicographic order are kept in registers (ties -> lowest j)
-// Targets are streamed by bulk copy like the energy kernels; target chunks are merged in
-// index order afterwards, so the result is exact and deterministic.  sigma is then
+// All rows: the pruned search in spatial order (nn_prune_kernel).  Row ranges and pinned shapes: all
+// pairs, the targets streamed by bulk copy like the energy kernels and target chunks merged in
+// index order afterwards.  Either is exact and deterministic.  sigma is then
 //   exact:      sum_i d2min_i / (D N) in FP64
 //   quantised:  sum_i rn_u32(fl32(d2min_i / D) * 1e6) / 1e6 / N   (the reference's value)
 #include <cmath>
 
 #include "context.hpp"
 #include "pairs.cuh"
+#include "spatial.cuh"
 
 namespace dugma {
-
-// two nearest-neighbour targets (see the prologue): a = (-y0, -y0', -y1, -y1'), b = (-y2, -y2', 0, 0)
-struct __align__(16) NNRec2 {
-    float4 a, b;
-};
 
 template <int D, int IPT_, int K>
 struct NNBody {
@@ -205,15 +202,320 @@ __global__ void nn_merge_kernel(const float2* __restrict__ part, int n_jc, int r
     }
 }
 
-// sigma sums over the nearest squared distances: per-block partials over contiguous slices
-// (fixed order), then one block over the partials (fixed order), so the result is deterministic
-__global__ void sigma_partial_kernel(const float* __restrict__ dmin, int n, int D, double* __restrict__ pe,
-                                     unsigned long long* __restrict__ pq)
+// ---------------------------------------------------------------------------
+// The pruned search: one block per tile of 32 sources (one per lane, the same in each of its NW
+// warps), the targets' tiles split round-robin over the warps.  A warp first searches the tile nearest
+// to one of the sources' subgroups, then each of its tiles whose super tile and whose own sphere are
+// not farther than the worst of the lanes' k-th distances (group against sphere, then sources
+// against sphere), the warps sharing each lane's best k-th distance.  The distances are the FP32
+// operations of the all-pairs kernels and ties go to the lowest index, so the results are theirs bit
+// for bit: a tile is skipped only when every target in it is strictly farther, with 1e-5 to spare for
+// the roundings of the tests (and a sphere or source that is not finite skips nothing).
+// Bound by latency, a chain of dependent tile searches: a source needs 7-12 tiles of 32 targets instead
+// of all.  So a tile is brought in by one coalesced load (16 bytes a lane) that overlaps the search
+// before it and is then broadcast from shared memory (32 uniform loads from L2 took twice as long),
+// eight warps share the tiles of a group where a block per SM is all there is, and where many spheres
+// pass the group's test they are filtered 32 at a time against the sources, not one by one.
+// Measured on one B200, all pairs -> pruned: nearest distance 65536 x 65536 922 -> 29 us (update_sig
+// 931 -> 52 us a call), 4501 x 3907 9.5 -> 8.2 us and no merge or sums after it (26 -> 8.2 us); 8 nearest
+// of 30000 x 28001 660 -> 53 us.  The all-pairs kernels stay for row ranges and pinned shapes.
+// ---------------------------------------------------------------------------
+struct PruneArgs {
+    const SortedPoint* xpt;
+    const Bound *xtile, *xsub;
+    const NNRec2* rec;       // targets in spatial order at the pose
+    const float4* sphere;    // their tiles and, behind them, super tiles
+    int N, n_tiles, n_super, k_out;
+    int* idx;                // [N][k_out], by source index; with d2
+    float* d2;
+    float* dmin;             // [N], or, for the quantised sigma alone:
+    unsigned long long* qsum;   // its integer sum (zeroed; any order gives the same)
+    int* ticket;                // blocks done (zeroed); the last one writes sigma
+    double *out, *host_out, *pose_sig;   // as sigma_kernel's
+    const int* err;
+};
+
+// the reference's term of sigma: rn_u32(fl32(d2min / D) * 1e6)
+__device__ __forceinline__ unsigned quantised(float d2, int D)
 {
-    pdl_trigger();   // a dependent of the merge of the nearest distances; the final sum one of this kernel
+    return __float2uint_rn(__fmul_rn(__fdiv_rn(d2, (float)D), 1000000.0f));
+}
+
+// the quantised sigma of n sources, rounded to float as update_sig returns it
+__device__ __forceinline__ double quantised_sigma(unsigned long long sum, int n)
+{
+    return (double)__double2float_rn((double)sum / 1e6 / (double)n);
+}
+
+template <int D>
+__device__ __forceinline__ float dist2(const float* p, const float4& c)
+{
+    const float dx = p[0] - c.x, dy = p[1] - c.y;
+    float d = fmaf(dy, dy, dx * dx);
+    if (D == 3) {
+        const float dz = p[2] - c.z;
+        d = fmaf(dz, dz, d);
+    }
+    return d;
+}
+
+// certainly farther than `bound`?  d2: squared distance to a sphere's centre, r: the radii to take off
+// (NaN and inf: no)
+__device__ __forceinline__ bool beyond(float d2, float r, float bound)
+{
+    const float q = r + bound;
+    return d2 * (1.f - 1e-5f) > q * q;
+}
+
+// K = 0: the nearest squared distance only; else sorted lists of the K nearest
+template <int D, int K, int NW>
+__global__ void __launch_bounds__(32 * NW) nn_prune_kernel(PruneArgs a)
+{
+    constexpr int KL = K > 0 ? K : 1;
+    constexpr unsigned long long kNone = (unsigned long long)0x7f800000u << 32 | 0x7fffffffu;
+    __shared__ int s_bound[kTile];                      // bounds on the lanes' k-th distances (float bits)
+    __shared__ int s_best[kTile];                       // K = 0: the squared distances
+    __shared__ int s_first[NW];
+    __shared__ float s_x[3][kTile];
+    __shared__ __align__(16) float4 s_rec[NW][2][kTile];   // two tiles of records per warp
+    __shared__ unsigned long long s_list[K > 0 ? NW - 1 : 1][KL][kTile];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int pos = blockIdx.x * kTile + lane;
+    const bool in = pos < a.N;
+    pdl_trigger();
+    // (the sources are init's, not the prologue's)
+    SortedPoint s = a.xpt[in ? pos : 0];
+    const Bound g = a.xtile[blockIdx.x];
+    float2 X[3];
+#pragma unroll
+    for (int q = 0; q < 3; ++q) X[q] = make_float2(s.p[q], s.p[q]);
+    float best = in ? INFINITY : -1.f;      // K = 0; a lane without a source takes nothing
+    unsigned long long list[KL];            // K > 0: (distance bits, index), ascending
+#pragma unroll
+    for (int q = 0; q < KL; ++q) list[q] = in ? kNone : 0ull;
+    float bound = best;
+    if (warp == 0) {
+        s_best[lane] = s_bound[lane] = __float_as_int(bound);
+#pragma unroll
+        for (int q = 0; q < 3; ++q) s_x[q][lane] = s.p[q];
+    }
     pdl_wait();
-    __shared__ double s_exact[256];
-    __shared__ unsigned long long s_q[256];
+    __syncthreads();
+
+    auto insert = [&](unsigned long long key) {
+        if (!(key < list[KL - 1])) return;
+#pragma unroll
+        for (int q = 0; q < KL; ++q) {
+            const unsigned long long o = list[q];
+            const bool lt = key < o;
+            list[q] = lt ? key : o;
+            key = lt ? o : key;
+        }
+    };
+    auto key_of = [](float dd, float j) {
+        return (unsigned long long)__float_as_uint(dd) << 32 | __float_as_uint(j);
+    };
+    const float4* rec4 = reinterpret_cast<const float4*>(a.rec);
+    int buf = 0;
+    // the tile whose records the warp holds in v (one float4 a lane)
+    auto search = [&](float4 v) {
+        float4* r = s_rec[warp][buf];
+        buf ^= 1;
+        r[lane] = v;
+        __syncwarp();
+        float2 nearest = make_float2(best, best);
+        // only what can still be among the K nearest (the others' lists count too)
+        const float cut = bound * bound * (1.f + 1e-5f);
+#pragma unroll 4
+        for (int e = 0; e < kTile / 2; ++e) {
+            const float4 ra = r[2 * e], rb = r[2 * e + 1];
+            const float2 d0 = fadd2(X[0], make_float2(ra.x, ra.y)), d1 = fadd2(X[1], make_float2(ra.z, ra.w));
+            float2 dd;
+            if (D == 3) {
+                const float2 d2 = fadd2(X[2], make_float2(rb.x, rb.y));
+                dd = ffma2(d2, d2, ffma2(d1, d1, fmul2(d0, d0)));
+            } else {
+                dd = ffma2(d1, d1, fmul2(d0, d0));
+            }
+            if constexpr (K == 0) {
+                nearest.x = fminf(nearest.x, dd.x);
+                nearest.y = fminf(nearest.y, dd.y);
+            } else {
+                const float top = fminf(cut, __uint_as_float((unsigned)(list[KL - 1] >> 32)));
+                if (dd.x <= top) insert(key_of(dd.x, rb.z));
+                if (dd.y <= top) insert(key_of(dd.y, rb.w));
+            }
+        }
+        if constexpr (K == 0) best = fminf(nearest.x, nearest.y);
+        const float kth = K == 0 ? best : __uint_as_float((unsigned)(list[KL - 1] >> 32));
+        // (distances order like their bits; -1 comes first)
+        if (in) atomicMin(&s_bound[lane], __float_as_int(sqrt_fast(kth) * (1.f + 1e-6f)));
+        bound = __int_as_float(*(volatile int*)&s_bound[lane]);
+    };
+
+    const float4* super = a.sphere + a.n_tiles;
+    // lane = sphere: can any source still need it?  (many spheres at a time, one test each per source)
+    auto filter = [&](float4 c, bool go) {
+        bool any = false;
+#pragma unroll 4
+        for (int q = 0; q < kTile; ++q) {
+            const float x[3] = {s_x[0][q], s_x[1][q], s_x[2][q]};
+            const float b = __int_as_float(*(volatile int*)&s_bound[q]);
+            any |= b >= 0.f && !beyond(dist2<D>(x, c), c.w, b);
+        }
+        return __ballot_sync(0xffffffffu, go && any);
+    };
+    auto refresh = [&]() {   // this lane's bound, and the worst of the group's
+        bound = __int_as_float(*(volatile int*)&s_bound[lane]);
+        return __int_as_float(__reduce_max_sync(0xffffffffu, __float_as_int(bound)));
+    };
+    // a warp's tiles of up to NW super tiles at a time: fn(lane's tile or -1, its sphere)
+    constexpr int TPW = kSuper / NW;
+    auto each_tile = [&](unsigned mask, int sbase, auto&& fn) {
+        while (mask) {
+            int mine = -1;
+#pragma unroll
+            for (int k = 0; k < NW; ++k) {
+                const int bit = __ffs(mask) - 1;   // -1: none left
+                mask &= mask - 1;
+                if (k == lane / TPW) mine = bit;
+            }
+            int t = mine < 0 ? -1 : (sbase + mine) * kSuper + (lane % TPW) * NW + warp;
+            if (t >= a.n_tiles) t = -1;
+            fn(t, a.sphere[t < 0 ? 0 : t]);
+        }
+    };
+
+    // The warp's first tile: the one nearest to subgroup warp % 4, in the super tile nearest to it (of
+    // eight warps, the nearest even one and the nearest odd one); the same tile only once.
+    {
+        const Bound h = a.xsub[4 * blockIdx.x + warp % 4];
+        unsigned near = 0xffffffffu;
+        int s0 = 0;
+        for (int u = lane; u < a.n_super; u += 32) {
+            const unsigned key = __float_as_uint(dist2<D>(h.c, super[u]));
+            if (key < near) { near = key; s0 = u; }
+        }
+        unsigned least = __reduce_min_sync(0xffffffffu, near);
+        unsigned who = __ballot_sync(0xffffffffu, near == least);
+        s0 = __shfl_sync(0xffffffffu, s0, __ffs(who) - 1);
+        int t0 = s0 * kSuper + lane;
+        const bool own = t0 < a.n_tiles && (NW == 4 || lane % 2 == warp / 4);
+        near = own ? __float_as_uint(dist2<D>(h.c, a.sphere[t0])) : 0xffffffffu;
+        least = __reduce_min_sync(0xffffffffu, near);
+        who = __ballot_sync(0xffffffffu, own && near == least);
+        t0 = who ? s0 * kSuper + __ffs(who) - 1 : -1;
+        if (lane == 0) s_first[warp] = t0;
+        const float4 v = rec4[(size_t)max(t0, 0) * kTile + lane];
+        __syncthreads();
+        bool dup = t0 < 0;
+        for (int k = 0; k < warp; ++k) dup |= s_first[k] == t0;
+        if (!dup) search(v);
+        __syncthreads();   // (every warp's first bounds)
+    }
+    // the others
+    for (int base = 0; base < a.n_super; base += 32) {
+        const int u = min(base + lane, a.n_super - 1);
+        const float4 cs = super[u];
+        const float worst = refresh();
+        const bool go = base + lane < a.n_super && !beyond(dist2<D>(g.c, cs), cs.w + g.r, worst);
+        unsigned mask = __ballot_sync(0xffffffffu, go);
+        if (__popc(mask) > 2 * NW) mask = filter(cs, go);
+        each_tile(mask, base, [&](int t, float4 c) {
+            const float worst_now = refresh();
+            bool need = t >= 0 && !beyond(dist2<D>(g.c, c), c.w + g.r, worst_now);
+#pragma unroll
+            for (int k = 0; k < NW; ++k) need &= t != s_first[k];
+            unsigned todo = __ballot_sync(0xffffffffu, need);
+            if (__popc(todo) > 3) todo = filter(c, need);
+            if (!todo) return;
+            int from = __ffs(todo) - 1;
+            float4 v = rec4[(size_t)__shfl_sync(0xffffffffu, t, from) * kTile + lane];
+            while (todo) {
+                const float4 cu = make_float4(__shfl_sync(0xffffffffu, c.x, from), __shfl_sync(0xffffffffu, c.y, from),
+                                              __shfl_sync(0xffffffffu, c.z, from), __shfl_sync(0xffffffffu, c.w, from));
+                todo &= todo - 1;
+                const float4 vu = v;
+                from = todo ? __ffs(todo) - 1 : from;
+                const int tn = __shfl_sync(0xffffffffu, t, from);
+                if (todo) v = rec4[(size_t)tn * kTile + lane];   // the next one, meanwhile
+                if (__any_sync(0xffffffffu, in && !beyond(dist2<D>(s.p, cu), cu.w, bound))) search(vu);
+            }
+        });
+    }
+    // the warps' results
+    if constexpr (K == 0)
+        atomicMin(&s_best[lane], __float_as_int(best));
+    else if (warp > 0)
+#pragma unroll
+        for (int q = 0; q < KL; ++q) s_list[warp - 1][q][lane] = list[q];
+    __syncthreads();
+    if (warp > 0) return;
+    if constexpr (K == 0) {
+        const float d2 = __int_as_float(s_best[lane]);
+        if (!a.qsum) {
+            if (in) a.dmin[s.idx] = d2;
+            return;
+        }
+        const unsigned q = in ? quantised(d2, D) : 0u;
+        const unsigned lo = __reduce_add_sync(0xffffffffu, q & 0xffffu), hi = __reduce_add_sync(0xffffffffu, q >> 16);
+        if (lane == 0) {
+            atomicAdd(a.qsum, ((unsigned long long)hi << 16) + lo);
+            __threadfence();
+            if (atomicAdd(a.ticket, 1) == (int)gridDim.x - 1) {
+                __threadfence();
+                const double sig = quantised_sigma(__ldcg(a.qsum), a.N);
+                a.out[1] = sig;
+                if (a.pose_sig) a.pose_sig[kPoseSig] = sig;
+                if (a.host_out) {
+                    a.host_out[1] = sig;
+                    a.host_out[2] = (double)*a.err;
+                }
+            }
+        }
+    } else if (in) {
+        for (int w = 0; w < NW - 1; ++w)
+            for (int q = 0; q < KL; ++q) insert(s_list[w][q][lane]);
+#pragma unroll
+        for (int q = 0; q < KL; ++q)
+            if (q < a.k_out) {
+                a.idx[(size_t)s.idx * a.k_out + q] = (int)(unsigned)list[q];
+                a.d2[(size_t)s.idx * a.k_out + q] = __uint_as_float((unsigned)(list[q] >> 32));
+            }
+    }
+}
+
+// sigma from the nearest squared distances: per-block partials over contiguous slices (fixed
+// order), then the block that finishes last sums the partials (fixed order too, so the result is
+// deterministic); ticket was zeroed by the search prologue.  n_all: the sources, or 0 for the partial
+// sums of a row range.  host_out (optional, mapped pinned memory) receives out[0..1] and the error
+// word at [2]; pose_sig (optional) a device pose block whose sig becomes out[1].
+__global__ void __launch_bounds__(256) sigma_kernel(const float* dmin, int n, int D, int n_all, double* pe,
+                                                    unsigned long long* pq, int* ticket, double* out,
+                                                    double* host_out, const int* err, double* pose_sig)
+{
+    pdl_trigger();   // a dependent of the search
+    pdl_wait();
+    __shared__ double s_exact[8];
+    __shared__ unsigned long long s_q[8];
+    __shared__ bool s_last;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    auto block_total = [&](double& se, unsigned long long& sq) {   // (in thread 0)
+        se = warp_sum(se);
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) sq += __shfl_xor_sync(0xffffffffu, sq, o);
+        __syncthreads();
+        if (lane == 0) {
+            s_exact[warp] = se;
+            s_q[warp] = sq;
+        }
+        __syncthreads();
+        if (threadIdx.x == 0)
+            for (int w = 1; w < 8; ++w) {
+                se += s_exact[w];
+                sq += s_q[w];
+            }
+    };
     const int per = (n + gridDim.x - 1) / gridDim.x;
     const int b0 = blockIdx.x * per, b1 = min(n, b0 + per);
     double se = 0;
@@ -221,62 +523,37 @@ __global__ void sigma_partial_kernel(const float* __restrict__ dmin, int n, int 
     for (int i = b0 + threadIdx.x; i < b1; i += blockDim.x) {
         const float v = dmin[i];
         se += (double)v;
-        const float sv = __fmul_rn(__fdiv_rn(v, (float)D), 1000000.0f);
-        sq += (unsigned long long)__float2uint_rn(sv);
+        sq += (unsigned long long)quantised(v, D);
     }
-    s_exact[threadIdx.x] = se;
-    s_q[threadIdx.x] = sq;
-    __syncthreads();
-    for (int h = blockDim.x / 2; h > 0; h >>= 1) {
-        if (threadIdx.x < h) {
-            s_exact[threadIdx.x] += s_exact[threadIdx.x + h];
-            s_q[threadIdx.x] += s_q[threadIdx.x + h];
-        }
-        __syncthreads();
-    }
+    block_total(se, sq);
     if (threadIdx.x == 0) {
-        pe[blockIdx.x] = s_exact[0];
-        pq[blockIdx.x] = s_q[0];
+        pe[blockIdx.x] = se;
+        pq[blockIdx.x] = sq;
+        __threadfence();
+        s_last = atomicAdd(ticket, 1) == (int)gridDim.x - 1;
     }
-}
-
-// host_out (optional, mapped pinned memory) receives out[0..1] and the error word at [2];
-// pose_sig (optional) a device pose block whose sig becomes out[1]
-__global__ void sigma_final_kernel(const double* __restrict__ pe, const unsigned long long* __restrict__ pq, int nb,
-                                   int n, int D, double* __restrict__ out, double* __restrict__ host_out,
-                                   const int* __restrict__ err, double* __restrict__ pose_sig)
-{
-    pdl_wait();   // a dependent of sigma_partial_kernel
-    __shared__ double s_exact[256];
-    __shared__ unsigned long long s_q[256];
-    double se = 0;
-    unsigned long long sq = 0;
-    for (int i = threadIdx.x; i < nb; i += blockDim.x) {
-        se += pe[i];
-        sq += pq[i];
-    }
-    s_exact[threadIdx.x] = se;
-    s_q[threadIdx.x] = sq;
     __syncthreads();
-    for (int h = blockDim.x / 2; h > 0; h >>= 1) {
-        if (threadIdx.x < h) {
-            s_exact[threadIdx.x] += s_exact[threadIdx.x + h];
-            s_q[threadIdx.x] += s_q[threadIdx.x + h];
-        }
-        __syncthreads();
+    if (!s_last) return;
+    __threadfence();
+    se = 0;
+    sq = 0;
+    for (int i = threadIdx.x; i < (int)gridDim.x; i += blockDim.x) {
+        se += __ldcg(pe + i);
+        sq += __ldcg(pq + i);
     }
+    block_total(se, sq);
     if (threadIdx.x == 0) {
         double o0, o1;
-        if (n > 0) {
-            o0 = s_exact[0] / ((double)D * n);
-            o1 = (double)__double2float_rn((double)s_q[0] / 1e6 / (double)n);
+        if (n_all > 0) {
+            o0 = se / ((double)D * n_all);
+            o1 = quantised_sigma(sq, n_all);
         } else {   // the partial sums of a row range: sum d2min, and the sum of the quantised terms
-            o0 = s_exact[0];
-            o1 = (double)s_q[0];
+            o0 = se;
+            o1 = (double)sq;
         }
         out[0] = o0;
         out[1] = o1;
-        if (pose_sig) pose_sig[kPoseSig] = o1;   // the quantised sigma, rounded to float as update_sig returns it
+        if (pose_sig) pose_sig[kPoseSig] = o1;
         if (host_out) {
             host_out[0] = o0;
             host_out[1] = o1;
@@ -324,14 +601,30 @@ std::vector<KernelShape> nn_shapes()
     return s;
 }
 
-// Runs the brute-force search; dmin_dev (nullable) receives the nearest squared distance per source.
+template <int D, int NW>
+static void (*prune_kernel(int K))(PruneArgs)
+{
+    return K == 0 ? nn_prune_kernel<D, 0, NW>
+                  : (K == 1 ? nn_prune_kernel<D, 1, NW>
+                            : (K == 8 ? nn_prune_kernel<D, 8, NW> : nn_prune_kernel<D, 16, NW>));
+}
+
+static bool nn_pruned(const Context& c, const KernelShape* force, int rows)
+{
+    return !force && !c.nn_pinned && rows == c.N;
+}
+
+// Runs the search; dmin_dev (nullable) receives the nearest squared distance per source.
 // Source rows [i0, i1) (i1 < 0: all); idx/d2 rows are relative to i0, dmin is indexed absolutely.
 // The search: the targets' search records (the nearest-neighbour prologue, which also zeroes the
-// work counter, and the error word when reset_err; the pose by value when pv, or read from
-// pose_src), the pair kernel, the merge of its per-chunk lists.
+// work counters, and the error word when reset_err; the pose by value when pv, or read from
+// pose_src), then over all rows the pruned search in spatial order, and for a row range, or when a
+// kernel shape is asked for (force, nn_pinned), the all-pairs kernel and the merge of its per-chunk
+// lists.  quant: the pruned search also sums the quantised sigma (SigmaOpts) into out_dev[1].
 static int nn_run(Context& c, double* pose_dev, int k, int* idx_dev, float* d2_dev, float* dmin_dev,
                   cudaStream_t s, const KernelShape* force, int i0 = 0, int i1 = -1, const PoseBlock* pv = nullptr,
-                  const double* pose_src = nullptr, bool reset_err = false)
+                  const double* pose_src = nullptr, bool reset_err = false, const SigmaOpts* quant = nullptr,
+                  double* out_dev = nullptr)
 {
     if (i1 < 0) i1 = c.N;
     const int rows = i1 - i0;
@@ -339,7 +632,23 @@ static int nn_run(Context& c, double* pose_dev, int k, int* idx_dev, float* d2_d
         DUGMA_RET(launch_pose_in(c, pose_src, pose_dev, s, reset_err));
         reset_err = false;
     }
-    DUGMA_RET(launch_nn_prologue(c, pose_dev, s, pv, c.counter, reset_err ? c.err : nullptr));
+    const bool pruned = nn_pruned(c, force, rows);
+    DUGMA_RET(launch_nn_prologue(c, pose_dev, s, pv, c.counter, reset_err ? c.err : nullptr, pruned));
+    if (pruned) {
+        const int K = !idx_dev ? 0 : (k <= 1 ? 1 : (k <= 8 ? 8 : 16));
+        const int nx = (c.N + kTile - 1) / kTile;
+        constexpr int kSpan = kTile * kSuper;
+        const PruneArgs a{c.xpt, c.xtile, c.xsub, reinterpret_cast<const NNRec2*>(c.yp32), c.ysphere, c.N,
+                          (c.M + kTile - 1) / kTile, (c.M + kSpan - 1) / kSpan, k, idx_dev, d2_dev, dmin_dev,
+                          quant ? reinterpret_cast<unsigned long long*>(c.counter + 2) : nullptr, c.counter + 1, out_dev,
+                          quant ? quant->host_out : nullptr, quant ? quant->pose_sig : nullptr, c.err};
+        // eight warps a group up to two groups per SM, else four
+        const bool wide = nx <= 2 * c.num_sms;
+        auto fn = wide ? (c.D == 3 ? prune_kernel<3, 8>(K) : prune_kernel<2, 8>(K))
+                       : (c.D == 3 ? prune_kernel<3, 4>(K) : prune_kernel<2, 4>(K));
+        DUGMA_CK(launch_dependent(c.pdl, fn, nx, wide ? 256 : 128, 0, s, a));
+        return DUGMA_OK;
+    }
     const KernelShape want = force ? *force : c.shape_nn;
     const auto& vars = c.D == 3 ? nn_variants<3>() : nn_variants<2>();
     const NNVariant* v = &vars[0];
@@ -389,18 +698,18 @@ int launch_sigma(Context& c, double* pose_dev, double* out_dev, cudaStream_t s, 
     const bool whole = i1 < 0;
     if (whole) i1 = c.N;
     const int rows = i1 - i0;
+    const bool quant = !o.exact && whole && nn_pruned(c, nullptr, rows);
     DUGMA_RET(nn_run(c, pose_dev, 1, nullptr, nullptr, c.dmin, s, nullptr, i0, i1, o.pose_value, o.pose_src,
-                     o.reset_err));
+                     o.reset_err, quant ? &o : nullptr, out_dev));
+    if (quant) return DUGMA_OK;
     // partials in the scratch region (the search's chunk lists there are merged by now, in stream order)
-    const int nb = std::max(1, std::min(2 * c.num_sms, (rows + 1023) / 1024));
+    const int nb = std::max(1, std::min(2 * c.num_sms, (rows + 511) / 512));
     DUGMA_RET(c.ensure_scratch(sizeof(double) * 2 * (size_t)nb));
     double* pe = c.scratch;
     unsigned long long* pq = reinterpret_cast<unsigned long long*>(c.scratch + nb);
-    DUGMA_CK(launch_dependent(c.pdl, sigma_partial_kernel, nb, 256, 0, s, (const float*)(c.dmin + i0), rows, c.D, pe,
-                              pq));
-    DUGMA_CK(launch_dependent(c.pdl, sigma_final_kernel, 1, 256, 0, s, (const double*)pe,
-                              (const unsigned long long*)pq, nb, whole ? c.N : 0, c.D, out_dev, o.host_out,
-                              (const int*)c.err, o.pose_sig));
+    DUGMA_CK(launch_dependent(c.pdl, sigma_kernel, nb, 256, 0, s, (const float*)(c.dmin + i0), rows, c.D,
+                              whole ? c.N : 0, pe, pq, c.counter + 1, out_dev, o.host_out, (const int*)c.err,
+                              o.pose_sig));
     return DUGMA_OK;
 }
 
