@@ -215,7 +215,7 @@ static void destroy_context(Context* c)
     if (!c) return;
     if (c->stream) cudaStreamSynchronize(c->stream);
     arena_release(c->dev, c->arena, c->arena_bytes);
-    void* bufs[] = {c->scratch_extra, c->yrec128, c->xrec128, c->yrec256, c->xrec256, c->mom_part, c->dedx};
+    void* bufs[] = {c->scratch_extra, c->yrec128, c->xrec128, c->yrec256, c->xrec256, c->mom_part, c->dedx, c->nn_out};
     for (void* b : bufs)
         if (b) cudaFree(b);
     pinned_release(c->host);
@@ -698,20 +698,29 @@ int dugma_nn(float* Ptr[6], const double* R, const double* t, int k, int* idx, f
     GET_CTX(c, Ptr);
     if (k < 1 || k > 16 || k > c->M) return set_error(DUGMA_ERR_ARG, "nn: k = %d must be in [1, min(16, M)]", k);
     DUGMA_RET(upload_pose(*c, R, t, 1.0));
-    int* di = nullptr;
-    float* dd = nullptr;
-    DUGMA_CK(cudaMallocAsync(&di, sizeof(int) * (size_t)c->N * k, c->stream));
-    DUGMA_CK(cudaMallocAsync(&dd, sizeof(float) * (size_t)c->N * k, c->stream));
-    int rc = launch_nn(*c, c->pose, k, di, dd, c->stream);
-    if (rc == DUGMA_OK) {
-        cudaMemcpyAsync(idx, di, sizeof(int) * (size_t)c->N * k, cudaMemcpyDeviceToHost, c->stream);
-        cudaMemcpyAsync(d2, dd, sizeof(float) * (size_t)c->N * k, cudaMemcpyDeviceToHost, c->stream);
-        rc = fetch(*c, c->out, 0, nullptr);
+    // results in the scratch, which the pruned search leaves alone (a pinned all-pairs shape keeps its
+    // lists there: then a buffer that stays with the context); allocating them per call took longer
+    // than the search
+    const size_t n = (size_t)c->N * k, bytes = (sizeof(int) + sizeof(float)) * n;
+    if (c->nn_pinned && n > c->nn_slots) {
+        if (c->nn_out) cudaFree(c->nn_out);
+        c->nn_out = nullptr;
+        c->nn_slots = 0;
+        if (cudaMalloc(&c->nn_out, bytes) != cudaSuccess) {
+            cudaGetLastError();
+            c->nn_out = nullptr;
+            return set_error(DUGMA_ERR_NOMEM, "nn: cannot allocate %zu bytes", bytes);
+        }
+        c->nn_slots = n;
+    } else if (!c->nn_pinned) {
+        DUGMA_RET(c->ensure_scratch(bytes));
     }
-    cudaFreeAsync(di, c->stream);
-    cudaFreeAsync(dd, c->stream);
-    cudaStreamSynchronize(c->stream);
-    return rc;
+    int* di = static_cast<int*>(c->nn_pinned ? c->nn_out : (void*)c->scratch);
+    float* dd = reinterpret_cast<float*>(di + n);
+    DUGMA_RET(launch_nn(*c, c->pose, k, di, dd, c->stream));
+    DUGMA_CK(cudaMemcpyAsync(idx, di, sizeof(int) * n, cudaMemcpyDeviceToHost, c->stream));
+    DUGMA_CK(cudaMemcpyAsync(d2, dd, sizeof(float) * n, cudaMemcpyDeviceToHost, c->stream));
+    return fetch(*c, c->out, 0, nullptr);
 }
 
 int dugma_energy_grad_async(float* Ptr[6], const double* pose_dev, int model, double* out_dev, double* dEdx_dev,

@@ -101,6 +101,8 @@ struct Context {
     float4* ysphere = nullptr;                // the target tiles' and super tiles' spheres at a pose
     bool nn_pinned = false;                   // a nearest-neighbour kernel shape was pinned: no pruning
     double* dedx = nullptr;                   // dE/dx rows (allocated on first request)
+    void* nn_out = nullptr;                   // dugma_nn's results under a pinned shape (on request)
+    size_t nn_slots = 0;                      // its (index, distance) pairs
     double* mom = nullptr;                    // surrogate moments (512 doubles)
     double* mom_part = nullptr;               // per-block moment partials (with the 128-byte records)
     // scratch: a region of the arena, replaced by a separate allocation if a launch needs more

@@ -113,14 +113,18 @@ extern "C" int dugma_knn_covariance(const double* points, int n, int D, int k, d
         for (int q = 0; q < 16; ++q) h[q] = 0.0;
         for (int q = 0; q < D * D; ++q) h[q] = D == 3 ? ident[q] : ident2[q];
         h[kPoseSig] = 1.0;
+        // workspace: the context's scratch, which the pruned search leaves alone
+        const size_t nk = (size_t)n * kk, nd = (size_t)n * D;
+        rc = c->ensure_scratch(sizeof(double) * (nd * D + nd) + (sizeof(int) + sizeof(float)) * nk);
+        if (rc != DUGMA_OK) break;
+        covd = c->scratch;
+        ptsd = covd + nd * D;
+        idx = reinterpret_cast<int*>(ptsd + nd);
+        d2 = reinterpret_cast<float*>(idx + nk);
         if (cudaMemcpyAsync(c->pose, h, sizeof(double) * 16, cudaMemcpyHostToDevice, s) != cudaSuccess ||
-            cudaMallocAsync(&idx, sizeof(int) * (size_t)n * kk, s) != cudaSuccess ||
-            cudaMallocAsync(&d2, sizeof(float) * (size_t)n * kk, s) != cudaSuccess ||
-            cudaMallocAsync(&covd, sizeof(double) * (size_t)n * D * D, s) != cudaSuccess ||
-            cudaMallocAsync(&ptsd, sizeof(double) * (size_t)n * D, s) != cudaSuccess ||
-            cudaMemcpyAsync(ptsd, points, sizeof(double) * (size_t)n * D, cudaMemcpyHostToDevice, s) != cudaSuccess) {
+            cudaMemcpyAsync(ptsd, points, sizeof(double) * nd, cudaMemcpyHostToDevice, s) != cudaSuccess) {
             cudaGetLastError();
-            rc = set_error(DUGMA_ERR_NOMEM, "knn_covariance: device allocation failed");
+            rc = set_error(DUGMA_ERR_CUDA, "knn_covariance: copy failed");
             break;
         }
         rc = launch_nn(*c, c->pose, kk, idx, d2, s);
@@ -134,10 +138,6 @@ extern "C" int dugma_knn_covariance(const double* points, int n, int D, int k, d
             cudaMemcpyAsync(cov, covd, sizeof(double) * (size_t)n * D * D, cudaMemcpyDeviceToHost, s) != cudaSuccess)
             rc = set_error(DUGMA_ERR_CUDA, "knn_covariance: kernel failed");
     } while (false);
-    if (idx) cudaFreeAsync(idx, s);
-    if (d2) cudaFreeAsync(d2, s);
-    if (covd) cudaFreeAsync(covd, s);
-    if (ptsd) cudaFreeAsync(ptsd, s);
     if (cudaStreamSynchronize(s) != cudaSuccess && rc == DUGMA_OK)
         rc = set_error(DUGMA_ERR_CUDA, "knn_covariance: kernel failed");
     dugma_fr_m(Ptr);
