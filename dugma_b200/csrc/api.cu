@@ -497,6 +497,9 @@ int dugma_init(const double* X, const double* X_C, const double* Y, const double
     // the kernels of a call each wait for the one before (DUGMA_NO_PDL set): no early launch
     const char* no_pdl = getenv("DUGMA_NO_PDL");
     c->pdl = !(no_pdl && *no_pdl && *no_pdl != '0');
+    // every pair evaluated, also those whose terms are known to be 0 (DUGMA_ALL_PAIRS set)
+    const char* all = getenv("DUGMA_ALL_PAIRS");
+    c->all_pairs = all && *all && *all != '0';
     const char* no_map = getenv("DUGMA_NO_MAPPED_STAGING");
     if ((no_map && *no_map && *no_map != '0') ||
         cudaHostGetDevicePointer((void**)&c->host_dev, c->host, 0) != cudaSuccess) {
@@ -604,7 +607,8 @@ int dugma_energy(float* Ptr[6], const double* R, const double* t, double sig, in
         return mapped_fetch(*c, 1, E);
     }
     DUGMA_RET(upload_pose(*c, R, t, sig));
-    DUGMA_RET(launch_pairs(*c, c->pose, model, false, 0, c->N, c->out, nullptr, c->stream));
+    io.sig = sig;
+    DUGMA_RET(launch_pairs(*c, c->pose, model, false, 0, c->N, c->out, nullptr, c->stream, nullptr, &io));
     return fetch(*c, c->out, 1, E);
 }
 
@@ -622,7 +626,9 @@ static int energy_grad_impl(Context* c, const double* R, const double* t, double
     } else {
         DUGMA_RET(upload_pose(*c, R, t, sig));
         if (dEdx && !c->dedx) DUGMA_CK(cudaMalloc(&c->dedx, sizeof(double) * (size_t)c->N * c->D));
-        DUGMA_RET(launch_pairs(*c, c->pose, model, true, i0, i1, c->out, dEdx ? c->dedx : nullptr, c->stream));
+        io.sig = sig;
+        DUGMA_RET(launch_pairs(*c, c->pose, model, true, i0, i1, c->out, dEdx ? c->dedx : nullptr, c->stream, nullptr,
+                               &io));
         if (dEdx)
             DUGMA_CK(cudaMemcpyAsync(dEdx, c->dedx, sizeof(double) * (size_t)(i1 - i0) * c->D, cudaMemcpyDeviceToHost,
                                      c->stream));
@@ -681,8 +687,10 @@ int dugma_energy_fd_grad(float* Ptr[6], const double* R, const double* t, double
     DUGMA_CK(cudaMemcpyAsync(poses, hp, sizeof(double) * 16 * nev, cudaMemcpyHostToDevice, c->stream));
     DUGMA_CK(cudaMemsetAsync(c->err, 0, sizeof(int), c->stream));
     int rc = DUGMA_OK;
+    EvalIO io;
+    io.sig = sig;
     for (int k = 0; k < nev && rc == DUGMA_OK; ++k)
-        rc = launch_pairs(*c, poses + 16 * k, model, false, 0, c->N, c->out + k, nullptr, c->stream);
+        rc = launch_pairs(*c, poses + 16 * k, model, false, 0, c->N, c->out + k, nullptr, c->stream, nullptr, &io);
     double ev[16];
     if (rc == DUGMA_OK) rc = fetch(*c, c->out, nev, ev);
     cudaStreamSynchronize(c->stream);

@@ -310,6 +310,73 @@ __device__ __forceinline__ float2 fld(const YRec2& r, int f)
     return (f & 1) ? make_float2(q.z, q.w) : make_float2(q.x, q.y);
 }
 
+// One source's contribution to the pose gradient (added to acc[1..]) and dE/dx_i from its z-frame
+// moments, in FP64: with U the record's Cholesky factor (U^T U = |k| B), V = U^-1,
+//   B D2 = U^T D2z / |k|,   sum e2 d x B d = sum_ab Q2z_ab (V e_a) x (U^T e_b) / |k|.
+// w: the source's weight (0, neglected: U = 0 and no contribution); q2 packed.
+template <int D>
+__device__ __forceinline__ void chol_contract(double w, const float2* B, const float2* X, const double* t,
+                                              const double* s1, const double* d2, const double* q2, double* acc,
+                                              double* dx)
+{
+    constexpr int NS = Sym<D>::N, NR = Sym<D>::NR;
+    const double kinv = 1.0 / K_EXP2, rk = -kinv;
+    double gt[3] = {0, 0, 0};
+    if (w != 0.0) {
+        double U[3][3] = {{0, 0, 0}, {0, 0, 0}, {0, 0, 0}}, Qm[3][3];
+#pragma unroll
+        for (int q = 0; q < NS; ++q) {
+            const int ra = Sym<D>::a(q), rb = Sym<D>::b(q);
+            U[ra][rb] = (double)B[q].x;
+            Qm[ra][rb] = Qm[rb][ra] = q2[q];
+        }
+        double V[3][3] = {{0, 0, 0}, {0, 0, 0}, {0, 0, 0}};
+        V[0][0] = 1.0 / U[0][0];
+        V[1][1] = 1.0 / U[1][1];
+        V[0][1] = -U[0][1] * V[0][0] * V[1][1];
+        if (D == 3) {
+            V[2][2] = 1.0 / U[2][2];
+            V[1][2] = -U[1][2] * V[1][1] * V[2][2];
+            V[0][2] = (U[0][1] * U[1][2] - U[0][2] * U[1][1]) * V[0][0] * V[1][1] * V[2][2];
+        }
+        double p[3];
+#pragma unroll
+        for (int q = 0; q < D; ++q) {
+            double bd = 0;
+#pragma unroll
+            for (int cc = 0; cc < D; ++cc) bd += U[cc][q] * d2[cc];
+            gt[q] = s1[q] * kinv + rk * bd;
+            p[q] = (double)X[q].x - t[q];
+        }
+        if (D == 3) {
+            double qx[3] = {0, 0, 0};
+#pragma unroll
+            for (int aa = 0; aa < 3; ++aa)
+#pragma unroll
+                for (int bb = 0; bb < 3; ++bb) {
+                    const double q = Qm[aa][bb];
+                    qx[0] += q * (V[1][aa] * U[bb][2] - V[2][aa] * U[bb][1]);
+                    qx[1] += q * (V[2][aa] * U[bb][0] - V[0][aa] * U[bb][2]);
+                    qx[2] += q * (V[0][aa] * U[bb][1] - V[1][aa] * U[bb][0]);
+                }
+            acc[1] += w * (p[1] * gt[2] - p[2] * gt[1] - rk * qx[0]);
+            acc[2] += w * (p[2] * gt[0] - p[0] * gt[2] - rk * qx[1]);
+            acc[3] += w * (p[0] * gt[1] - p[1] * gt[0] - rk * qx[2]);
+        } else {
+            double qx = 0;
+#pragma unroll
+            for (int aa = 0; aa < 2; ++aa)
+#pragma unroll
+                for (int bb = 0; bb < 2; ++bb) qx += Qm[aa][bb] * (V[0][aa] * U[bb][1] - V[1][aa] * U[bb][0]);
+            acc[1] += w * (p[0] * gt[1] - p[1] * gt[0] - rk * qx);
+        }
+#pragma unroll
+        for (int q = 0; q < D; ++q) acc[1 + NR + q] += w * gt[q];
+    }
+#pragma unroll
+    for (int q = 0; q < D; ++q) dx[q] = -w * gt[q];
+}
+
 // CHOL: the source side in the Cholesky form of the x record (U^T U = |k| B_i, z = U d): the B
 // exponent is lv - |z|^2 (9 FP32 operations in 3D, as the Horner form), a sum of squares, so the FP32
 // rounding of the record moves it by ~sqrt(cond B_i) ulps instead of ~cond B_i; the e2 moments are
@@ -463,79 +530,30 @@ struct PackedBody {
         else
             finish_horner(a, jc, acc);
     }
-    // Cholesky form: with U the record's factor (U^T U = |k| B), V = U^-1 and the z-frame moments,
-    //   B D2 = U^T D2z / |k|,   sum e2 d x B d = sum_ab Q2z_ab (V e_a) x (U^T e_b) / |k|.
+    // Cholesky form (chol_contract)
     __device__ void finish_chol(const PairArgs& a, int jc, double (&acc)[NV])
     {
-        const double kinv = 1.0 / K_EXP2, rk = -kinv;
 #pragma unroll
         for (int ii = 0; ii < IPT; ++ii) {
             if (row[ii] < 0) continue;
             const int i = row[ii];
             const double w = (double)a.wx[i] * G;
             acc[0] += w * E64[ii];
-            if (!GRAD) continue;
-            double gt[3] = {0, 0, 0};
-            if (w != 0.0) {   // neglected sources carry U = 0 and weight 0
-                double U[3][3] = {{0, 0, 0}, {0, 0, 0}, {0, 0, 0}}, Qm[3][3], s1[3], d2[3];
-#pragma unroll
-                for (int q = 0; q < NS; ++q) {
-                    const int ra = Sym<D>::a(q), rb = Sym<D>::b(q);
-                    U[ra][rb] = (double)B[ii][q].x;
-                    Qm[ra][rb] = Qm[rb][ra] = (double)Q2[ii][q].x + (double)Q2[ii][q].y;
-                }
+            if constexpr (GRAD) {
+                double s1[3], d2[3], q2[6], dx[3];
 #pragma unroll
                 for (int q = 0; q < D; ++q) {
                     s1[q] = (double)S1[ii][q].x + (double)S1[ii][q].y;
                     d2[q] = (double)D2[ii][q].x + (double)D2[ii][q].y;
                 }
-                double V[3][3] = {{0, 0, 0}, {0, 0, 0}, {0, 0, 0}};
-                V[0][0] = 1.0 / U[0][0];
-                V[1][1] = 1.0 / U[1][1];
-                V[0][1] = -U[0][1] * V[0][0] * V[1][1];
-                if (D == 3) {
-                    V[2][2] = 1.0 / U[2][2];
-                    V[1][2] = -U[1][2] * V[1][1] * V[2][2];
-                    V[0][2] = (U[0][1] * U[1][2] - U[0][2] * U[1][1]) * V[0][0] * V[1][1] * V[2][2];
+#pragma unroll
+                for (int q = 0; q < NS; ++q) q2[q] = (double)Q2[ii][q].x + (double)Q2[ii][q].y;
+                chol_contract<D>(w, B[ii], X[ii], t, s1, d2, q2, acc, dx);
+                if (a.dx_part) {
+                    const int rows = a.i_end - a.i0;
+#pragma unroll
+                    for (int q = 0; q < D; ++q) a.dx_part[((size_t)jc * rows + (i - a.i0)) * D + q] = dx[q];
                 }
-                double p[3];
-#pragma unroll
-                for (int q = 0; q < D; ++q) {
-                    double bd = 0;
-#pragma unroll
-                    for (int cc = 0; cc < D; ++cc) bd += U[cc][q] * d2[cc];
-                    gt[q] = s1[q] * kinv + rk * bd;
-                    p[q] = (double)X[ii][q].x - t[q];
-                }
-                if (D == 3) {
-                    double qx[3] = {0, 0, 0};
-#pragma unroll
-                    for (int aa = 0; aa < 3; ++aa)
-#pragma unroll
-                        for (int bb = 0; bb < 3; ++bb) {
-                            const double q = Qm[aa][bb];
-                            qx[0] += q * (V[1][aa] * U[bb][2] - V[2][aa] * U[bb][1]);
-                            qx[1] += q * (V[2][aa] * U[bb][0] - V[0][aa] * U[bb][2]);
-                            qx[2] += q * (V[0][aa] * U[bb][1] - V[1][aa] * U[bb][0]);
-                        }
-                    acc[1] += w * (p[1] * gt[2] - p[2] * gt[1] - rk * qx[0]);
-                    acc[2] += w * (p[2] * gt[0] - p[0] * gt[2] - rk * qx[1]);
-                    acc[3] += w * (p[0] * gt[1] - p[1] * gt[0] - rk * qx[2]);
-                } else {
-                    double qx = 0;
-#pragma unroll
-                    for (int aa = 0; aa < 2; ++aa)
-#pragma unroll
-                        for (int bb = 0; bb < 2; ++bb) qx += Qm[aa][bb] * (V[0][aa] * U[bb][1] - V[1][aa] * U[bb][0]);
-                    acc[1] += w * (p[0] * gt[1] - p[1] * gt[0] - rk * qx);
-                }
-#pragma unroll
-                for (int q = 0; q < D; ++q) acc[1 + NR + q] += w * gt[q];
-            }
-            if (a.dx_part) {
-                const int rows = a.i_end - a.i0;
-#pragma unroll
-                for (int q = 0; q < D; ++q) a.dx_part[((size_t)jc * rows + (i - a.i0)) * D + q] = -w * gt[q];
             }
         }
     }

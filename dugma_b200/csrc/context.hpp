@@ -51,8 +51,9 @@ struct KernelShape {
 
 constexpr int kCounters = 8;      // ints of Context::counter
 constexpr int kInitParts = 256;   // most blocks per cloud of init's statistics
-constexpr int kInitOut = 10;      // scalars init hands to the host: log2 of the largest weights, the CONV
-                                  // scale, det <= 0 and indefinite counts, mean traces, mean squared radii
+constexpr int kInitOut = 11;      // scalars init hands to the host: log2 of the largest weights, the CONV
+                                  // scale, det <= 0 and indefinite counts, mean traces, mean squared radii, largest
+                                  // inverse trace
 
 struct SortedPoint;
 struct Bound;
@@ -73,6 +74,7 @@ struct Context {
     double Lmax_x = 0, Lmax_y = 0;
     double trace_x = 0, trace_y = 0;          // mean covariance trace
     double rho2_x = 0, rho2_y = 0;            // mean squared distance to the cloud's mean
+    float inv_trace = 0;                      // largest trace of a weighted inverse covariance
     double cscale = 1.0;                      // CONV covariances are stored divided by this
     // per-evaluation records
     YRec* yrec = nullptr;
@@ -88,7 +90,8 @@ struct Context {
     double* out = nullptr;                    // 64 doubles of results
     int* err = nullptr;                       // device error word
     int* counter = nullptr;                   // work-queue counters (kCounters: [0] items,
-                                              // [1] blocks done, [2, 3] sigma's integer sum), then hist
+                                              // [1] blocks done, [2, 3] sigma's integer sum, [4] the
+                                              // evaluation is sparse), then hist
     // the clouds in spatial order (spatial.cuh), made by init
     int cell_bits = 0, cells = 0;             // grid bits per axis, cells
     int* hist = nullptr;                      // 2 x cells
@@ -116,6 +119,7 @@ struct Context {
     bool no_alloc = false;                    // scratch is fixed: ensure_scratch fails rather than allocating
     bool fused_coef = true;                   // compi over all rows in one pass (false: one pass per side)
     bool pdl = true;                          // a call's dependent kernels launched early (programmatic dependent launch)
+    bool all_pairs = false;                   // every pair evaluated whatever its exponentials (no sparse.cu)
     int coef_kernel = 0;                      // the one pass: 0 FP32 pipe only (the fastest); 1 source-side
                                               // sums on the tensor cores
     int coef_grid[4] = {0, 0, 0, 0};          // that pass's work grid (SB, groups, chunk tiles, chunks), set on first use
@@ -175,7 +179,21 @@ int launch_pair_variant(Context& c, KernelFn fn, const KernelShape& sh, const vo
                         size_t yrec_size, int nv, double Lmax, const double* pose_dev, int i0, int i1,
                         double* out_dev, double* dEdx_dev, double** h_part, int h_width, int* n_jc_out,
                         cudaStream_t s, const float* w_stationary = nullptr, bool counter_zeroed = false,
-                        double* host_out = nullptr);
+                        double* host_out = nullptr, const int* skip = nullptr);
+// How that launch splits `rows` x `total` streamed records (tiles of sh.tj): tiles per chunk, chunks.
+void pair_split(const Context& c, KernelFn fn, const KernelShape& sh, int rows, size_t yrec_size, int* jc_tiles,
+                int* n_jc);
+// CUDA events around the main pairwise kernel when timing is on (dugma_timing)
+int timing_begin(Context& c, cudaStream_t s);
+int timing_end(Context& c, cudaStream_t s);
+// The REF energy or adjoint over the pairs above the FP32 flush (sparse.cu), from the records of the
+// packed kernels' prologue: the same sums as the all-pairs kernel with tiles of tile_rec and chunks of
+// chunk_rec records.  go (nullable, device): nothing is done unless it is set.
+constexpr double kSparseMinPairs = 4e6, kSparseMinPairsAuto = 64e6;
+constexpr int kSparseMaxTargets = 1 << 20;
+double sparse_sigma(const Context& c);   // evaluations with a sigma below this go that way
+int sparse_launch(Context& c, const double* pose_dev, bool grad, int tile_rec, int chunk_rec, double* out_dev,
+                  double* dEdx_dev, cudaStream_t s, double* host_out, const int* go);
 // Nearest-neighbour prologue: only the target records of the search (c.yp32), y' = R y + t as the
 // full prologue rounds it.  The pose is *pv when given (then also written to pose_dev), else read
 // from pose_dev; reset_counter / reset_err (optional) are zeroed for the kernels that follow.
@@ -188,10 +206,11 @@ int launch_pose_in(Context& c, const double* src, double* pose_dev, cudaStream_t
 // Per-evaluation prologue: y records (layout 0 = adjoint, 1 = Horner energy, 2 / 3 their paired
 // forms), x records in the Cholesky form (xchol, from c.ux) or the Horner form; reset_counter and
 // reset_err (optional) are zeroed for the kernels that follow; the pose is *pv when given (and then
-// also written to pose_out, if given), else read from pose_dev.
+// also written to pose_out, if given), else read from pose_dev.  c.counter[4] is set to sig <
+// sparse_below.
 int launch_prologue(Context& c, const double* pose_dev, int ylayout, cudaStream_t s, bool xchol = false,
                     int* reset_counter = nullptr, const PoseBlock* pv = nullptr, double* pose_out = nullptr,
-                    int* reset_err = nullptr);
+                    int* reset_err = nullptr, double sparse_below = 0.0);
 // Pairwise energy (grad = false) or fused adjoint (grad = true) over source rows [i0, i1);
 // writes {E, g} to out_dev and, if dEdx_dev, dE/dx for rows [i0, i1) (relative index).
 // Options of an evaluation that issues no copy or memset (REF model).  The pose: *pv by value to the
@@ -199,12 +218,13 @@ int launch_prologue(Context& c, const double* pose_dev, int ylayout, cudaStream_
 // staging a captured graph reads at each launch) by a one-block kernel first; either way it is
 // written to pose_out (the device pose block the pair kernel reads) and the error word is zeroed.
 // The results (nv values) and, behind them, the error word are written to host_out (mapped pinned
-// memory) as well.
+// memory) as well.  With sig only, nothing but the choice of kernel changes.
 struct EvalIO {
     const PoseBlock* pv = nullptr;
     const double* pose_src = nullptr;
     double* pose_out = nullptr;
     double* host_out = nullptr;
+    double sig = 0.0;                        // the pose's sigma where the host knows it (else 0)
 };
 int launch_pairs(Context& c, const double* pose_dev, int model, bool grad, int i0, int i1,
                  double* out_dev, double* dEdx_dev, cudaStream_t s, const KernelShape* force = nullptr,

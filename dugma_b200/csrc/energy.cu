@@ -44,9 +44,11 @@ __global__ void __launch_bounds__(NT, MINB) pair_kernel_occ(PairArgs a)
 // host_out (optional, mapped pinned memory) receives out[0..nv) and the error word at [nv]
 __global__ void __launch_bounds__(1024) reduce_items_kernel(const double* __restrict__ part, int n_items, int nv,
                                                              double* __restrict__ out, double* __restrict__ host_out,
-                                                             const int* __restrict__ err)
+                                                             const int* __restrict__ err, const int* skip)
 {
+    pdl_trigger();
     pdl_wait();   // a dependent of the pair kernel: its partials
+    if (skip && *skip) return;
     __shared__ double red[1024];
     const int v = blockIdx.x;
     if (v >= nv) return;
@@ -67,9 +69,12 @@ __global__ void __launch_bounds__(1024) reduce_items_kernel(const double* __rest
     }
 }
 
-__global__ void reduce_chunks_kernel(const double* __restrict__ part, int n_jc, size_t n, double* __restrict__ out)
+__global__ void reduce_chunks_kernel(const double* __restrict__ part, int n_jc, size_t n, double* __restrict__ out,
+                                     const int* skip)
 {
+    pdl_trigger();
     pdl_wait();   // a dependent of the pair kernel (or of reduce_items_kernel after it): its partials
+    if (skip && *skip) return;
     for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < n; e += (size_t)gridDim.x * blockDim.x) {
         double s = 0;
         for (int c = 0; c < n_jc; ++c) s += part[(size_t)c * n + e];
@@ -166,13 +171,9 @@ static int occupancy_blocks(KernelFn fn, int nt)
     return nb;
 }
 
-// Splits [i0, i1) x targets into items and launches `fn`, then the reductions.
-int launch_pair_variant(Context& c, KernelFn fn, const KernelShape& sh, const void* xrec, const void* yrec,
-                        size_t yrec_size, int nv, double Lmax, const double* pose_dev, int i0, int i1,
-                        double* out_dev, double* dEdx_dev, double** h_part, int h_width, int* n_jc_out,
-                        cudaStream_t s, const float* w_stationary, bool counter_zeroed, double* host_out)
+void pair_split(const Context& c, KernelFn fn, const KernelShape& sh, int rows, size_t yrec_size, int* jc_tiles_out,
+                int* n_jc_out)
 {
-    const int rows = i1 - i0;
     const int BI = sh.ipt * sh.nt;
     const int n_ib = (rows + BI - 1) / BI;
     const int total_tiles = (int)(yrec_size / sh.tj);
@@ -186,8 +187,45 @@ int launch_pair_variant(Context& c, KernelFn fn, const KernelShape& sh, const vo
     if (sh.max_chunk > 0) n_jc = std::max(n_jc, (total_tiles * sh.tj + sh.max_chunk - 1) / sh.max_chunk);
     if (sh.min_chunk > 0) n_jc = std::min(n_jc, std::max(1, total_tiles * sh.tj / sh.min_chunk));
     n_jc = std::min(n_jc, total_tiles);
-    const int jc_tiles = (total_tiles + n_jc - 1) / n_jc;
-    n_jc = (total_tiles + jc_tiles - 1) / jc_tiles;
+    *jc_tiles_out = (total_tiles + n_jc - 1) / n_jc;
+    *n_jc_out = (total_tiles + *jc_tiles_out - 1) / *jc_tiles_out;
+}
+
+int timing_begin(Context& c, cudaStream_t s)
+{
+    if (!c.timing) return DUGMA_OK;
+    if (c.tused == c.tevents.size()) {
+        cudaEvent_t e0, e1;
+        DUGMA_CK(cudaEventCreate(&e0));
+        DUGMA_CK(cudaEventCreate(&e1));
+        c.tevents.push_back({e0, e1});
+    }
+    DUGMA_CK(cudaEventRecord(c.tevents[c.tused].first, s));
+    return DUGMA_OK;
+}
+
+int timing_end(Context& c, cudaStream_t s)
+{
+    if (!c.timing) return DUGMA_OK;
+    DUGMA_CK(cudaEventRecord(c.tevents[c.tused].second, s));
+    ++c.tused;
+    return DUGMA_OK;
+}
+
+// Splits [i0, i1) x targets into items and launches `fn`, then the reductions.
+int launch_pair_variant(Context& c, KernelFn fn, const KernelShape& sh, const void* xrec, const void* yrec,
+                        size_t yrec_size, int nv, double Lmax, const double* pose_dev, int i0, int i1,
+                        double* out_dev, double* dEdx_dev, double** h_part, int h_width, int* n_jc_out,
+                        cudaStream_t s, const float* w_stationary, bool counter_zeroed, double* host_out,
+                        const int* skip)
+{
+    const int rows = i1 - i0;
+    const int BI = sh.ipt * sh.nt;
+    const int n_ib = (rows + BI - 1) / BI;
+    const int total_tiles = (int)(yrec_size / sh.tj);
+    const int resident = c.num_sms * occupancy_blocks(fn, sh.nt);
+    int jc_tiles = 0, n_jc = 0;
+    pair_split(c, fn, sh, rows, yrec_size, &jc_tiles, &n_jc);
     const int n_items = n_ib * n_jc;
     size_t need = sizeof(double) * (size_t)n_items * 8;
     const size_t dx_off = need;
@@ -216,32 +254,22 @@ int launch_pair_variant(Context& c, KernelFn fn, const KernelShape& sh, const vo
     a.h_part = h_part ? reinterpret_cast<double*>(reinterpret_cast<char*>(c.scratch) + h_off) : nullptr;
     a.counter = c.counter;
     a.err = c.err;
+    a.skip = skip;
     if (h_part) *h_part = a.h_part;
     if (n_jc_out) *n_jc_out = n_jc;
     if (!counter_zeroed) DUGMA_CK(cudaMemsetAsync(c.counter, 0, sizeof(int), s));
     const int grid = std::min(resident, n_items);
-    cudaEvent_t ev1 = nullptr;
-    if (c.timing) {
-        if (c.tused == c.tevents.size()) {
-            cudaEvent_t e0, e1;
-            DUGMA_CK(cudaEventCreate(&e0));
-            DUGMA_CK(cudaEventCreate(&e1));
-            c.tevents.push_back({e0, e1});
-        }
-        DUGMA_CK(cudaEventRecord(c.tevents[c.tused].first, s));
-        ev1 = c.tevents[c.tused].second;
-        ++c.tused;
-    }
+    DUGMA_RET(timing_begin(c, s));
     DUGMA_CK(launch_dependent(c.pdl, fn, grid, sh.nt, 0, s, a));
-    if (ev1) DUGMA_CK(cudaEventRecord(ev1, s));
+    DUGMA_RET(timing_end(c, s));
     if (out_dev)
         DUGMA_CK(launch_dependent(c.pdl, reduce_items_kernel, nv, 1024, 0, s, (const double*)a.partials, n_items, nv,
-                                  out_dev, host_out, (const int*)c.err));
+                                  out_dev, host_out, (const int*)c.err, skip));
     if (dEdx_dev) {
         const size_t n = (size_t)rows * c.D;
         const int g = (int)std::min<size_t>((n + 255) / 256, (size_t)c.num_sms * 8);
         DUGMA_CK(launch_dependent(c.pdl, reduce_chunks_kernel, g, 256, 0, s, (const double*)a.dx_part, n_jc, n,
-                                  dEdx_dev));
+                                  dEdx_dev, skip));
     }
     return DUGMA_OK;
 }
@@ -276,15 +304,36 @@ int launch_pairs(Context& c, const double* pose_dev, int model, bool grad, int i
     const int layout = (grad ? 0 : 1) + (v->shape.pack == 2 ? 2 : 0);
     if (io && (io->pv || io->pose_src) && !io->pose_out)
         return set_error(DUGMA_ERR_ARG, "a pose by value or from host memory needs a device pose block");
+    // All rows by the packed kernels and a sigma that leaves most pairs under the FP32 flush: only
+    // the others (sparse.cu).  Where only the device knows sigma (a pose in device memory, a captured
+    // graph) both ways are enqueued and the prologue's flag lets one of them run; that costs an
+    // all-pairs evaluation two launches that return at once, so it takes kSparseMinPairsAuto pairs.
+    const double below = !force && xchol && i0 == 0 && i1 == c.N ? sparse_sigma(c) : 0.0;
+    const double sig = io ? (io->pv ? io->pv->v[kPoseSig] : io->sig) : 0.0;
+    const bool known = sig > 0.0;
+    const bool both = !known && below > 0.0 && (double)c.N * c.M >= kSparseMinPairsAuto;
+    const bool sparse = known && sig < below;
     if (io && io->pose_src) DUGMA_RET(launch_pose_in(c, io->pose_src, io->pose_out, s, true));
     const double* pose_read = io && io->pose_src ? io->pose_out : pose_dev;
     DUGMA_RET(launch_prologue(c, pose_read, layout, s, xchol, c.counter, io ? io->pv : nullptr,
-                              io ? io->pose_out : nullptr, io && io->pv ? c.err : nullptr));
+                              io ? io->pose_out : nullptr, io && io->pv ? c.err : nullptr, both ? below : 0.0));
     const int nv = grad ? 1 + (c.D == 3 ? 6 : 3) : 1;
-    return launch_pair_variant(c, v->fn, v->shape, c.xrec, c.yrec, (size_t)c.M_pad / v->shape.pack, nv, c.Lmax_y,
-                               io && io->pose_out ? io->pose_out : pose_dev, i0, i1, out_dev,
-                               grad ? dEdx_dev : nullptr, nullptr, 0, nullptr, s, nullptr, true,
-                               io ? io->host_out : nullptr);
+    const double* pose = io && io->pose_out ? io->pose_out : pose_dev;
+    double* host_out = io ? io->host_out : nullptr;
+    const int* flag = both ? c.counter + 4 : nullptr;
+    if (!sparse)
+        DUGMA_RET(launch_pair_variant(c, v->fn, v->shape, c.xrec, c.yrec, (size_t)c.M_pad / v->shape.pack, nv, c.Lmax_y,
+                                      pose, i0, i1, out_dev, grad ? dEdx_dev : nullptr, nullptr, 0, nullptr, s, nullptr,
+                                      true, host_out, flag));
+    if (sparse || both) {
+        int jc_tiles = 0, n_jc = 0;
+        pair_split(c, v->fn, v->shape, c.N, (size_t)c.M_pad / 2, &jc_tiles, &n_jc);
+        // (the energy's sums end with each tile: its chunks are only a split of the work)
+        const int chunk = grad ? jc_tiles * v->shape.tj : 512;
+        DUGMA_RET(sparse_launch(c, pose, grad, v->shape.tj, chunk, out_dev, grad ? dEdx_dev : nullptr, s, host_out,
+                                flag));
+    }
+    return DUGMA_OK;
 }
 
 // ---------------------------------------------------------------------------

@@ -33,6 +33,7 @@ struct PairArgs {
     double* h_part;        // coefficient passes: [n_jc][rows][16] or nullptr
     int* counter;
     int* err;
+    const int* skip;       // nullable: when set, the kernel returns at once
 };
 
 // Bodies with a fold_tile(tile, first record index, records) member finish each tile with the
@@ -61,6 +62,7 @@ __device__ __forceinline__ void run_pairs(const PairArgs& a, Body& body)
     // let them be scheduled, then wait for the prologue's records, pose and zeroed counter
     pdl_trigger();
     pdl_wait();
+    if (a.skip && *a.skip) return;
     const int tid = threadIdx.x;
     if (tid == 0) {
 #pragma unroll

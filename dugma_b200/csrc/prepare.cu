@@ -43,7 +43,7 @@ struct InitArgs {
     double* part;          // [2][kInitParts][5] partial sums
     int nb, bits;
     int* counter;          // [0] det <= 0, [2 + cloud] largest weight (float bits), [4 + cloud] weighted
-                           // points without a Cholesky factor
+                           // points without a Cholesky factor, [6] largest trace of an inverse covariance
     double *out, *host;    // kInitOut scalars for the host (host: nullable, mapped)
 };
 
@@ -179,7 +179,7 @@ __global__ void __launch_bounds__(256) init_points_kernel(InitArgs ia)
     const double inv_scale = 1.0 / conv_scale(ia, tot, D);
     float lo[3];
     const float inv = cell_grid(tot[blockIdx.y], n, D, ia.bits, lo);
-    int wmax = 0;
+    int wmax = 0, tmax = 0;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         float pf[D];
 #pragma unroll
@@ -236,7 +236,13 @@ __global__ void __launch_bounds__(256) init_points_kernel(InitArgs ia)
         for (int k = 0; k < D * D; ++k) cl.cinv[(size_t)i * D * D + k] = o[k];
         w[i] = wi;
         // positive floats order like their bit patterns
-        if (wi > 0.0f) wmax = max(wmax, __float_as_int(wi));
+        if (wi > 0.0f) {
+            float tr = 0.f;
+#pragma unroll
+            for (int a = 0; a < D; ++a) tr += fabsf(o[a * (D + 1)]);
+            wmax = max(wmax, __float_as_int(wi));
+            tmax = max(tmax, __float_as_int(tr));
+        }
         double pk[NS], u[NS];
 #pragma unroll
         for (int k = 0; k < NS; ++k) {
@@ -255,7 +261,11 @@ __global__ void __launch_bounds__(256) init_points_kernel(InitArgs ia)
     // the largest weight (order-independent, so deterministic); log2 is monotonic, so log2 of the
     // largest weight is the largest log2
     wmax = __reduce_max_sync(0xffffffffu, wmax);
-    if ((threadIdx.x & 31) == 0 && wmax > 0) atomicMax(ia.counter + 2 + blockIdx.y, wmax);
+    tmax = __reduce_max_sync(0xffffffffu, tmax);
+    if ((threadIdx.x & 31) == 0 && wmax > 0) {
+        atomicMax(ia.counter + 2 + blockIdx.y, wmax);
+        atomicMax(ia.counter + 6, tmax);
+    }
 }
 
 // hist[c] <- the points in the cells before c; one block of 1024 threads per cloud
@@ -315,7 +325,8 @@ __global__ void sort_points_kernel(InitArgs ia)
         s.p[2] = 0.f;
 #pragma unroll
         for (int a = 0; a < D; ++a) s.p[a] = c.p32[(size_t)i * D + a];
-        s.a = fmaxf(lw + kFlushExp, -1.f);
+        // (the source's weight is no part of the exponent)
+        s.a = blockIdx.y == 0 ? (lw > -INFINITY ? kFlushExp : -1.f) : fmaxf(lw + kFlushExp, -1.f);
         s.L = c.L[i];
         s.idx = i;
         s.pad[0] = s.pad[1] = 0.f;
@@ -511,8 +522,10 @@ __global__ void __launch_bounds__(1024) bounds_kernel(InitArgs ia)
                 v = (double)ia.counter[q == 3 ? 0 : q];
             } else if (q < 8) {
                 v = tot[q - 6][0] / ia.cl[q - 6].n;   // mean covariance trace
-            } else {
+            } else if (q < 10) {
                 v = mean_radius2(tot[q - 8], ia.cl[q - 8].n, D);
+            } else {
+                v = (double)__int_as_float(ia.counter[6]);
             }
             ia.out[q] = v;
             if (ia.host) ia.host[q] = v;
@@ -585,6 +598,7 @@ int launch_init(Context& c, const double* X, const double* XC, const double* Y, 
     c.trace_y = c.host[7];
     c.rho2_x = c.host[8];
     c.rho2_y = c.host[9];
+    c.inv_trace = (float)c.host[10];
     return DUGMA_OK;
 }
 
@@ -650,14 +664,18 @@ __global__ void prologue_kernel(const double* __restrict__ pose, const float* __
                                 const float* __restrict__ x, const float* __restrict__ xinv,
                                 const float* __restrict__ lwx, int N, int N_pad, XRec* __restrict__ xrec,
                                 const double* __restrict__ ux, int* __restrict__ reset_counter, const PoseBlock pv,
-                                int use_pv, double* __restrict__ pose_out, int* __restrict__ reset_err)
+                                int use_pv, double* __restrict__ pose_out, int* __restrict__ reset_err,
+                                double sparse_below)
 {
     pdl_trigger();   // the pair kernel may be scheduled now; it waits for this kernel's writes
     constexpr int NS = Sym<D>::N;
     // the pose pv by value (use_pv; block 0 also writes it to pose_out, if given, for the kernels
     // that follow) or from pose
     if (blockIdx.x == 0 && threadIdx.x == 0) {
-        if (reset_counter) *reset_counter = 0;
+        if (reset_counter) {
+            reset_counter[0] = reset_counter[1] = 0;
+            reset_counter[4] = (use_pv ? pv.v[kPoseSig] : pose[kPoseSig]) < sparse_below;
+        }
         if (reset_err) *reset_err = 0;
         if (use_pv && pose_out)
 #pragma unroll
@@ -853,7 +871,7 @@ int launch_nn_prologue(Context& c, double* pose_dev, cudaStream_t s, const PoseB
 }
 
 int launch_prologue(Context& c, const double* pose_dev, int ylayout, cudaStream_t s, bool xchol, int* reset_counter,
-                    const PoseBlock* pv, double* pose_out, int* reset_err)
+                    const PoseBlock* pv, double* pose_out, int* reset_err, double sparse_below)
 {
     PoseBlock pb{};
     if (pv) pb = *pv;
@@ -866,11 +884,11 @@ int launch_prologue(Context& c, const double* pose_dev, int ylayout, cudaStream_
     if (c.D == 3)
         prologue_kernel<3><<<g, bs, 0, s>>>(pose_dev, c.y, c.yinv, c.lwy, c.M, c.M_pad, ylayout, c.yrec, nullptr,
                                             c.x, c.xinv, c.lwx, c.N, c.N_pad, c.xrec, ux, reset_counter, pb,
-                                            pv ? 1 : 0, pose_out, reset_err);
+                                            pv ? 1 : 0, pose_out, reset_err, sparse_below);
     else
         prologue_kernel<2><<<g, bs, 0, s>>>(pose_dev, c.y, c.yinv, c.lwy, c.M, c.M_pad, ylayout, c.yrec, nullptr,
                                             c.x, c.xinv, c.lwx, c.N, c.N_pad, c.xrec, ux, reset_counter, pb,
-                                            pv ? 1 : 0, pose_out, reset_err);
+                                            pv ? 1 : 0, pose_out, reset_err, sparse_below);
     DUGMA_CK(cudaGetLastError());
     return DUGMA_OK;
 }

@@ -1,0 +1,218 @@
+// reach.cuh -- which streamed points can reach a group of stationary ones.
+//
+// A pair's two terms are 2^(lv_j - |k| d^T C'_j d) and 2^(lv_j - |k| d^T B_i d), and ex2.approx.ftz
+// flushes a result below 2^-126 to 0.  With L a bound on the largest variance behind either matrix
+// (SortedPoint::L, x sig), both exponents are at most lv_j - |k| |d|^2 / (sig max(L_i, L_j)), so a pair with
+//     |d|^2 > (sig / |k|) a_j max(L_i, L_j),     a_j = lv_j + 127.5
+// adds exactly +0 to every sum the kernels keep, and leaving it out changes no bit.
+//
+// find_reach marks, for one tile of 32 stationary points, the records (pairs of streamed points by
+// index) of which a point passes that test for some stationary point: super tiles against the
+// tile's four subgroups, tiles against them, points against them, then points against points.  The
+// tests run in FP32 with room for their rounding, for that of the evaluation (in L, see variance_bound)
+// and for what a pose that is no exact rotation stretches.  What is not finite, or so large that the
+// evaluation could overflow, is marked.
+#pragma once
+
+#include "spatial.cuh"
+
+namespace dugma {
+
+struct ReachSide {
+    const SortedPoint* pt;
+    const Bound *tile, *sub, *super;
+    int n;
+};
+
+struct ReachArgs {
+    ReachSide st, sm;      // stationary, streamed
+    const double* pose;
+    float inv_trace;       // largest trace of an inverse covariance (overflow limit)
+};
+
+// one block of 4 warps
+struct ReachShared {
+    float4 pt[kTile];      // position, L
+    float2 pa[kTile];      // a, slack
+    float4 sub[4];         // centre, radius
+    float2 sa[4];          // a, L
+};
+
+// R y + t in FP32 (stretch, Lscale: how much R can stretch a length and a variance)
+struct PoseF {
+    float R[9], t[3], tsize;
+    float stretch, Lscale;
+};
+
+template <int D>
+__device__ __forceinline__ PoseF pose_f32(const double* pose)
+{
+    PoseF p;
+    double f = 0;
+    p.tsize = 0.f;
+#pragma unroll
+    for (int a = 0; a < D; ++a) {
+#pragma unroll
+        for (int b = 0; b < D; ++b) {
+            double v = a == b ? -1.0 : 0.0;
+#pragma unroll
+            for (int k = 0; k < D; ++k) v = fma(pose[k + D * a], pose[k + D * b], v);
+            f = fma(v, v, f);
+            p.R[a + D * b] = (float)pose[a + D * b];
+        }
+        p.t[a] = (float)pose[kPoseT + a];
+        p.tsize += fabsf(p.t[a]);
+    }
+    // |R v| lies between sqrt(1 - dev) |v| and sqrt(1 + dev) |v|
+    const float dev = sqrtf((float)f) * (1.f + 1e-6f);
+    p.stretch = sqrtf(1.f + dev) * (1.f + 1e-6f);
+    p.Lscale = dev < 0.5f ? (1.f + 1e-6f) / (1.f - dev) : INFINITY;
+    return p;
+}
+
+// position and, in w, the size its rounding error scales with
+template <int D>
+__device__ __forceinline__ float4 move_f32(const PoseF& p, const float* y)
+{
+    float v[3] = {0.f, 0.f, 0.f};
+    float size = p.tsize;
+#pragma unroll
+    for (int a = 0; a < D; ++a) {
+        float s = p.t[a];
+#pragma unroll
+        for (int k = 0; k < D; ++k) s = fmaf(p.R[a + D * k], y[k], s);
+        v[a] = s;
+        size += fabsf(s) + fabsf(y[a]);
+    }
+    return make_float4(v[0], v[1], v[2], size);
+}
+
+template <int D>
+__device__ __forceinline__ float dist2_f32(const float4& p, const float4& q)
+{
+    const float dx = p.x - q.x, dy = p.y - q.y;
+    float d = fmaf(dy, dy, dx * dx);
+    if (D == 3) {
+        const float dz = p.z - q.z;
+        d = fmaf(dz, dz, d);
+    }
+    return d;
+}
+
+// The records that reach tile `group` of the stationary side, into bits (shared, one per record; all
+// 128 threads; the caller zeroes bits before and synchronises after).  POSE_SM: the streamed side is
+// the targets' (moved by the pose), else the stationary side is.
+template <int D, bool POSE_SM>
+__device__ __forceinline__ void find_reach(const ReachArgs& a, int group, uint32_t* bits, ReachShared& sh)
+{
+    constexpr int NW = 4, TPW = kSuper / NW;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const PoseF P = pose_f32<D>(a.pose);
+    const float sigk = (float)(a.pose[kPoseSig] * (1.0 / -K_EXP2)) * (1.f + 1e-6f);
+    // beyond this squared distance a form could overflow, and 0 x inf is no 0
+    const float d2max = fminf(1e36f * sigk / (a.inv_trace + 1e-30f), 1e30f);
+    // a sphere or point as the tests see it
+    auto place = [&](const float* c, float& r, bool posed) {
+        float4 q = make_float4(c[0], c[1], D == 3 ? c[2] : 0.f, 0.f);
+        if (posed) {
+            q = move_f32<D>(P, c);
+            r = fmaf(r, P.stretch, 1e-6f * q.w);
+        }
+        return q;
+    };
+    if (threadIdx.x < kTile) {
+        const int i = group * kTile + lane;
+        SortedPoint s = a.st.pt[i < a.st.n ? i : 0];
+        float slack = 0.f;
+        float4 q = place(s.p, slack, !POSE_SM);
+        q.w = POSE_SM ? s.L : s.L * P.Lscale;
+        sh.pt[lane] = q;
+        // a lane without a point, and a point without weight (a = -1), reaches nothing
+        sh.pa[lane] = make_float2(i < a.st.n ? s.a : -1.f, 1001.f * slack * slack);
+    } else if (threadIdx.x < kTile + 4) {
+        const Bound b = a.st.sub[4 * group + lane];
+        float r = b.r;
+        float4 q = place(b.c, r, !POSE_SM);
+        q.w = r;
+        sh.sub[lane] = q;
+        sh.sa[lane] = make_float2(b.a, POSE_SM ? b.L : b.L * P.Lscale);
+    }
+    __syncthreads();
+    // can something at q (radius r, a, L) reach a point of the subgroups?  one bit each
+    auto subs = [&](const float4& q, float r, float aa, float L) {
+        unsigned m = 0;
+#pragma unroll
+        for (int s = 0; s < 4; ++s) {
+            const float4 c = sh.sub[s];
+            const float2 e = sh.sa[s];
+            const float T = sigk * fminf(aa, e.x) * fmaxf(L, e.y);
+            const float rr = r + c.w, reach = fmaf(sqrt_fast(fmaxf(T, 0.f)), 1.f + 2e-6f, rr);
+            const float d2 = dist2_f32<D>(q, c);
+            const bool out = d2 * (1.f - 1e-5f) > reach * reach && d2 < 0.2f * d2max && rr * rr < 0.2f * d2max;
+            m |= (unsigned)!out << s;
+        }
+        return m;
+    };
+    const int n_tiles = (a.sm.n + kTile - 1) / kTile, n_super = (n_tiles + kSuper - 1) / kSuper;
+    for (int base = 0; base < n_super; base += 32) {
+        bool go = base + lane < n_super;
+        if (go) {
+            const Bound b = a.sm.super[base + lane];
+            float r = b.r;
+            const float4 q = place(b.c, r, POSE_SM);
+            go = subs(q, r, b.a, POSE_SM ? b.L * P.Lscale : b.L) != 0;
+        }
+        unsigned mask = __ballot_sync(0xffffffffu, go);
+        while (mask) {   // the warp's tiles of up to NW super tiles at a time
+            int mine = -1;
+#pragma unroll
+            for (int k = 0; k < NW; ++k) {
+                const int bit = __ffs(mask) - 1;   // -1: none left
+                mask &= mask - 1;
+                if (k == lane / TPW) mine = bit;
+            }
+            const int t = (base + mine) * kSuper + (lane % TPW) * NW + warp;
+            go = mine >= 0 && t < n_tiles;
+            if (go) {
+                const Bound b = a.sm.tile[t];
+                float r = b.r;
+                const float4 q = place(b.c, r, POSE_SM);
+                go = subs(q, r, b.a, POSE_SM ? b.L * P.Lscale : b.L) != 0;
+            }
+            unsigned todo = __ballot_sync(0xffffffffu, go);
+            while (todo) {   // lane = point of the tile
+                const int from = __ffs(todo) - 1;
+                todo &= todo - 1;
+                const int j = __shfl_sync(0xffffffffu, t, from) * kTile + lane;
+                unsigned m = 0;
+                SortedPoint s;
+                float4 q = make_float4(0.f, 0.f, 0.f, 0.f);
+                float L = 0.f, slack = 0.f;
+                if (j < a.sm.n) {
+                    s = a.sm.pt[j];
+                    q = place(s.p, slack, POSE_SM);
+                    L = POSE_SM ? s.L * P.Lscale : s.L;
+                    m = subs(q, slack, s.a, L);
+                    slack = 1001.f * slack * slack;
+                }
+                bool hit = false;
+#pragma unroll
+                for (int g = 0; g < 4; ++g) {
+                    if (!__any_sync(0xffffffffu, m >> g & 1u)) continue;
+#pragma unroll
+                    for (int e = 0; e < kSub; ++e) {
+                        const float4 c = sh.pt[g * kSub + e];
+                        const float2 ca = sh.pa[g * kSub + e];
+                        const float T = sigk * fminf(s.a, ca.x) * fmaxf(L, c.w);
+                        const float d2 = dist2_f32<D>(q, c);
+                        // (d - slack)^2 > T follows from d^2 > 1.001 T + 1001 slack^2
+                        hit |= (m >> g & 1u) && !(d2 > fmaf(T, 1.002f, slack + ca.y) && d2 < d2max);
+                    }
+                }
+                if (hit) atomicOr(&bits[s.idx >> 6], 1u << (s.idx >> 1 & 31));
+            }
+        }
+    }
+}
+
+}  // namespace dugma

@@ -1,0 +1,90 @@
+"""Evaluations over the pairs above the FP32 flush against all pairs (DUGMA_ALL_PAIRS=1 at init):
+the same FP32 terms and sums, so equal to the rounding of FP64 additions (1e-12 of the result; a
+gradient's sums cancel by less than 1e3 here), on clouds whose covariances follow the spacing, with
+outliers, ill-conditioned and neglected covariances, coincident and far points, poses that are no
+rotation, and points that are not finite or near overflow."""
+import numpy as np
+import pytest
+
+from dugma_b200 import api, synth
+
+pytestmark = pytest.mark.gpu
+
+
+def _problem(kind, n, m, seed):
+    rng = np.random.default_rng(seed)
+    k = max(n, m)
+    if kind == "curve":
+        P = synth.workload5(trial=seed, n=k)
+    elif kind == "outliers":
+        P = synth.workload1(trial=seed, n=k)
+    elif kind == "harmonic":
+        P = synth.workload2(trial=seed, n=k)
+    else:
+        P = synth.workload0(trial=seed, n=k)
+    i, j = rng.permutation(k)[:n], rng.permutation(k)[:m]
+    X, XC, Y, YC = P.X[i].copy(), P.X_C[i].copy(), P.Y[j].copy(), P.Y_C[j].copy()
+    D = X.shape[1]
+    if kind == "neglected":
+        XC[::7] = 0.0
+        YC[::5, 0, 0] *= -1.0
+    elif kind == "coincident":
+        X[: n // 2] = X[0]
+        Y[: m // 3] = (X[0] - P.t_G) @ P.R_G      # R_G^T (x - t)
+    elif kind == "far":
+        Y[m // 2:] += 1e3
+        X[0] = -1e4
+    elif kind == "mixed_scales":
+        XC *= np.exp(rng.uniform(-4, 4, n))[:, None, None]
+        YC *= np.exp(rng.uniform(-4, 4, m))[:, None, None]
+    elif kind == "not_finite":
+        Y[3, 0] = np.inf
+    elif kind == "huge":
+        Y[5] = 3e18
+        XC[0] = 1e-18 * np.eye(D)
+    return X, XC, Y, YC, P.R_G, P.t_G
+
+
+def _evaluate(monkeypatch, prob, R, t, sig, all_pairs):
+    if all_pairs:
+        monkeypatch.setenv("DUGMA_ALL_PAIRS", "1")
+    else:
+        monkeypatch.delenv("DUGMA_ALL_PAIRS", raising=False)
+    _, h = api.init(*prob[:4])
+    out = {}
+    try:
+        for name, fn in (("grad", lambda: api.energy_grad(h, R, t, sig)[:2]),
+                         ("grad_dx", lambda: api.energy_grad(h, R, t, sig, with_dx=True)),
+                         ("energy", lambda: (api.energy(h, R, t, sig),)),
+                         ("fd", lambda: (api.energy_fd_grad(h, R, t, sig)[0],))):
+            try:
+                out[name] = [np.asarray(v) for v in fn()]
+            except api.DugmaError as e:
+                out[name] = e.code
+    finally:
+        api.fr_m(h)
+    return out
+
+
+KINDS = ["sphere", "outliers", "harmonic", "curve", "neglected", "coincident", "far", "mixed_scales", "not_finite",
+         "huge"]
+
+
+@pytest.mark.filterwarnings("ignore")
+@pytest.mark.parametrize("n,m", [(2049, 2001), (5000, 901), (1025, 4097)])
+@pytest.mark.parametrize("kind", KINDS)
+def test_same_sums_as_all_pairs(kind, n, m, monkeypatch):
+    prob = _problem(kind, n, m, 3)
+    R, t = prob[4], prob[5]
+    for scale in (1.0, 1.05):        # a rotation, and a matrix that stretches
+        for sig in (2e-4, 4e-3, 3e-2):
+            a = _evaluate(monkeypatch, prob, scale * R, t + 0.01, sig, False)
+            b = _evaluate(monkeypatch, prob, scale * R, t + 0.01, sig, True)
+            for name in b:
+                if isinstance(b[name], int) or isinstance(a[name], int):
+                    assert isinstance(b[name], int) and a[name] == b[name], (name, a[name], b[name])
+                    continue
+                for u, v in zip(a[name], b[name]):
+                    assert np.all(np.isfinite(u) == np.isfinite(v)), name
+                    u, v = u[np.isfinite(u)], v[np.isfinite(v)]
+                    assert np.linalg.norm(u - v) <= 1e-12 * np.linalg.norm(v), (name, sig, u, v)
