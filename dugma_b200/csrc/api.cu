@@ -445,7 +445,8 @@ int dugma_init(const double* X, const double* X_C, const double* Y, const double
     const int nxt = (N + kTile - 1) / kTile, nyt = (M + kTile - 1) / kTile;
     const int nxs = (nxt + kSuper - 1) / kSuper, nys = (nyt + kSuper - 1) / kSuper;
     const size_t staging = sizeof(double) * ((size_t)N * D * (D + 1) + (size_t)M * D * (D + 1));
-    const size_t scratch_bytes = std::max(staging, (size_t)4 << 20);
+    // (at least what the sparse coefficient pass's rows take)
+    const size_t scratch_bytes = std::max({staging, (size_t)4 << 20, sizeof(double) * 16 * ((size_t)N + M)});
     struct Slot {
         void** p;
         size_t bytes;

@@ -17,6 +17,7 @@
 #include "coef_map.h"
 #include "context.hpp"
 #include "pairs.cuh"
+#include "reach.cuh"
 #include "umma.cuh"
 
 namespace dugma {
@@ -62,7 +63,8 @@ __device__ __forceinline__ void write_pair_half(Rec256* __restrict__ out, int j,
 // ---------------------------------------------------------------------------
 // One thread per point: indices [0, M_pad) are the targets, [M_pad, M_pad + N_pad) the sources.
 // The pose is pv when use_pv (block 0 then writes it to `pose` for the kernels that follow), else
-// read from `pose`.  reset_counter and reset_err (each optional) are zeroed for those kernels.
+// read from `pose`.  reset_counter and reset_err (each optional) are zeroed for those kernels, and
+// reset_counter[4] set to sig < sparse_below.
 // CHOL: each matrix as the upper Cholesky factor U' of |k| B (U'^T U' = |k| B; the sources' from
 // init's FP64 factor ux of sym(Sigma_x^-1), the targets' of C'_j in FP64 here), so that an exponent is
 // lv - |U' d|^2, a sum of squares whose FP32 rounding grows with sqrt(cond B) instead of cond B; the
@@ -74,12 +76,16 @@ __global__ void coef_prologue_kernel(const PoseBlock pv, int use_pv, double* __r
                                      Rec128* __restrict__ yr, Rec256* __restrict__ yr2, const float* __restrict__ x,
                                      const float* __restrict__ xinv, const float* __restrict__ lwx, int N, int N_pad,
                                      Rec128* __restrict__ xr, Rec256* __restrict__ xr2, int* __restrict__ reset_counter,
-                                     int* __restrict__ reset_err, const double* __restrict__ ux)
+                                     int* __restrict__ reset_err, const double* __restrict__ ux,
+                                     const float* __restrict__ wx, double Lmax_x, double sparse_below)
 {
     pdl_trigger();   // the one-pass kernel may be scheduled now; it waits for this kernel's writes
     constexpr int NS = Sym<D>::N, NF = Feat<D>::N;
     if (blockIdx.x == 0 && threadIdx.x == 0) {
-        if (reset_counter) *reset_counter = 0;
+        if (reset_counter) {
+            *reset_counter = 0;
+            reset_counter[4] = (use_pv ? pv.v[kPoseSig] : pose[kPoseSig]) < sparse_below;
+        }
         if (reset_err) *reset_err = 0;
         if (use_pv)
 #pragma unroll
@@ -125,6 +131,11 @@ __global__ void coef_prologue_kernel(const PoseBlock pv, int use_pv, double* __r
             r.v3 = D == 3 ? make_float4(bp[4], bp[5], 0.f, 0.f) : make_float4(0.f, 0.f, 0.f, 0.f);
             for (int q = 0; q < 16; ++q) r.g[q] = q < NF ? __double2float_rn(f[q]) : 0.f;
             xr[i] = r;
+            // for the sparse pass the pairs carry fw = (w / 2^Lmax_x) f(x), as the one pass forms it
+            if (wx) {
+                const double ws = i < N ? (double)wx[i] * exp2(-Lmax_x) : 0.0;
+                for (int q = 0; q < NF; ++q) r.g[q] = __double2float_rn(ws * (double)r.g[q]);
+            }
             write_pair_half(xr2, i, r);
             continue;
         }
@@ -361,6 +372,7 @@ struct FusedCoefArgs {
     double* h1_part;       // [n_grp][M][16]
     int* counter;
     int* err;
+    const int* skip;       // nullable: when set, the kernel returns at once
 };
 
 template <int D>
@@ -401,6 +413,7 @@ __global__ void __launch_bounds__(128, 3) coef_fused_kernel(FusedCoefArgs a)
     // kernel a dependent of this one
     pdl_trigger();
     pdl_wait();
+    if (a.skip && *a.skip) return;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     if (tid == 0) {
         for (int st = 0; st < STAGES; ++st) mbar_init(&bars[st], 1);
@@ -589,6 +602,222 @@ __global__ void __launch_bounds__(128, 3) coef_fused_kernel(FusedCoefArgs a)
             }
         }
     }
+}
+
+// ---------------------------------------------------------------------------
+// The moments' sums over the pairs above the FP32 flush (reach.cuh, as sparse.cu does the energy): a
+// block takes one tile of 32 sources (blockIdx.x < n_st0) against the targets, or one of 32 targets
+// against the sources, marks the records that can reach it and sums those alone:
+//   side 0 (lane = source)  H2 += p g_j per target record, FP32 over the same runs of records that the one
+//                           pass folds (FOLD tiles from each chunk's start), FP64 across them;
+//   side 1 (lane = target)  T += p fw_i per source pair, the even and odd sources' sums of each 64
+//                           sources, the four 64s of a source block, then FP64 across blocks: the
+//                           order of the one pass's phase 2.
+// Each p is formed twice, by the same operations on the same records (with d negated on side 1,
+// which no form's value depends on), and what is left out adds exact zeros, so the sums are the one
+// pass's up to the rounding of their FP64 additions, in one copy per side instead of one per chunk
+// and group.  Bound like sparse_kernel by the search for the records.  Measured on one B200, harmonic
+// surface 16384 x 15000: the one pass 505 us and its copies' moments 36 us, here 35 and 14 us (compi
+// 614 -> 89 us a call).
+// ---------------------------------------------------------------------------
+struct CoefSparseArgs {
+    ReachSide x, y;
+    float inv_trace;
+    const double* pose;
+    const Rec128 *xrec, *yrec;     // by index
+    const Rec256 *xpair, *ypair;   // pairs: fw behind the sources, monomials behind the targets
+    const float* wx;
+    double Lmax_x, Lmax_y;
+    int n_st0;                     // source tiles
+    int n_rec[2], words[2];        // streamed records of side 0 (targets), side 1 (sources)
+    int jc_tiles, total_tiles, runs_per_chunk, n_units[2];
+    double *h2, *h1;               // [N][16], [M][16]
+    const int* go;                 // nullable: nothing is done unless set
+};
+
+struct CoefSparseShape {
+    static constexpr int BATCH = 4, UNITS = 16;   // records loaded together; units listed together per warp
+    static constexpr size_t kRec = 4 * 2 * BATCH * sizeof(Rec256), kList = 4 * UNITS * 64 * sizeof(uint16_t),
+                            kSums = 4 * 10 * 32 * sizeof(double);
+    static constexpr size_t kFixed = (sizeof(ReachShared) + 15) / 16 * 16 + kRec + kList + kSums;
+};
+
+template <int D, int SIDE>
+__device__ __forceinline__ void coef_sparse_side(const CoefSparseArgs& a, int group, unsigned char* smem)
+{
+    using S = CoefSparseShape;
+    constexpr int NF = Feat<D>::N, NS = Sym<D>::N;
+    ReachShared& sh = *reinterpret_cast<ReachShared*>(smem);
+    unsigned char* work = smem + (sizeof(ReachShared) + 15) / 16 * 16;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    float2(*rec)[S::BATCH * 32] = reinterpret_cast<float2(*)[S::BATCH * 32]>(work) + 2 * warp;
+    uint16_t* list = reinterpret_cast<uint16_t*>(work + S::kRec) + S::UNITS * 64 * warp;
+    double(*sums)[10][32] = reinterpret_cast<double(*)[10][32]>(work + S::kRec + S::kList);
+    uint32_t* bits = reinterpret_cast<uint32_t*>(work + S::kRec + S::kList + S::kSums);
+    {
+        ReachArgs r;
+        r.st = SIDE == 0 ? a.x : a.y;
+        r.sm = SIDE == 0 ? a.y : a.x;
+        r.pose = a.pose;
+        r.inv_trace = a.inv_trace;
+        find_reach<D, SIDE == 0>(r, group, bits, sh);
+    }
+    __syncthreads();
+    const ReachSide& st = SIDE == 0 ? a.x : a.y;
+    const int pos = group * kTile + lane;
+    const bool in = pos < st.n;
+    const int i = in ? st.pt[pos].idx : 0;
+    float2 PH[3], PL[3], Mx[6], lvs, h[NF];
+    {
+        const Rec128 r = (SIDE == 0 ? a.xrec : a.yrec)[i];
+        const float hv[3] = {r.v0.x, r.v0.y, r.v0.z}, lo[3] = {r.v1.x, r.v1.y, r.v1.z};
+        const float mv[6] = {r.v2.x, r.v2.y, r.v2.z, r.v2.w, r.v3.x, r.v3.y};
+#pragma unroll
+        for (int q = 0; q < D; ++q) {
+            PH[q] = make_float2(hv[q], hv[q]);
+            PL[q] = make_float2(lo[q], lo[q]);
+        }
+#pragma unroll
+        for (int q = 0; q < NS; ++q) Mx[q] = make_float2(mv[q], mv[q]);
+        lvs = make_float2(r.v0.w, r.v0.w);
+    }
+#pragma unroll
+    for (int q = 0; q < NF; ++q) {
+        h[q] = make_float2(0.f, 0.f);
+        sums[warp][q][lane] = 0.0;
+    }
+    float T[NF];   // side 1: the source block's sums so far
+#pragma unroll
+    for (int q = 0; q < NF; ++q) T[q] = 0.f;
+    // the end of a unit (side 0: a run; side 1: 64 sources, `last` of their block)
+    auto fold = [&](bool last) {
+#pragma unroll
+        for (int q = 0; q < NF; ++q) {
+            if (SIDE == 0) {
+                sums[warp][q][lane] += (double)h[q].x + (double)h[q].y;
+            } else {
+                T[q] += h[q].x + h[q].y;
+                if (last) {
+                    sums[warp][q][lane] += (double)T[q];
+                    T[q] = 0.f;
+                }
+            }
+            h[q] = make_float2(0.f, 0.f);
+        }
+    };
+    const float2* recs = reinterpret_cast<const float2*>(SIDE == 0 ? a.ypair : a.xpair);
+    const int n_units = a.n_units[SIDE];
+    // 64 units at a time, 16 of them this warp's (side 1: four blocks of four units)
+    for (int ubase = 0; ubase < n_units; ubase += 4 * S::UNITS) {
+        // lane's unit: its records [r0, r1) and their marks
+        auto first_rec = [&](int u) {
+            if (SIDE == 1) return 32 * u;
+            const int c = u / a.runs_per_chunk, m = u - c * a.runs_per_chunk;
+            return 16 * (c * a.jc_tiles + 4 * m);
+        };
+        auto unit_of = [&](int l) {
+            return ubase + (SIDE == 0 ? 4 * l + warp : 16 * (l >> 2) + 4 * warp + (l & 3));
+        };
+        const int base = first_rec(ubase);
+        const int u = unit_of(lane);
+        unsigned long long marks = 0;
+        int r0 = 0;
+        if (lane < S::UNITS && u < n_units) {
+            r0 = first_rec(u);
+            if (SIDE == 1) {
+                marks = bits[r0 >> 5];
+            } else {
+                const int c = u / a.runs_per_chunk;
+                const int end = min(16 * min((c + 1) * a.jc_tiles, a.total_tiles), r0 + 64), w = r0 >> 5;
+                if (end > r0) {   // (the last chunk's runs may lie past the end)
+                    marks = bits[w] | (unsigned long long)(w + 1 < a.words[0] ? bits[w + 1] : 0u) << 32;
+                    if (r0 & 16)
+                        marks = marks >> 16 | (unsigned long long)(w + 2 < a.words[0] ? bits[w + 2] : 0u) << 48;
+                    marks &= end - r0 >= 64 ? ~0ull : (1ull << (end - r0)) - 1;
+                }
+            }
+        }
+        int at = __popcll(marks);
+        const int own = at;
+#pragma unroll
+        for (int o = 1; o < S::UNITS; o <<= 1) {
+            const int v = __shfl_up_sync(0xffffffffu, at, o);
+            if (lane >= o) at += v;
+        }
+        const int n = __shfl_sync(0xffffffffu, at, S::UNITS - 1);
+        if (n == 0) continue;
+        at -= own;
+        // a list entry: record - base; 0x8000 on a unit's first, 0x4000 on a source block's first (side 1)
+        unsigned any = __ballot_sync(0xffffffffu, marks != 0);
+        const bool opens = SIDE == 1 && (any & ((1u << lane) - 1) & 0xfu << (lane & ~3)) == 0;
+        for (bool head = true; marks; head = false) {
+            list[at++] = (uint16_t)((r0 - base + __ffsll(marks) - 1) | (head ? 0x8000 | (opens ? 0x4000 : 0) : 0));
+            marks &= marks - 1;
+        }
+        __syncwarp();
+        float2 v[S::BATCH];
+        auto fetch = [&](int b) {
+#pragma unroll
+            for (int k = 0; k < S::BATCH; ++k)
+                v[k] = recs[(size_t)(base + (list[min(b + k, n - 1)] & 0x3fff)) * 32 + lane];
+        };
+        fetch(0);
+        for (int b = 0, buf = 0; b < n; b += S::BATCH, buf ^= 1) {
+#pragma unroll
+            for (int k = 0; k < S::BATCH; ++k) rec[buf][32 * k + lane] = v[k];
+            __syncwarp();
+            if (b + S::BATCH < n) fetch(b + S::BATCH);
+            const Rec256* rr = reinterpret_cast<const Rec256*>(rec[buf]);
+            const int m = min(S::BATCH, n - b);
+            for (int k = 0; k < m; ++k) {
+                const unsigned e = list[b + k];
+                if (e & 0x8000 && b + k > 0) fold((e & 0x4000) != 0);
+                const Rec256& r = rr[k];
+                float2 d[3], ms[6];
+#pragma unroll
+                for (int q = 0; q < D; ++q) d[q] = fadd2(fadd2(PH[q], fld256(r, q)), SIDE == 0 ? fld256(r, 4 + q) : PL[q]);
+#pragma unroll
+                for (int q = 0; q < NS; ++q) ms[q] = fld256(r, 8 + q);
+                const float2 lv = SIDE == 0 ? fld256(r, 3) : lvs;
+                const float2 p = SIDE == 0 ? fadd2(pexp2<D, true>(Mx, d, lv), pexp2<D, true>(ms, d, lv))
+                                           : fadd2(pexp2<D, true>(ms, d, lv), pexp2<D, true>(Mx, d, lv));
+#pragma unroll
+                for (int q = 0; q < NF; ++q) h[q] = ffma2(p, fld256(r, 16 + q), h[q]);
+            }
+        }
+        fold(true);
+        __syncwarp();   // (the list is rewritten)
+    }
+    __syncthreads();
+    if (warp > 0 || !in) return;
+    const double sgm = 1.0 / a.pose[kPoseSig];
+    const double Gs = pow(sgm, (double)D);
+    const double w = SIDE == 0 ? (double)a.wx[i] * (Gs * exp2(a.Lmax_y)) : Gs * exp2(a.Lmax_x + a.Lmax_y);
+    double* o = (SIDE == 0 ? a.h2 : a.h1) + (size_t)i * 16;
+#pragma unroll
+    for (int q = 0; q < NF; ++q) {
+        double t = sums[0][q][lane];
+#pragma unroll
+        for (int k = 1; k < 4; ++k) t += sums[k][q][lane];
+        o[q] = w * t;
+    }
+}
+
+template <int D>
+__global__ void __launch_bounds__(128, 5) coef_sparse_kernel(CoefSparseArgs a)
+{
+    using S = CoefSparseShape;
+    extern __shared__ __align__(128) unsigned char smem[];
+    const int side = (int)blockIdx.x < a.n_st0 ? 0 : 1;
+    uint32_t* bits = reinterpret_cast<uint32_t*>(smem + S::kFixed);
+    pdl_trigger();   // a dependent of the coefficient prologue, and the moments kernel one of this
+    for (int w = threadIdx.x; w < a.words[side]; w += 128) bits[w] = 0;
+    pdl_wait();
+    if (a.go && !*a.go) return;
+    if (side == 0)
+        coef_sparse_side<D, 0>(a, blockIdx.x, smem);
+    else
+        coef_sparse_side<D, 1>(a, blockIdx.x - a.n_st0, smem);
 }
 
 // ---------------------------------------------------------------------------
@@ -978,6 +1207,8 @@ struct MomSide {
     const float* p;       // the side's points, D per row
     const float* cinv;    // its inverse covariances, D x D per row
     double* out;          // [nblk][moments] block partials
+    const int* sparse;    // nullable: when set, h1 holds the rows, one copy
+    const double* h1;
 };
 
 // Moments from the per-point H: blockIdx.y picks the side (s0 or s1), and the side's nblk blocks
@@ -993,11 +1224,11 @@ __global__ void __launch_bounds__(kMomThreads) moments_kernel(const MomSide s0, 
     pdl_wait();
     const MomSide ms = blockIdx.y == 0 ? s0 : s1;
     if ((int)blockIdx.x >= ms.nblk) return;
-    const double* __restrict__ hpart = ms.h;
     const float* __restrict__ p = ms.p;
     const float* __restrict__ cinv = ms.cinv;
     double* __restrict__ block_out = ms.out;
-    const int n_jc = ms.copies, n = ms.n, side = ms.side;
+    const int n_jc = ms.sparse && *ms.sparse ? 1 : ms.copies, n = ms.n, side = ms.side;
+    const double* __restrict__ hpart = ms.sparse && *ms.sparse ? ms.h1 : ms.h;
     constexpr int NS = Sym<D>::N, NF = Feat<D>::N;
     constexpr int NM = D == 3 ? kNumMoments3D : kNumMoments2D;
     const signed char(*tab)[4] = D == 3 ? c_moment3 : c_moment2;
@@ -1259,11 +1490,27 @@ extern "C" int dugma_coef_work_grid(int N, int M, int resident, int grid[4])
 
 namespace dugma {
 
-// Every source row against every target row in one pass (coef_fused_kernel), then the moments
+// coef_sparse_kernel's dynamic shared memory limit, once per device
+template <int D>
+static int coef_sparse_setup(int dev)
+{
+    static std::mutex mu;
+    static bool done[64];
+    std::lock_guard<std::mutex> lk(mu);
+    if (dev >= 64 || !done[dev]) {
+        DUGMA_CK(cudaFuncSetAttribute(coef_sparse_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      (int)(CoefSparseShape::kFixed + kSparseMaxTargets / 64 * sizeof(uint32_t))));
+        if (dev < 64) done[dev] = true;
+    }
+    return DUGMA_OK;
+}
+
+// Every source row against every target row in one pass (coef_fused_kernel), or the pairs above the
+// FP32 flush (sparse; with flag given both are enqueued and the flag lets one run), then the moments
 // of both sides from the H2 copies (one per target chunk) and the H1 copies (one per source group).
 template <int D, bool CHOL>
 static int coef_fused_launch(Context& c, const double* pose_dev, double* moments_dev, cudaStream_t s,
-                             double* host_moments)
+                             double* host_moments, bool sparse, const int* flag)
 {
     constexpr int NM = D == 3 ? kNumMoments3D : kNumMoments2D;
     const int kind = c.coef_kernel;
@@ -1285,8 +1532,10 @@ static int coef_fused_launch(Context& c, const double* pose_dev, double* moments
         c.coef_grid[3] = fg.n_jc;
     }
     const int SB = c.coef_grid[0], n_grp = c.coef_grid[1], jc_tiles = c.coef_grid[2], n_jc = c.coef_grid[3];
-    const size_t h2_doubles = (size_t)n_jc * c.N * 16, h1_doubles = (size_t)n_grp * c.M * 16;
+    const bool dense = !sparse || flag;
+    const size_t h2_doubles = (size_t)(dense ? n_jc : 1) * c.N * 16, h1_doubles = (size_t)(dense ? n_grp : 1) * c.M * 16;
     DUGMA_RET(c.ensure_scratch(sizeof(double) * (h2_doubles + h1_doubles)));
+    double *rows2 = c.scratch, *rows1 = c.scratch + (size_t)c.N * 16;   // the sparse pass's (only one pass runs)
     FusedCoefArgs a{};
     a.xrec = c.xrec128;
     a.yrec = static_cast<const Rec256*>(c.yrec256);
@@ -1306,32 +1555,56 @@ static int coef_fused_launch(Context& c, const double* pose_dev, double* moments
     a.h1_part = c.scratch + h2_doubles;
     a.counter = c.counter;
     a.err = c.err;
+    a.skip = flag;
     // (the coefficient prologue zeroed c.counter)
-    cudaEvent_t ev1 = nullptr;
-    if (c.timing) {
-        if (c.tused == c.tevents.size()) {
-            cudaEvent_t e0, e1;
-            DUGMA_CK(cudaEventCreate(&e0));
-            DUGMA_CK(cudaEventCreate(&e1));
-            c.tevents.push_back({e0, e1});
-        }
-        DUGMA_CK(cudaEventRecord(c.tevents[c.tused].first, s));
-        ev1 = c.tevents[c.tused].second;
-        ++c.tused;
+    DUGMA_RET(timing_begin(c, s));
+    if (dense) {
+        const int grid = std::min(resident, n_grp * n_jc);
+        if (kind == 1)
+            DUGMA_CK(launch_dependent(c.pdl, coef_tc_kernel<D, 1, CHOL>, grid, TcCoefShape<D, 1>::NT,
+                                      TcCoefShape<D, 1>::kBytes, s, a));
+        else
+            DUGMA_CK(launch_dependent(c.pdl, coef_fused_kernel<D, CHOL>, grid, FusedCoefShape<D>::NT,
+                                      FusedCoefShape<D>::kBytes, s, a));
+        DUGMA_CK(cudaGetLastError());
     }
-    const int grid = std::min(resident, n_grp * n_jc);
-    if (kind == 1)
-        DUGMA_CK(launch_dependent(c.pdl, coef_tc_kernel<D, 1, CHOL>, grid, TcCoefShape<D, 1>::NT,
-                                  TcCoefShape<D, 1>::kBytes, s, a));
-    else
-        DUGMA_CK(launch_dependent(c.pdl, coef_fused_kernel<D, CHOL>, grid, FusedCoefShape<D>::NT,
-                                  FusedCoefShape<D>::kBytes, s, a));
-    DUGMA_CK(cudaGetLastError());
-    if (ev1) DUGMA_CK(cudaEventRecord(ev1, s));
+    if (sparse) {
+        static_assert(FusedCoefShape<D>::FOLD == 4 && FusedCoefShape<D>::TJ == 16 && FusedCoefShape<D>::BI == 256,
+                      "the sparse pass's units are the one pass's folds");
+        DUGMA_RET(coef_sparse_setup<D>(c.dev));
+        CoefSparseArgs sa{};
+        sa.x = {c.xpt, c.xtile, c.xsub, c.xsuper, c.N};
+        sa.y = {c.ypt, c.ytile, c.ysub, c.ysuper, c.M};
+        sa.inv_trace = c.inv_trace;
+        sa.pose = pose_dev;
+        sa.xrec = c.xrec128;
+        sa.yrec = c.yrec128;
+        sa.xpair = static_cast<const Rec256*>(c.xrec256);
+        sa.ypair = static_cast<const Rec256*>(c.yrec256);
+        sa.wx = c.wx;
+        sa.Lmax_x = c.Lmax_x;
+        sa.Lmax_y = c.Lmax_y;
+        sa.n_st0 = (c.N + kTile - 1) / kTile;
+        sa.n_rec[0] = c.M_pad / 2;
+        sa.n_rec[1] = c.N_pad / 2;
+        for (int k = 0; k < 2; ++k) sa.words[k] = (sa.n_rec[k] + 31) / 32;
+        sa.jc_tiles = jc_tiles;
+        sa.total_tiles = total_tiles;
+        sa.runs_per_chunk = (jc_tiles + 3) / 4;
+        sa.n_units[0] = n_jc * sa.runs_per_chunk;
+        sa.n_units[1] = (sa.n_rec[1] + 31) / 32;
+        sa.h2 = rows2;
+        sa.h1 = rows1;
+        sa.go = flag;
+        const size_t bytes = CoefSparseShape::kFixed + sizeof(uint32_t) * std::max(sa.words[0], sa.words[1]);
+        DUGMA_CK(launch_dependent(c.pdl, coef_sparse_kernel<D>, sa.n_st0 + (c.M + kTile - 1) / kTile, 128, bytes, s, sa));
+    }
+    DUGMA_RET(timing_end(c, s));
     const int nblk = std::max(1, std::min(2 * c.num_sms, (std::max(c.N, c.M) + 31) / 32));
     const int nb0 = std::min(nblk, c.N), nb1 = std::min(nblk, c.M);
-    const MomSide m0{a.h2_part, n_jc, c.N, nb0, 0, c.x, c.xinv, c.mom_part};
-    const MomSide m1{a.h1_part, n_grp, c.M, nb1, 1, c.y, c.yinv, c.mom_part + (size_t)nblk * NM};
+    const MomSide m0{dense ? a.h2_part : rows2, dense ? n_jc : 1, c.N, nb0, 0, c.x, c.xinv, c.mom_part, flag, rows2};
+    const MomSide m1{dense ? a.h1_part : rows1, dense ? n_grp : 1, c.M, nb1, 1, c.y, c.yinv,
+                     c.mom_part + (size_t)nblk * NM, flag, rows1};
     DUGMA_CK(launch_dependent(c.pdl, moments_kernel<D>, dim3(std::max(nb0, nb1), 2), kMomThreads, 0, s, m0, m1,
                               (const double*)pose_dev));
     DUGMA_CK(launch_dependent(c.pdl, moments_reduce_kernel, (NM + 7) / 8, 256, 0, s, (const double*)c.mom_part, nb0,
@@ -1355,16 +1628,29 @@ static int coef_impl(Context& c, double* pose_dev, double* moments_dev, cudaStre
     // the Cholesky form of every matrix when every weighted point's inverse covariance has a factor,
     // else the Horner form throughout
     const bool chol = c.ux && c.x_indef == 0 && c.y_indef == 0;
+    // The sparse pass by the rule of the energy's (sparse_sigma).  A call and an EM step at the same
+    // sigma go the same way (their coefficients are the same bits); in the EM step, where only the device
+    // knows sigma, both passes are enqueued and the prologue's flag lets one run, so the pass is taken up
+    // from kSparseCoefMinPairs pairs, where the launch that returns at once is lost in the other.
+    const double below = fused && chol && c.coef_kernel == 0 && c.N <= kSparseMaxTargets &&
+                                 (double)c.N * c.M >= kSparseCoefMinPairs
+                             ? sparse_sigma(c)
+                             : 0.0;
+    const double sig = o.pose_value ? o.pose_value[kPoseSig] : 0.0;
+    const bool both = !(sig > 0.0) && below > 0.0;
+    const bool sparse = both || (sig > 0.0 && sig < below);
+    const int* flag = both ? c.counter + 4 : nullptr;
     const int pg = std::min((n + 127) / 128, c.num_sms * 8);
     auto prologue = chol ? coef_prologue_kernel<D, true> : coef_prologue_kernel<D, false>;
     prologue<<<pg, 128, 0, s>>>(pb, o.pose_value ? 1 : 0, pose_dev, c.y, c.yinv, c.lwy, c.M, c.M_pad, c.yrec128,
                                 static_cast<Rec256*>(c.yrec256), c.x, c.xinv, c.lwx, c.N, c.N_pad, c.xrec128,
                                 static_cast<Rec256*>(c.xrec256), fused ? c.counter : nullptr,
-                                o.reset_err ? c.err : nullptr, (const double*)c.ux);
+                                o.reset_err ? c.err : nullptr, (const double*)c.ux, sparse ? (const float*)c.wx : nullptr,
+                                c.Lmax_x, both ? below : 0.0);
     DUGMA_CK(cudaGetLastError());
     if (fused)
-        return chol ? coef_fused_launch<D, true>(c, pose_dev, moments_dev, s, o.host_moments)
-                    : coef_fused_launch<D, false>(c, pose_dev, moments_dev, s, o.host_moments);
+        return chol ? coef_fused_launch<D, true>(c, pose_dev, moments_dev, s, o.host_moments, sparse, flag)
+                    : coef_fused_launch<D, false>(c, pose_dev, moments_dev, s, o.host_moments, false, nullptr);
     constexpr int NM = D == 3 ? kNumMoments3D : kNumMoments2D;
     // per side: 2 sources per thread x 128 threads when there are rows enough for two blocks
     // per SM, else 1 x 64 (more blocks for small clouds); items cover at least rows / 8
@@ -1410,8 +1696,9 @@ static int coef_impl(Context& c, double* pose_dev, double* moments_dev, cudaStre
         const int nb = std::min(nblk, rows);
         nb_side[side] = nb;
         const size_t o1 = (size_t)r0 * c.D, o2 = (size_t)r0 * c.D * c.D;
-        const MomSide ms = side == 0 ? MomSide{hp, n_jc, rows, nb, 0, c.x + o1, c.xinv + o2, mom}
-                                     : MomSide{hp, n_jc, rows, nb, 1, c.y + o1, c.yinv + o2, mom + (size_t)nblk * NM};
+        const MomSide ms = side == 0 ? MomSide{hp, n_jc, rows, nb, 0, c.x + o1, c.xinv + o2, mom, nullptr, nullptr}
+                                     : MomSide{hp, n_jc, rows, nb, 1, c.y + o1, c.yinv + o2, mom + (size_t)nblk * NM,
+                                               nullptr, nullptr};
         moments_kernel<D><<<dim3(nb, 1), kMomThreads, 0, s>>>(ms, ms, pose_dev);
         if (cudaGetLastError() != cudaSuccess) rc = set_error(DUGMA_ERR_CUDA, "moments kernel launch failed");
     }

@@ -189,7 +189,7 @@ int timing_end(Context& c, cudaStream_t s);
 // The REF energy or adjoint over the pairs above the FP32 flush (sparse.cu), from the records of the
 // packed kernels' prologue: the same sums as the all-pairs kernel with tiles of tile_rec and chunks of
 // chunk_rec records.  go (nullable, device): nothing is done unless it is set.
-constexpr double kSparseMinPairs = 4e6, kSparseMinPairsAuto = 64e6;
+constexpr double kSparseMinPairs = 4e6, kSparseMinPairsAuto = 64e6, kSparseCoefMinPairs = 24e6;
 constexpr int kSparseMaxTargets = 1 << 20;
 double sparse_sigma(const Context& c);   // evaluations with a sigma below this go that way
 int sparse_launch(Context& c, const double* pose_dev, bool grad, int tile_rec, int chunk_rec, double* out_dev,

@@ -240,6 +240,7 @@ __global__ void __launch_bounds__(256) reduce_rows_kernel(const double* rows, in
 // many as make the all-pairs kernel, with four sources a thread, the better one.
 double sparse_sigma(const Context& c)
 {
+    // (the same rule for the coefficients' sparse pass, coef.cu)
     if (c.x_indef > 0 || c.y_indef > 0 || !c.ux || !c.xpt || c.no_alloc || c.all_pairs) return 0.0;
     if ((double)c.N * c.M < kSparseMinPairs || c.M > kSparseMaxTargets) return 0.0;
     const double v = (c.trace_x + c.trace_y) / (2.0 * c.D), r2 = std::min(c.rho2_x, c.rho2_y);

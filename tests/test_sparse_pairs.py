@@ -45,7 +45,14 @@ def _problem(kind, n, m, seed):
     return X, XC, Y, YC, P.R_G, P.t_G
 
 
-def _evaluate(monkeypatch, prob, R, t, sig, all_pairs):
+ENERGY = {"grad": lambda h, R, t, sig: api.energy_grad(h, R, t, sig)[:2],
+          "grad_dx": lambda h, R, t, sig: api.energy_grad(h, R, t, sig, with_dx=True),
+          "energy": lambda h, R, t, sig: (api.energy(h, R, t, sig),),
+          "fd": lambda h, R, t, sig: (api.energy_fd_grad(h, R, t, sig)[0],)}
+COEF = {"compi": lambda h, R, t, sig: (api.compi(h, R, t, sig=sig),)}
+
+
+def _evaluate(monkeypatch, calls, prob, R, t, sig, all_pairs):
     if all_pairs:
         monkeypatch.setenv("DUGMA_ALL_PAIRS", "1")
     else:
@@ -53,12 +60,9 @@ def _evaluate(monkeypatch, prob, R, t, sig, all_pairs):
     _, h = api.init(*prob[:4])
     out = {}
     try:
-        for name, fn in (("grad", lambda: api.energy_grad(h, R, t, sig)[:2]),
-                         ("grad_dx", lambda: api.energy_grad(h, R, t, sig, with_dx=True)),
-                         ("energy", lambda: (api.energy(h, R, t, sig),)),
-                         ("fd", lambda: (api.energy_fd_grad(h, R, t, sig)[0],))):
+        for name, fn in calls.items():
             try:
-                out[name] = [np.asarray(v) for v in fn()]
+                out[name] = [np.asarray(v) for v in fn(h, R, t, sig)]
             except api.DugmaError as e:
                 out[name] = e.code
     finally:
@@ -70,16 +74,13 @@ KINDS = ["sphere", "outliers", "harmonic", "curve", "neglected", "coincident", "
          "huge"]
 
 
-@pytest.mark.filterwarnings("ignore")
-@pytest.mark.parametrize("n,m", [(2049, 2001), (5000, 901), (1025, 4097)])
-@pytest.mark.parametrize("kind", KINDS)
-def test_same_sums_as_all_pairs(kind, n, m, monkeypatch):
+def _compare(monkeypatch, calls, kind, n, m, sigs):
     prob = _problem(kind, n, m, 3)
     R, t = prob[4], prob[5]
     for scale in (1.0, 1.05):        # a rotation, and a matrix that stretches
-        for sig in (2e-4, 4e-3, 3e-2):
-            a = _evaluate(monkeypatch, prob, scale * R, t + 0.01, sig, False)
-            b = _evaluate(monkeypatch, prob, scale * R, t + 0.01, sig, True)
+        for sig in sigs:
+            a = _evaluate(monkeypatch, calls, prob, scale * R, t + 0.01, sig, False)
+            b = _evaluate(monkeypatch, calls, prob, scale * R, t + 0.01, sig, True)
             for name in b:
                 if isinstance(b[name], int) or isinstance(a[name], int):
                     assert isinstance(b[name], int) and a[name] == b[name], (name, a[name], b[name])
@@ -88,3 +89,30 @@ def test_same_sums_as_all_pairs(kind, n, m, monkeypatch):
                     assert np.all(np.isfinite(u) == np.isfinite(v)), name
                     u, v = u[np.isfinite(u)], v[np.isfinite(v)]
                     assert np.linalg.norm(u - v) <= 1e-12 * np.linalg.norm(v), (name, sig, u, v)
+
+
+@pytest.mark.filterwarnings("ignore")
+@pytest.mark.parametrize("n,m", [(2049, 2001), (5000, 901), (1025, 4097)])
+@pytest.mark.parametrize("kind", KINDS)
+def test_energy_same_sums_as_all_pairs(kind, n, m, monkeypatch):
+    _compare(monkeypatch, ENERGY, kind, n, m, (2e-4, 4e-3, 3e-2))
+
+
+@pytest.mark.filterwarnings("ignore")
+@pytest.mark.parametrize("n,m", [(5001, 4901), (33000, 801), (1025, 25001)])
+@pytest.mark.parametrize("kind", KINDS)
+def test_compi_same_sums_as_all_pairs(kind, n, m, monkeypatch):
+    _compare(monkeypatch, COEF, kind, n, m, (4e-4, 2e-2))
+
+
+@pytest.mark.parametrize("widen", [1.0, 1e4])   # (1e4: sigma beyond the rule, all pairs run)
+def test_em_step_is_update_sig_and_compi(widen):
+    """An EM step decides on the device what compi decides on the host: the same bits either way."""
+    X, XC, Y, YC, R, t = _problem("sphere", 5001, 4999, 1)
+    _, h = api.init(X, XC * widen, Y, YC * widen)
+    em = api.EMGraph(h)
+    sig, A = em(R, t + 0.01)
+    assert sig == api.update_sig(h, R, t + 0.01)
+    assert np.array_equal(A, api.compi(h, R, t + 0.01, sig=sig))
+    em.close()
+    api.fr_m(h)
