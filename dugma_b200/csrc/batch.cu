@@ -10,6 +10,10 @@
 //      atomic counter, each item reducing into its own partial slot;
 //   4. sums each pq's item partials in a fixed order.
 // Steps 2-4 are captured once as a CUDA graph per pose count and replayed afterwards.
+// A (problem, pose) whose sigma leaves most pairs of points under the FP32 flush is evaluated over the
+// others instead of step 3 (sparse.cu: the same sums): one block per tile of its sources, in slabs
+// of (problem, pose)s whose rows fit 256 MB.  One B200, 24 problems of 500 - 8000 points x 8 poses:
+// 5.0 ms over all pairs, see the design notes for the sparse figure.
 #include <algorithm>
 #include <cmath>
 #include <cstring>
@@ -17,8 +21,7 @@
 #include <string>
 #include <vector>
 
-#include "bodies.cuh"
-#include "context.hpp"
+#include "sparse.cuh"
 
 namespace dugma {
 
@@ -37,7 +40,14 @@ struct PQDesc {
     YRec2* yrec;
     double Lmax;
     int N, M, M_pad;
+    ReachSide rx, ry;   // the clouds in spatial order
+    float inv_trace;
+    int row0;           // the pair's first row in its slab
 };
+
+// in a pose block: nonzero where the pair (problem, pose) is evaluated over the pairs of points above
+// the FP32 flush only (sparse.cu)
+constexpr int kPoseSparse = 14;
 
 struct BatchItem {
     int pq, ib, tile0, ntiles;
@@ -150,6 +160,10 @@ __global__ void __launch_bounds__(NT) batch_pairs_kernel(const PQDesc* __restric
         if (item >= n_items) break;
         const BatchItem it = items[item];
         const PQDesc pd = desc[it.pq];
+        if (pd.pose[kPoseSparse] != 0.0) {
+            __syncthreads();   // (s_item is read)
+            continue;
+        }
         PairArgs a{};
         a.xrec = pd.xrec;
         a.yrec = pd.yrec;
@@ -200,16 +214,48 @@ __global__ void __launch_bounds__(NT) batch_pairs_kernel(const PQDesc* __restric
     }
 }
 
-// out[pq][v] = sum of the pq's item partials, in the fixed order of its item index list
-__global__ void batch_reduce_kernel(const double* __restrict__ partials, const int* __restrict__ pq_start,
-                                    const int* __restrict__ pq_items, int nv, double* __restrict__ out)
+// The sparse pairs of a slab: tile blockIdx.x of the sources of pair pq0 + blockIdx.y (sparse.cu).
+template <int D>
+__global__ void __launch_bounds__(128, 6) batch_sparse_kernel(const PQDesc* __restrict__ desc, int pq0, int tile_shift,
+                                                              int chunk_rec, double* __restrict__ rows)
+{
+    extern __shared__ __align__(16) unsigned char smem[];
+    const PQDesc& pd = desc[pq0 + blockIdx.y];
+    if ((int)blockIdx.x * kTile >= pd.N || pd.pose[kPoseSparse] == 0.0) return;
+    SparseArgs a{};
+    a.reach = {pd.rx, pd.ry, pd.pose, pd.inv_trace};
+    a.xrec = pd.xrec;
+    a.yrec = pd.yrec;
+    a.wx = pd.wx;
+    a.pose = pd.pose;
+    a.Lmax = pd.Lmax;
+    a.n_rec = pd.M_pad / 2;
+    a.words = (a.n_rec + 31) / 32;
+    a.tile_shift = tile_shift;
+    a.chunk_rec = chunk_rec;
+    a.rows = rows + (size_t)pd.row0 * 8;
+    uint32_t* bits = reinterpret_cast<uint32_t*>(smem + kSparseFixed);
+    for (int w = threadIdx.x; w < a.words; w += 128) bits[w] = 0;
+    sparse_tile<D, true>(a, blockIdx.x, smem);
+}
+
+// out[pq][v] = sum of the pair's item partials, in the fixed order of its item index list, or of its
+// sources' rows
+__global__ void batch_reduce_kernel(const PQDesc* __restrict__ desc, int pq0, const double* __restrict__ partials,
+                                    const int* __restrict__ pq_start, const int* __restrict__ pq_items,
+                                    const double* __restrict__ rows, int nv, double* __restrict__ out)
 {
     __shared__ double red[128];
-    const int pq = blockIdx.x;
-    const int b = pq_start[pq], e = pq_start[pq + 1];
+    const int pq = pq0 + blockIdx.x;
+    const bool sparse = desc[pq].pose[kPoseSparse] != 0.0;
+    const int b = sparse ? 0 : pq_start[pq], e = sparse ? desc[pq].N : pq_start[pq + 1];
+    const double* r = rows + (size_t)desc[pq].row0 * 8;
     for (int v = 0; v < nv; ++v) {
         double s = 0;
-        for (int k = b + threadIdx.x; k < e; k += blockDim.x) s += partials[(size_t)pq_items[k] * 8 + v];
+        if (sparse)
+            for (int k = threadIdx.x; k < e; k += blockDim.x) s += r[(size_t)k * 8 + v];
+        else
+            for (int k = b + threadIdx.x; k < e; k += blockDim.x) s += partials[(size_t)pq_items[k] * 8 + v];
         red[threadIdx.x] = s;
         __syncthreads();
         for (int h = blockDim.x / 2; h > 0; h >>= 1) {
@@ -249,12 +295,15 @@ static const BatchShape& batch_shape_of(int D, int k)
     return D == 3 ? batch_variants<3>()[k].sh : batch_variants<2>()[k].sh;
 }
 
+constexpr size_t kSlabRows = (size_t)4 << 20;   // source rows of one sparse launch (256 MB)
+
 struct Batch {
     int D = 3, P = 0;
     int shape = 0;                    // index into batch_variants<D>()
     int prepared_shape = -1;          // the shape the pose-count state below was built for
     std::vector<float*> ptrs;          // 6 per problem
     std::vector<Context*> ctx;
+    std::vector<double> below;         // per problem: poses with a smaller sigma are sparse
     cudaStream_t stream = nullptr;
     // per pose-count state
     int n_poses = 0, n_items = 0, nv = 0;
@@ -271,6 +320,11 @@ struct Batch {
     std::vector<std::pair<cudaEvent_t, cudaEvent_t>> tevents;
     size_t tused = 0;
     int max_span = 0;
+    double* rows = nullptr;           // a slab's source rows (sparse pairs)
+    std::vector<int> slab;            // the slabs' first pairs, and n_pq
+    int max_tiles = 0, max_words = 0; // source tiles, target bitmap words of the largest problem
+    bool all_pairs = false;           // no pair sparse (while the dense shapes are timed)
+    bool any_dense = true, any_sparse = false;   // of the evaluation at hand
     bool chol = true;                 // every problem's weighted sources have Cholesky factors
     cudaGraphExec_t exec = nullptr;
     cudaGraph_t graph = nullptr;
@@ -324,6 +378,24 @@ static int batch_prepare(Batch& b, int n_poses)
                 }
         }
     }
+    // slabs of at most kSlabRows source rows
+    std::vector<int> row0(n_pq);
+    b.slab.assign(1, 0);
+    size_t slab_rows = 0, most_rows = 0;
+    b.max_tiles = b.max_words = 0;
+    for (int pq = 0; pq < n_pq; ++pq) {
+        const Context& c = *b.ctx[pq / n_poses];
+        if (slab_rows + c.N > kSlabRows && slab_rows > 0) {
+            b.slab.push_back(pq);
+            slab_rows = 0;
+        }
+        row0[pq] = (int)slab_rows;
+        slab_rows += c.N;
+        most_rows = std::max(most_rows, slab_rows);
+        b.max_tiles = std::max(b.max_tiles, (c.N + kTile - 1) / kTile);
+        b.max_words = std::max(b.max_words, (c.M_pad / 2 + 31) / 32);
+    }
+    b.slab.push_back(n_pq);
     std::vector<int> order(items.size());
     std::iota(order.begin(), order.end(), 0);
     std::stable_sort(order.begin(), order.end(), [&](int a, int b2) { return cost[a] > cost[b2]; });
@@ -343,8 +415,9 @@ static int batch_prepare(Batch& b, int n_poses)
     const size_t s_poses = up(sizeof(double) * 16 * n_pq), s_desc = up(sizeof(PQDesc) * n_pq),
                  s_items = up(sizeof(BatchItem) * sorted.size()), s_start = up(sizeof(int) * (n_pq + 1)),
                  s_list = up(sizeof(int) * sorted.size()), s_ctr = 256, s_part = up(sizeof(double) * 8 * sorted.size()),
-                 s_out = up(sizeof(double) * b.nv * n_pq), s_y = up(ybytes), s_x = up(xbytes);
-    const size_t total = s_poses + s_desc + s_items + s_start + s_list + s_ctr + s_part + s_out + s_y + s_x;
+                 s_out = up(sizeof(double) * b.nv * n_pq), s_y = up(ybytes), s_x = up(xbytes),
+                 s_rows = up(sizeof(double) * 8 * most_rows);
+    const size_t total = s_poses + s_desc + s_items + s_start + s_list + s_ctr + s_part + s_out + s_y + s_x + s_rows;
     if (cudaMalloc(&b.mem, total) != cudaSuccess) {
         cudaGetLastError();
         b.mem = nullptr;
@@ -361,7 +434,8 @@ static int batch_prepare(Batch& b, int n_poses)
     b.partials = reinterpret_cast<double*>(m); m += s_part;
     b.out = reinterpret_cast<double*>(m); m += s_out;
     char* ybase = m; m += s_y;
-    char* xbase = m;
+    char* xbase = m; m += s_x;
+    b.rows = reinterpret_cast<double*>(m);
     std::vector<PQDesc> desc(n_pq);
     for (int p = 0; p < b.P; ++p) {
         const Context& c = *b.ctx[p];
@@ -383,6 +457,10 @@ static int batch_prepare(Batch& b, int n_poses)
             d.N = c.N;
             d.M = c.M;
             d.M_pad = c.M_pad;
+            d.rx = {c.xpt, c.xtile, c.xsub, c.xsuper, c.N};
+            d.ry = {c.ypt, c.ytile, c.ysub, c.ysuper, c.M};
+            d.inv_trace = c.inv_trace;
+            d.row0 = row0[pq];
         }
     }
     DUGMA_CK(cudaMemcpy(b.desc, desc.data(), sizeof(PQDesc) * n_pq, cudaMemcpyHostToDevice));
@@ -414,10 +492,26 @@ static int batch_enqueue(Batch& b, cudaStream_t s)
     batch_prologue_kernel<D><<<dim3(gx, n_pq), 256, 0, s>>>(b.desc, b.max_span);
     DUGMA_CK(cudaGetLastError());
     DUGMA_CK(cudaMemsetAsync(b.counter, 0, 8 * sizeof(int), s));
-    fn<<<grid, var.sh.nt, 0, s>>>(b.desc, b.items, b.n_items, b.partials, b.counter, b.err);
-    DUGMA_CK(cudaGetLastError());
-    batch_reduce_kernel<<<n_pq, 128, 0, s>>>(b.partials, b.pq_start, b.pq_items, b.nv, b.out);
-    DUGMA_CK(cudaGetLastError());
+    if (b.any_dense) {
+        fn<<<grid, var.sh.nt, 0, s>>>(b.desc, b.items, b.n_items, b.partials, b.counter, b.err);
+        DUGMA_CK(cudaGetLastError());
+    }
+    if (!b.any_sparse) {
+        batch_reduce_kernel<<<n_pq, 128, 0, s>>>(b.desc, 0, b.partials, b.pq_start, b.pq_items, b.rows, b.nv, b.out);
+        DUGMA_CK(cudaGetLastError());
+        return DUGMA_OK;
+    }
+    int shift = 0;
+    while (1 << shift < var.sh.tj) ++shift;
+    const size_t smem = kSparseFixed + sizeof(uint32_t) * b.max_words;
+    DUGMA_CK(cudaFuncSetAttribute(batch_sparse_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    for (size_t k = 0; k + 1 < b.slab.size(); ++k) {
+        const int q0 = b.slab[k], nq = b.slab[k + 1] - q0;
+        batch_sparse_kernel<D><<<dim3(b.max_tiles, nq), 128, smem, s>>>(b.desc, q0, shift, var.sh.chunk, b.rows);
+        DUGMA_CK(cudaGetLastError());
+        batch_reduce_kernel<<<nq, 128, 0, s>>>(b.desc, q0, b.partials, b.pq_start, b.pq_items, b.rows, b.nv, b.out);
+        DUGMA_CK(cudaGetLastError());
+    }
     return DUGMA_OK;
 }
 
@@ -436,6 +530,11 @@ static int batch_launch(Batch& b)
         DUGMA_CK(cudaEventRecord(b.tevents[b.tused].first, b.stream));
         ev1 = b.tevents[b.tused].second;
         ++b.tused;
+    }
+    if (b.any_sparse) {   // (a few launches that the kernels outlast: not captured)
+        DUGMA_RET(b.D == 3 ? batch_enqueue<3>(b, b.stream) : batch_enqueue<2>(b, b.stream));
+        if (ev1) DUGMA_CK(cudaEventRecord(ev1, b.stream));
+        return DUGMA_OK;
     }
     if (!b.exec) {
         DUGMA_RET(b.D == 3 ? batch_enqueue<3>(b, b.stream) : batch_enqueue<2>(b, b.stream));
@@ -457,6 +556,7 @@ static int batch_eval(Batch& b, int n_poses, const double* poses, double* out)
 {
     DUGMA_RET(batch_prepare(b, n_poses));
     const int n_pq = b.P * n_poses, D = b.D;
+    b.any_dense = b.any_sparse = false;
     for (int k = 0; k < n_pq; ++k) {
         double* h = b.host + 16 * (size_t)k;
         for (int q = 0; q < 16; ++q) h[q] = 0.0;
@@ -465,6 +565,9 @@ static int batch_eval(Batch& b, int n_poses, const double* poses, double* out)
         for (int a = 0; a < D; ++a) h[kPoseT + a] = src[9 + a];
         h[kPoseSig] = src[12];
         if (!(src[12] > 0)) return set_error(DUGMA_ERR_ARG, "batch_energy_grad: sig of pose %d is not positive", k);
+        const bool sparse = !b.all_pairs && src[12] < b.below[k / n_poses];
+        h[kPoseSparse] = sparse ? 1.0 : 0.0;
+        (sparse ? b.any_sparse : b.any_dense) = true;
     }
     DUGMA_CK(cudaMemcpyAsync(b.poses, b.host, sizeof(double) * 16 * n_pq, cudaMemcpyHostToDevice, b.stream));
     DUGMA_RET(batch_launch(b));
@@ -505,6 +608,7 @@ int dugma_batch_create(int n_problems, int D, const int* N, const int* M, const 
         b->ctx.push_back(find_context(&b->ptrs[6 * (size_t)p]));
         if (b->ctx.back()->x_indef > 0) b->chol = false;
     }
+    for (const Context* c : b->ctx) b->below.push_back(b->chol ? sparse_sigma(*c) : 0.0);
     if (cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking) != cudaSuccess) {
         for (int k = 0; k < n_problems; ++k) dugma_fr_m(&b->ptrs[6 * (size_t)k]);
         delete b;
@@ -578,6 +682,7 @@ int dugma_batch_autotune(void* batch, int n_poses, const double* poses, char* re
     DUGMA_CK(cudaEventCreate(&e0));
     DUGMA_CK(cudaEventCreate(&e1));
     b->timing = false;
+    b->all_pairs = true;   // the shapes are the all-pairs kernel's
     int rc = DUGMA_OK;
     for (int k = 0; k < n && rc == DUGMA_OK; ++k) {
         b->shape = k;
@@ -604,6 +709,7 @@ int dugma_batch_autotune(void* batch, int n_poses, const double* poses, char* re
     }
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
+    b->all_pairs = false;
     b->timing = was_timing;
     b->tused = was_used;
     b->shape = best_k;

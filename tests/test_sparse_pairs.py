@@ -116,3 +116,28 @@ def test_em_step_is_update_sig_and_compi(widen):
     assert np.array_equal(A, api.compi(h, R, t + 0.01, sig=sig))
     em.close()
     api.fr_m(h)
+
+
+def test_batch_same_sums_as_all_pairs(monkeypatch):
+    """Problems of uneven sizes, sparse and dense poses mixed, every tile shape."""
+    probs = [_problem(k, n, m, 5) for k, n, m in (("sphere", 2500, 3001), ("outliers", 5000, 1999), ("sphere", 300, 280),
+                                                  ("harmonic", 3333, 2222))]
+    R = np.array([[p[4], p[4] @ p[4], np.eye(3)] for p in probs])
+    t = np.array([[p[5] + 0.01, p[5], p[5]] for p in probs])
+    sig = np.array([[2e-3, 1e-2, 3.0]] * len(probs))
+    out = []
+    for all_pairs in (False, True):
+        if all_pairs:
+            monkeypatch.setenv("DUGMA_ALL_PAIRS", "1")
+        b = api.Batch([p[:4] for p in probs])
+        got = []
+        for shape in api.Batch.shapes():
+            b.set_shape(shape)
+            got += list(b.energy_grad(R, t, sig))
+        again = b.energy_grad(R, t, sig)
+        assert all(np.array_equal(u, v) for u, v in zip(got[-2:], again))
+        b.close()
+        out.append(got)
+    for u, v in zip(*out):
+        assert np.all(np.linalg.norm((u - v).reshape(len(probs), 3, -1), axis=2)
+                      <= 1e-12 * np.linalg.norm(v.reshape(len(probs), 3, -1), axis=2))
