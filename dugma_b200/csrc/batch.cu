@@ -42,6 +42,7 @@ struct PQDesc {
     int N, M, M_pad;
     ReachSide rx, ry;   // the clouds in spatial order
     float inv_trace;
+    double wmax;        // 2^Lmax
     int row0;           // the pair's first row in its slab
 };
 
@@ -228,7 +229,7 @@ __global__ void __launch_bounds__(128, 6) batch_sparse_kernel(const PQDesc* __re
     a.yrec = pd.yrec;
     a.wx = pd.wx;
     a.pose = pd.pose;
-    a.Lmax = pd.Lmax;
+    a.wmax = pd.wmax;
     a.n_rec = pd.M_pad / 2;
     a.words = (a.n_rec + 31) / 32;
     a.tile_shift = tile_shift;
@@ -240,31 +241,39 @@ __global__ void __launch_bounds__(128, 6) batch_sparse_kernel(const PQDesc* __re
 }
 
 // out[pq][v] = sum of the pair's item partials, in the fixed order of its item index list, or of its
-// sources' rows
-__global__ void batch_reduce_kernel(const PQDesc* __restrict__ desc, int pq0, const double* __restrict__ partials,
-                                    const int* __restrict__ pq_start, const int* __restrict__ pq_items,
-                                    const double* __restrict__ rows, int nv, double* __restrict__ out)
+// sources' rows.  Thread (k, v) adds value v of every 32nd entry (a warp reads four whole rows, eight
+// loads ahead), then the threads' sums in fixed order.
+__global__ void __launch_bounds__(256) batch_reduce_kernel(const PQDesc* __restrict__ desc, int pq0,
+                                                           const double* __restrict__ partials,
+                                                           const int* __restrict__ pq_start,
+                                                           const int* __restrict__ pq_items,
+                                                           const double* __restrict__ rows, int nv,
+                                                           double* __restrict__ out)
 {
-    __shared__ double red[128];
+    __shared__ double red[256];
     const int pq = pq0 + blockIdx.x;
     const bool sparse = desc[pq].pose[kPoseSparse] != 0.0;
-    const int b = sparse ? 0 : pq_start[pq], e = sparse ? desc[pq].N : pq_start[pq + 1];
-    const double* r = rows + (size_t)desc[pq].row0 * 8;
-    for (int v = 0; v < nv; ++v) {
-        double s = 0;
-        if (sparse)
-            for (int k = threadIdx.x; k < e; k += blockDim.x) s += r[(size_t)k * 8 + v];
-        else
-            for (int k = b + threadIdx.x; k < e; k += blockDim.x) s += partials[(size_t)pq_items[k] * 8 + v];
-        red[threadIdx.x] = s;
-        __syncthreads();
-        for (int h = blockDim.x / 2; h > 0; h >>= 1) {
-            if (threadIdx.x < h) red[threadIdx.x] += red[threadIdx.x + h];
-            __syncthreads();
+    const int v = threadIdx.x & 7, k0 = threadIdx.x >> 3;
+    double s = 0;
+    if (v < nv) {
+        if (sparse) {
+            const double* r = rows + (size_t)desc[pq].row0 * 8 + v;
+            const int n = desc[pq].N;
+#pragma unroll 8
+            for (int k = k0; k < n; k += 32) s += r[(size_t)k * 8];
+        } else {
+            const int e = pq_start[pq + 1];
+#pragma unroll 4
+            for (int k = pq_start[pq] + k0; k < e; k += 32) s += partials[(size_t)pq_items[k] * 8 + v];
         }
-        if (threadIdx.x == 0) out[(size_t)pq * nv + v] = red[0];
+    }
+    red[threadIdx.x] = s;
+    __syncthreads();
+    for (int h = 128; h >= 8; h >>= 1) {
+        if ((int)threadIdx.x < h) red[threadIdx.x] += red[threadIdx.x + h];
         __syncthreads();
     }
+    if ((int)threadIdx.x < nv) out[(size_t)pq * nv + v] = red[threadIdx.x];
 }
 
 using BatchKernelFn = void (*)(const PQDesc*, const BatchItem*, int, double*, int*, int*);
@@ -460,6 +469,7 @@ static int batch_prepare(Batch& b, int n_poses)
             d.rx = {c.xpt, c.xtile, c.xsub, c.xsuper, c.N};
             d.ry = {c.ypt, c.ytile, c.ysub, c.ysuper, c.M};
             d.inv_trace = c.inv_trace;
+            d.wmax = std::exp2(c.Lmax_y);
             d.row0 = row0[pq];
         }
     }
@@ -497,7 +507,7 @@ static int batch_enqueue(Batch& b, cudaStream_t s)
         DUGMA_CK(cudaGetLastError());
     }
     if (!b.any_sparse) {
-        batch_reduce_kernel<<<n_pq, 128, 0, s>>>(b.desc, 0, b.partials, b.pq_start, b.pq_items, b.rows, b.nv, b.out);
+        batch_reduce_kernel<<<n_pq, 256, 0, s>>>(b.desc, 0, b.partials, b.pq_start, b.pq_items, b.rows, b.nv, b.out);
         DUGMA_CK(cudaGetLastError());
         return DUGMA_OK;
     }
@@ -509,7 +519,7 @@ static int batch_enqueue(Batch& b, cudaStream_t s)
         const int q0 = b.slab[k], nq = b.slab[k + 1] - q0;
         batch_sparse_kernel<D><<<dim3(b.max_tiles, nq), 128, smem, s>>>(b.desc, q0, shift, var.sh.chunk, b.rows);
         DUGMA_CK(cudaGetLastError());
-        batch_reduce_kernel<<<nq, 128, 0, s>>>(b.desc, q0, b.partials, b.pq_start, b.pq_items, b.rows, b.nv, b.out);
+        batch_reduce_kernel<<<nq, 256, 0, s>>>(b.desc, q0, b.partials, b.pq_start, b.pq_items, b.rows, b.nv, b.out);
         DUGMA_CK(cudaGetLastError());
     }
     return DUGMA_OK;

@@ -627,7 +627,7 @@ struct CoefSparseArgs {
     const Rec128 *xrec, *yrec;     // by index
     const Rec256 *xpair, *ypair;   // pairs: fw behind the sources, monomials behind the targets
     const float* wx;
-    double Lmax_x, Lmax_y;
+    double wmax_x, wmax_y;         // 2^Lmax of either side
     int n_st0;                     // source tiles
     int n_rec[2], words[2];        // streamed records of side 0 (targets), side 1 (sources)
     int jc_tiles, total_tiles, runs_per_chunk, n_units[2];
@@ -654,19 +654,23 @@ __device__ __forceinline__ void coef_sparse_side(const CoefSparseArgs& a, int gr
     uint16_t* list = reinterpret_cast<uint16_t*>(work + S::kRec) + S::UNITS * 64 * warp;
     double(*sums)[10][32] = reinterpret_cast<double(*)[10][32]>(work + S::kRec + S::kList);
     uint32_t* bits = reinterpret_cast<uint32_t*>(work + S::kRec + S::kList + S::kSums);
-    {
-        ReachArgs r;
-        r.st = SIDE == 0 ? a.x : a.y;
-        r.sm = SIDE == 0 ? a.y : a.x;
-        r.pose = a.pose;
-        r.inv_trace = a.inv_trace;
-        find_reach<D, SIDE == 0>(r, group, bits, sh);
-    }
-    __syncthreads();
     const ReachSide& st = SIDE == 0 ? a.x : a.y;
     const int pos = group * kTile + lane;
     const bool in = pos < st.n;
-    const int i = in ? st.pt[pos].idx : 0;
+    const int i = st.pt[in ? pos : 0].idx;
+    double* const o = (SIDE == 0 ? a.h2 : a.h1) + (size_t)i * 16;
+    ReachArgs reach;
+    reach.st = st;
+    reach.sm = SIDE == 0 ? a.y : a.x;
+    reach.pose = a.pose;
+    reach.inv_trace = a.inv_trace;
+    const bool marked = find_reach<D, SIDE == 0>(reach, group, bits, sh);
+    if (!__syncthreads_or(marked)) {   // nothing reaches these points
+        if (warp == 0 && in)
+#pragma unroll
+            for (int q = 0; q < NF; ++q) o[q] = 0.0;
+        return;
+    }
     float2 PH[3], PL[3], Mx[6], lvs, h[NF];
     {
         const Rec128 r = (SIDE == 0 ? a.xrec : a.yrec)[i];
@@ -737,18 +741,18 @@ __device__ __forceinline__ void coef_sparse_side(const CoefSparseArgs& a, int gr
                 }
             }
         }
+        const unsigned any = __ballot_sync(0xffffffffu, marks != 0);
+        if (!any) continue;
         int at = __popcll(marks);
         const int own = at;
 #pragma unroll
-        for (int o = 1; o < S::UNITS; o <<= 1) {
-            const int v = __shfl_up_sync(0xffffffffu, at, o);
-            if (lane >= o) at += v;
+        for (int k = 1; k < S::UNITS; k <<= 1) {
+            const int v = __shfl_up_sync(0xffffffffu, at, k);
+            if (lane >= k) at += v;
         }
         const int n = __shfl_sync(0xffffffffu, at, S::UNITS - 1);
-        if (n == 0) continue;
         at -= own;
         // a list entry: record - base; 0x8000 on a unit's first, 0x4000 on a source block's first (side 1)
-        unsigned any = __ballot_sync(0xffffffffu, marks != 0);
         const bool opens = SIDE == 1 && (any & ((1u << lane) - 1) & 0xfu << (lane & ~3)) == 0;
         for (bool head = true; marks; head = false) {
             list[at++] = (uint16_t)((r0 - base + __ffsll(marks) - 1) | (head ? 0x8000 | (opens ? 0x4000 : 0) : 0));
@@ -791,9 +795,8 @@ __device__ __forceinline__ void coef_sparse_side(const CoefSparseArgs& a, int gr
     __syncthreads();
     if (warp > 0 || !in) return;
     const double sgm = 1.0 / a.pose[kPoseSig];
-    const double Gs = pow(sgm, (double)D);
-    const double w = SIDE == 0 ? (double)a.wx[i] * (Gs * exp2(a.Lmax_y)) : Gs * exp2(a.Lmax_x + a.Lmax_y);
-    double* o = (SIDE == 0 ? a.h2 : a.h1) + (size_t)i * 16;
+    const double Gs = D == 3 ? sgm * sgm * sgm : sgm * sgm;
+    const double w = SIDE == 0 ? (double)a.wx[i] * (Gs * a.wmax_y) : Gs * a.wmax_x * a.wmax_y;
 #pragma unroll
     for (int q = 0; q < NF; ++q) {
         double t = sums[0][q][lane];
@@ -1582,8 +1585,8 @@ static int coef_fused_launch(Context& c, const double* pose_dev, double* moments
         sa.xpair = static_cast<const Rec256*>(c.xrec256);
         sa.ypair = static_cast<const Rec256*>(c.yrec256);
         sa.wx = c.wx;
-        sa.Lmax_x = c.Lmax_x;
-        sa.Lmax_y = c.Lmax_y;
+        sa.wmax_x = std::exp2(c.Lmax_x);
+        sa.wmax_y = std::exp2(c.Lmax_y);
         sa.n_st0 = (c.N + kTile - 1) / kTile;
         sa.n_rec[0] = c.M_pad / 2;
         sa.n_rec[1] = c.N_pad / 2;

@@ -48,23 +48,26 @@ template <int D>
 __device__ __forceinline__ PoseF pose_f32(const double* pose)
 {
     PoseF p;
-    double f = 0;
     p.tsize = 0.f;
 #pragma unroll
     for (int a = 0; a < D; ++a) {
 #pragma unroll
-        for (int b = 0; b < D; ++b) {
-            double v = a == b ? -1.0 : 0.0;
-#pragma unroll
-            for (int k = 0; k < D; ++k) v = fma(pose[k + D * a], pose[k + D * b], v);
-            f = fma(v, v, f);
-            p.R[a + D * b] = (float)pose[a + D * b];
-        }
+        for (int b = 0; b < D; ++b) p.R[a + D * b] = (float)pose[a + D * b];
         p.t[a] = (float)pose[kPoseT + a];
         p.tsize += fabsf(p.t[a]);
     }
-    // |R v| lies between sqrt(1 - dev) |v| and sqrt(1 + dev) |v|
-    const float dev = sqrtf((float)f) * (1.f + 1e-6f);
+    float f = 0.f;   // |R^T R - I|_F^2
+#pragma unroll
+    for (int a = 0; a < D; ++a)
+#pragma unroll
+        for (int b = 0; b < D; ++b) {
+            float v = a == b ? -1.f : 0.f;
+#pragma unroll
+            for (int k = 0; k < D; ++k) v = fmaf(p.R[k + D * a], p.R[k + D * b], v);
+            f = fmaf(v, v, f);
+        }
+    // |R v| lies between sqrt(1 - dev) |v| and sqrt(1 + dev) |v| (2e-6 for the FP32 products)
+    const float dev = fmaf(sqrtf(f), 1.f + 1e-6f, 2e-6f);
     p.stretch = sqrtf(1.f + dev) * (1.f + 1e-6f);
     p.Lscale = dev < 0.5f ? (1.f + 1e-6f) / (1.f - dev) : INFINITY;
     return p;
@@ -100,10 +103,10 @@ __device__ __forceinline__ float dist2_f32(const float4& p, const float4& q)
 }
 
 // The records that reach tile `group` of the stationary side, into bits (shared, one per record; all
-// 128 threads; the caller zeroes bits before and synchronises after).  POSE_SM: the streamed side is
+// 128 threads; the caller zeroes bits before and synchronises after).  True for a lane that marked any.  POSE_SM: the streamed side is
 // the targets' (moved by the pose), else the stationary side is.
 template <int D, bool POSE_SM>
-__device__ __forceinline__ void find_reach(const ReachArgs& a, int group, uint32_t* bits, ReachShared& sh)
+__device__ __forceinline__ bool find_reach(const ReachArgs& a, int group, uint32_t* bits, ReachShared& sh)
 {
     constexpr int NW = 4, TPW = kSuper / NW;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -153,6 +156,7 @@ __device__ __forceinline__ void find_reach(const ReachArgs& a, int group, uint32
         }
         return m;
     };
+    bool marked = false;
     const int n_tiles = (a.sm.n + kTile - 1) / kTile, n_super = (n_tiles + kSuper - 1) / kSuper;
     for (int base = 0; base < n_super; base += 32) {
         bool go = base + lane < n_super;
@@ -210,9 +214,11 @@ __device__ __forceinline__ void find_reach(const ReachArgs& a, int group, uint32
                     }
                 }
                 if (hit) atomicOr(&bits[s.idx >> 6], 1u << (s.idx >> 1 & 31));
+                marked |= hit;
             }
         }
     }
+    return marked;
 }
 
 }  // namespace dugma

@@ -17,6 +17,8 @@
 // and broadcast from shared memory) less.  Measured on one B200, adjoint kernel, all pairs -> here:
 // 65536 x 65536 harmonic 6300 -> 67 us; 240000 x 239999 depth views 83500 -> 490 us; 6000 x 5501
 // with outliers 70 -> 24 us; 20011 x 17003 in 2D 370 -> 20 us.
+#include <algorithm>
+#include <cmath>
 #include <mutex>
 
 #include "sparse.cuh"
@@ -121,7 +123,7 @@ static int sparse_impl(Context& c, const double* pose_dev, int tile_rec, int chu
     a.yrec = reinterpret_cast<const YRec2*>(c.yrec);
     a.wx = c.wx;
     a.pose = pose_dev;
-    a.Lmax = c.Lmax_y;
+    a.wmax = std::exp2(c.Lmax_y);
     a.n_rec = c.M_pad / 2;
     a.words = (a.n_rec + 31) / 32;
     while (1 << a.tile_shift < tile_rec) ++a.tile_shift;

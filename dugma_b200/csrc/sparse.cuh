@@ -13,7 +13,7 @@ struct SparseArgs {
     const YRec2* yrec;     // by target index, pairs
     const float* wx;
     const double* pose;
-    double Lmax;
+    double wmax;           // 2^Lmax of the targets' weights
     int n_rec, words;      // records, words of their bitmap
     int tile_shift;        // log2 records per tile (FP32 sum of the energy)
     int chunk_rec;         // records per chunk (FP32 sums of the moments)
@@ -45,12 +45,20 @@ __device__ __forceinline__ void sparse_tile(const SparseArgs& a, int group, unsi
     float(*rec)[kSparseBatch * 32] = reinterpret_cast<float(*)[kSparseBatch * 32]>(work) + 2 * warp;
     uint16_t* list = reinterpret_cast<uint16_t*>(work + kSparseRec) + kSparseChunk * warp;
 
-    find_reach<D, true>(a.reach, group, bits, sh);
-    __syncthreads();
-
     const int pos = group * kTile + lane;
     const bool in = pos < a.reach.st.n;
-    const int i = in ? a.reach.st.pt[pos].idx : 0;
+    const int i = a.reach.st.pt[in ? pos : 0].idx;
+    const bool marked = find_reach<D, true>(a.reach, group, bits, sh);
+    if (!__syncthreads_or(marked)) {   // nothing reaches these sources
+        if (warp == 0 && in) {
+#pragma unroll
+            for (int v = 0; v < NV; ++v) a.rows[(size_t)i * 8 + v] = 0.0;
+            if (GRAD && a.dx)
+#pragma unroll
+                for (int q = 0; q < D; ++q) a.dx[(size_t)i * D + q] = 0.0;
+        }
+        return;
+    }
     Body body;
     {
         float x[3], b[6];
@@ -70,6 +78,7 @@ __device__ __forceinline__ void sparse_tile(const SparseArgs& a, int group, unsi
         // the chunk's marked records, ascending
         const int nw = (min(a.chunk_rec, a.n_rec - base) + 31) / 32;
         uint32_t w = lane < nw ? bits[base / 32 + lane] : 0u;
+        if (!__any_sync(0xffffffffu, w != 0)) continue;
         int at = __popc(w);
         const int own = at;
 #pragma unroll
@@ -78,7 +87,6 @@ __device__ __forceinline__ void sparse_tile(const SparseArgs& a, int group, unsi
             if (lane >= o) at += u;
         }
         const int n = __shfl_sync(0xffffffffu, at, 31);
-        if (n == 0) continue;
         at -= own;
         while (w) {
             list[at++] = (uint16_t)(32 * lane + __ffs(w) - 1);
@@ -136,12 +144,12 @@ __device__ __forceinline__ void sparse_tile(const SparseArgs& a, int group, unsi
         return s;
     };
     const double sg = 1.0 / a.pose[kPoseSig];
-    const double wt = (double)a.wx[i] * pow(sg, (double)D) * exp2(a.Lmax);
+    const double wt = (double)a.wx[i] * (D == 3 ? sg * sg * sg : sg * sg) * a.wmax;
     double acc[NV], dx[3] = {0, 0, 0};
 #pragma unroll
     for (int v = 0; v < NV; ++v) acc[v] = 0.0;
     acc[0] = wt * total(0);
-    if constexpr (GRAD) {
+    if constexpr (GRAD) if (acc[0] != 0.0) {   // (no term, no moments)
         double s1[3], d2[3], q2[6];
 #pragma unroll
         for (int q = 0; q < D; ++q) {
@@ -154,10 +162,10 @@ __device__ __forceinline__ void sparse_tile(const SparseArgs& a, int group, unsi
 #pragma unroll
         for (int q = 0; q < D; ++q) t[q] = a.pose[kPoseT + q];
         chol_contract<D>(wt, body.B[0], body.X[0], t, s1, d2, q2, acc, dx);
-        if (a.dx)
-#pragma unroll
-            for (int q = 0; q < D; ++q) a.dx[(size_t)i * D + q] = dx[q];
     }
+    if (GRAD && a.dx)
+#pragma unroll
+        for (int q = 0; q < D; ++q) a.dx[(size_t)i * D + q] = dx[q];
 #pragma unroll
     for (int v = 0; v < NV; ++v) a.rows[(size_t)i * 8 + v] = acc[v];
 }
