@@ -191,6 +191,8 @@ int timing_end(Context& c, cudaStream_t s);
 // chunk_rec records.  go (nullable, device): nothing is done unless it is set.
 constexpr double kSparseMinPairs = 4e6, kSparseMinPairsAuto = 64e6, kSparseCoefMinPairs = 24e6;
 constexpr int kSparseMaxTargets = 1 << 20;
+constexpr int kRowBlocks = 256;
+int reduce_rows(Context& c, int nv, double* out_dev, cudaStream_t s, double* host_out, const int* go);
 double sparse_sigma(const Context& c);   // evaluations with a sigma below this go that way
 int sparse_launch(Context& c, const double* pose_dev, bool grad, int tile_rec, int chunk_rec, double* out_dev,
                   double* dEdx_dev, cudaStream_t s, double* host_out, const int* go);

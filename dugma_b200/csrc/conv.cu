@@ -20,10 +20,13 @@
 // The packed kernels run every pair of a tile through the FP32 fast path without a branch
 // and only flag a pair that fails the test; a flagged tile is redone from the per-source
 // sums saved at its start with the exact per-pair rules, so the common case is straight-line.
+#include <algorithm>
 #include <cmath>
+#include <mutex>
 
 #include "context.hpp"
 #include "pairs.cuh"
+#include "reach.cuh"
 
 namespace dugma {
 
@@ -826,6 +829,155 @@ __global__ void __launch_bounds__(NT, MINB) conv_kernel(PairArgs a)
 }
 
 
+// ---------------------------------------------------------------------------
+// The pairs whose term is not 0 (sparse.cu's way): a block takes a tile of 32 sources, marks the target
+// records that can reach one of them and evaluates those, with the packed body's own tiles, items
+// and exact rules; each source's contribution goes to its row.
+// A pair counts nothing where its exponent E = |k| d^T S^-1 d >= |k| |d|^2 / (sig (L_i + L_j)) is
+//   - in the fast path (FP32, flushed below 2^-126) above 285: a pair passes the fast path's test when
+//     det is at least 1e-6 of the diagonal's product, and then FP32 has E to a factor 0.45 at worst;
+//   - in the FP64 path (its term a float, 0 below 2^-149) above 150 + log2(det^-1/2), with det at least
+//     (2 / largest inverse trace / c)^D.
+// Every covariance has to be positive definite for the bound on S.  Bound like sparse_kernel by the
+// search.  Measured on one B200, 16000 x 16384 harmonic surface, energy_grad per call: 758 us over all
+// pairs, 85 us here.
+// ---------------------------------------------------------------------------
+struct ConvSparseArgs {
+    ReachArgs reach;
+    PairArgs pair;         // xrec, yrec, ycov, pose, Lmax (the covariance scale)
+    int n_rec, words, tile_shift, chunk_rec;
+    double *rows, *dx;     // [N][8]; [N][D] or null
+};
+
+struct ConvSparseShape {
+    static constexpr int BATCH = 4, CHUNK = 512;
+    static constexpr size_t kRec = 4 * 2 * BATCH * sizeof(YRec2), kList = 4 * CHUNK * sizeof(uint16_t),
+                            kSums = 4 * 10 * 32 * sizeof(double);
+    static constexpr size_t kFixed = (sizeof(ReachShared) + 15) / 16 * 16 + kRec + kList + kSums;
+};
+
+template <int D, bool GRAD>
+__global__ void __launch_bounds__(128, 3) conv_sparse_kernel(ConvSparseArgs a)
+{
+    using S = ConvSparseShape;
+    using Body = PackedConvBody<D, 1, GRAD, 128>;
+    constexpr int NS = Sym<D>::N, NV = Body::NV;
+    extern __shared__ __align__(16) unsigned char smem[];
+    ReachShared& sh = *reinterpret_cast<ReachShared*>(smem);
+    unsigned char* work = smem + (sizeof(ReachShared) + 15) / 16 * 16;
+    uint32_t* bits = reinterpret_cast<uint32_t*>(smem + S::kFixed);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    float(*rec)[S::BATCH * 32] = reinterpret_cast<float(*)[S::BATCH * 32]>(work) + 2 * warp;
+    uint16_t* list = reinterpret_cast<uint16_t*>(work + S::kRec) + S::CHUNK * warp;
+    double(*sums)[10][32] = reinterpret_cast<double(*)[10][32]>(work + S::kRec + S::kList);
+    pdl_trigger();
+    for (int w = threadIdx.x; w < a.words; w += 128) bits[w] = 0;
+    pdl_wait();
+    const int pos = blockIdx.x * kTile + lane;
+    const bool in = pos < a.reach.st.n;
+    const int i = a.reach.st.pt[in ? pos : 0].idx;
+    const bool marked = find_reach<D, true, true>(a.reach, blockIdx.x, bits, sh);
+    double acc[NV], dx[3] = {0, 0, 0};
+#pragma unroll
+    for (int v = 0; v < NV; ++v) acc[v] = 0.0;
+    if (__syncthreads_or(marked)) {
+        // one source per lane: the body's row range is that row, its dE/dx partial goes to dxl
+        double dxl[3] = {0, 0, 0};
+        PairArgs pa = a.pair;
+        pa.i0 = i;
+        pa.i_end = i + 1;
+        pa.dx_part = GRAD && a.dx ? dxl : nullptr;
+        Body body;
+        body.setup(pa);
+        body.load_src(pa, 0, i);
+        body.zero_all();
+        const float* recs = static_cast<const float*>(pa.yrec);
+        for (int base = warp * a.chunk_rec; base < a.n_rec; base += 4 * a.chunk_rec) {
+            const int nw = (min(a.chunk_rec, a.n_rec - base) + 31) / 32;
+            uint32_t w = lane < nw ? bits[base / 32 + lane] : 0u;
+            if (!__any_sync(0xffffffffu, w != 0)) continue;
+            int at = __popc(w);
+            const int own = at;
+#pragma unroll
+            for (int o = 1; o < 16; o <<= 1) {
+                const int u = __shfl_up_sync(0xffffffffu, at, o);
+                if (lane >= o) at += u;
+            }
+            const int n = __shfl_sync(0xffffffffu, at, 15);
+            at -= own;
+            while (w) {
+                list[at++] = (uint16_t)(32 * lane + __ffs(w) - 1);
+                w &= w - 1;
+            }
+            __syncwarp();
+            float v[S::BATCH];
+            auto fetch = [&](int b) {
+#pragma unroll
+                for (int k = 0; k < S::BATCH; ++k)
+                    v[k] = recs[(size_t)(base + list[min(b + k, n - 1)]) * 32 + lane];
+            };
+            int tile = list[0] >> a.tile_shift, first = 0;
+            // the end of a tile whose records are list[first, last)
+            auto end_tile = [&](int last) {
+                body.j0 = base;
+                if (body.bad) {   // redone by the exact rules
+                    body.restore();
+                    body.e[0] = make_float2(0.f, 0.f);
+                    for (int k = first; k < last; ++k)
+                        body.template pass<true>(static_cast<const YRec2*>(pa.yrec)[base + list[k]], base + list[k]);
+                    body.bad = false;
+                }
+                body.E64[0] += (double)body.e[0].x + (double)body.e[0].y;
+                body.e[0] = make_float2(0.f, 0.f);
+                body.save();
+                first = last;
+            };
+            fetch(0);
+            for (int b = 0, buf = 0; b < n; b += S::BATCH, buf ^= 1) {
+#pragma unroll
+                for (int k = 0; k < S::BATCH; ++k) rec[buf][32 * k + lane] = v[k];
+                __syncwarp();
+                if (b + S::BATCH < n) fetch(b + S::BATCH);
+                const YRec2* r = reinterpret_cast<const YRec2*>(rec[buf]);
+                const int m = min(S::BATCH, n - b);
+                for (int k = 0; k < m; ++k) {
+                    const int l = list[b + k], t = l >> a.tile_shift;
+                    if (t != tile) {
+                        end_tile(b + k);
+                        tile = t;
+                    }
+                    body.template pass<false>(r[k], base + l);
+                }
+            }
+            end_tile(n);
+            // the item's end: its sums into the source's contribution, and the body as new
+            body.finish(pa, 0, acc);
+#pragma unroll
+            for (int q = 0; q < D; ++q) dx[q] += dxl[q];
+            body.zero_all();
+            __syncwarp();   // (the list is rewritten)
+        }
+    }
+#pragma unroll
+    for (int v = 0; v < NV; ++v) sums[warp][v][lane] = acc[v];
+    if (GRAD)
+#pragma unroll
+        for (int q = 0; q < D; ++q) sums[warp][7 + q][lane] = dx[q];
+    __syncthreads();
+    if (warp > 0 || !in) return;
+    auto total = [&](int q) {
+        double s = sums[0][q][lane];
+#pragma unroll
+        for (int u = 1; u < 4; ++u) s += sums[u][q][lane];
+        return s;
+    };
+#pragma unroll
+    for (int v = 0; v < NV; ++v) a.rows[(size_t)i * 8 + v] = total(v);
+    if (GRAD && a.dx)
+#pragma unroll
+        for (int q = 0; q < D; ++q) a.dx[(size_t)i * D + q] = total(7 + q);
+}
+
 struct ConvVariant {
     KernelShape shape;
     KernelFn fn;
@@ -864,8 +1016,53 @@ std::vector<KernelShape> conv_shapes(bool grad)
     return s;
 }
 
+template <int D, bool GRAD>
+static int conv_sparse_launch(Context& c, KernelFn fn, const KernelShape& sh, const double* pose_dev, double* out_dev,
+                              double* dEdx_dev, cudaStream_t s, double cut)
+{
+    using S = ConvSparseShape;
+    static std::mutex mu;
+    static bool done[64];
+    {
+        std::lock_guard<std::mutex> lk(mu);
+        if (c.dev >= 64 || !done[c.dev]) {
+            DUGMA_CK(cudaFuncSetAttribute(conv_sparse_kernel<D, GRAD>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                          (int)(S::kFixed + kSparseMaxTargets / 64 * sizeof(uint32_t))));
+            if (c.dev < 64) done[c.dev] = true;
+        }
+    }
+    const size_t rows = (size_t)c.N * 8;
+    DUGMA_RET(c.ensure_scratch(sizeof(double) * (rows + kRowBlocks * 8)));
+    int jc_tiles = 0, n_jc = 0;
+    pair_split(c, fn, sh, c.N, (size_t)c.M_pad / 2, &jc_tiles, &n_jc);
+    ConvSparseArgs a{};
+    a.reach = {{c.xpt, c.xtile, c.xsub, c.xsuper, c.N}, {c.ypt, c.ytile, c.ysub, c.ysuper, c.M}, pose_dev, c.inv_trace,
+               (float)cut, (float)(1e9 * c.cscale)};
+    a.pair.xrec = c.xrec;
+    a.pair.yrec = c.yrec;
+    a.pair.ycov = c.ycov;
+    a.pair.xcov = c.xcov;
+    a.pair.pose = pose_dev;
+    a.pair.Lmax = c.cscale;
+    a.pair.N = c.N;
+    a.n_rec = c.M_pad / 2;
+    a.words = (a.n_rec + 31) / 32;
+    while (1 << a.tile_shift < sh.tj) ++a.tile_shift;
+    // (an item's largest term is redone in FP64, so energies too need the items' chunks)
+    a.chunk_rec = jc_tiles * sh.tj;
+    if (a.chunk_rec > S::CHUNK) return set_error(DUGMA_ERR_STATE, "sparse CONV: chunks of %d records", a.chunk_rec);
+    a.rows = c.scratch;
+    a.dx = dEdx_dev;
+    DUGMA_CK(cudaMemsetAsync(c.counter, 0, 2 * sizeof(int), s));
+    DUGMA_RET(timing_begin(c, s));
+    conv_sparse_kernel<D, GRAD><<<(c.N + kTile - 1) / kTile, 128, S::kFixed + sizeof(uint32_t) * a.words, s>>>(a);
+    DUGMA_CK(cudaGetLastError());
+    DUGMA_RET(timing_end(c, s));
+    return reduce_rows(c, GRAD ? 1 + (D == 3 ? 6 : 3) : 1, out_dev, s, nullptr, nullptr);
+}
+
 int conv_launch(Context& c, const double* pose_dev, bool grad, int i0, int i1, double* out_dev, double* dEdx_dev,
-                cudaStream_t s, const KernelShape* force)
+                cudaStream_t s, const KernelShape* force, double sig)
 {
     const KernelShape want = force ? *force : (grad ? c.shape_conv_adj : c.shape_conv_energy);
     const std::vector<ConvVariant>& vars = c.D == 3 ? conv_variants<3>(grad) : conv_variants<2>(grad);
@@ -894,6 +1091,15 @@ int conv_launch(Context& c, const double* pose_dev, bool grad, int i0, int i1, d
         DUGMA_CK(cudaGetLastError());
     }
     const int nv = grad ? 1 + (c.D == 3 ? 6 : 3) : 1;
+    if (packed && !force && i0 == 0 && i1 == c.N && sig > 0.0) {
+        const double cut = 2.0 + std::max(285.0, 150.0 + 0.5 * c.D * std::log2(std::max(1.0, 0.5 * c.cscale * c.inv_trace)));
+        // the reach's rule as the energy's (sparse_sigma), with this cut and two variances
+        if (c.nonpd == 0 && sig < sparse_sigma(c) * kFlushExp / (2.0 * cut))
+            return c.D == 3 ? (grad ? conv_sparse_launch<3, true>(c, v->fn, v->shape, pose_dev, out_dev, dEdx_dev, s, cut)
+                                    : conv_sparse_launch<3, false>(c, v->fn, v->shape, pose_dev, out_dev, nullptr, s, cut))
+                            : (grad ? conv_sparse_launch<2, true>(c, v->fn, v->shape, pose_dev, out_dev, dEdx_dev, s, cut)
+                                    : conv_sparse_launch<2, false>(c, v->fn, v->shape, pose_dev, out_dev, nullptr, s, cut));
+    }
     return launch_pair_variant(c, v->fn, v->shape, c.xrec, c.yrec, (size_t)c.M_pad / v->shape.pack, nv, c.cscale,
                                pose_dev, i0, i1, out_dev, grad ? dEdx_dev : nullptr, nullptr, 0, nullptr, s);
 }

@@ -156,7 +156,7 @@ std::vector<KernelShape> energy_shapes()
 }
 
 int conv_launch(Context& c, const double* pose_dev, bool grad, int i0, int i1, double* out_dev, double* dEdx_dev,
-                cudaStream_t s, const KernelShape* force);   // conv.cu
+                cudaStream_t s, const KernelShape* force, double sig);   // conv.cu
 
 static int occupancy_blocks(KernelFn fn, int nt)
 {
@@ -278,7 +278,8 @@ int launch_pairs(Context& c, const double* pose_dev, int model, bool grad, int i
                  double* dEdx_dev, cudaStream_t s, const KernelShape* force, const EvalIO* io)
 {
     if (i0 < 0 || i1 > c.N || i0 >= i1) return set_error(DUGMA_ERR_ARG, "bad source row range [%d, %d)", i0, i1);
-    if (model == DUGMA_MODEL_CONV) return conv_launch(c, pose_dev, grad, i0, i1, out_dev, dEdx_dev, s, force);
+    if (model == DUGMA_MODEL_CONV) 
+        return conv_launch(c, pose_dev, grad, i0, i1, out_dev, dEdx_dev, s, force, io ? io->sig : 0.0);
     if (model == DUGMA_MODEL_REF_F64) {
         if (grad)
             return set_error(DUGMA_ERR_ARG, "the FP64 reference-precision model has no adjoint (use the "

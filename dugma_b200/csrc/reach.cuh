@@ -8,8 +8,9 @@
 //
 // find_reach marks, for one tile of 32 stationary points, the records (pairs of streamed points by
 // index) of which a point passes that test for some stationary point: super tiles against the
-// tile's four subgroups, tiles against them, points against them, then points against points.  The
-// tests run in FP32 with room for their rounding, for that of the evaluation (in L, see variance_bound)
+// tile's four subgroups, tiles against them, points against them, then points against points.
+// CONV: the pair's matrix is the sum of both covariances, so the test is |d|^2 > (sig / |k|) cut (L_i + L_j).
+// The tests run in FP32 with room for their rounding, for that of the evaluation (in L, see variance_bound)
 // and for what a pose that is no exact rotation stretches.  What is not finite, or so large that the
 // evaluation could overflow, is marked.
 #pragma once
@@ -28,6 +29,8 @@ struct ReachArgs {
     ReachSide st, sm;      // stationary, streamed
     const double* pose;
     float inv_trace;       // largest trace of an inverse covariance (overflow limit)
+    float cut, big;        // CONV: the exponent that leaves nothing, and the variance beyond which nothing
+                           // is left out (conv.cu)
 };
 
 // one block of 4 warps
@@ -105,7 +108,7 @@ __device__ __forceinline__ float dist2_f32(const float4& p, const float4& q)
 // The records that reach tile `group` of the stationary side, into bits (shared, one per record; all
 // 128 threads; the caller zeroes bits before and synchronises after).  True for a lane that marked any.  POSE_SM: the streamed side is
 // the targets' (moved by the pose), else the stationary side is.
-template <int D, bool POSE_SM>
+template <int D, bool POSE_SM, bool CONV = false>
 __device__ __forceinline__ bool find_reach(const ReachArgs& a, int group, uint32_t* bits, ReachShared& sh)
 {
     constexpr int NW = 4, TPW = kSuper / NW;
@@ -113,7 +116,11 @@ __device__ __forceinline__ bool find_reach(const ReachArgs& a, int group, uint32
     const PoseF P = pose_f32<D>(a.pose);
     const float sigk = (float)(a.pose[kPoseSig] * (1.0 / -K_EXP2)) * (1.f + 1e-6f);
     // beyond this squared distance a form could overflow, and 0 x inf is no 0
-    const float d2max = fminf(1e36f * sigk / (a.inv_trace + 1e-30f), 1e30f);
+    const float d2max = CONV ? 1e20f : fminf(1e36f * sigk / (a.inv_trace + 1e-30f), 1e30f);
+    // the squared distance beyond which a pair of these a and L counts nothing
+    auto reach2 = [&](float a0, float L0, float a1, float L1) {
+        return CONV ? (L0 + L1 < a.big ? sigk * a.cut * (L0 + L1) : INFINITY) : sigk * fminf(a0, a1) * fmaxf(L0, L1);
+    };
     // a sphere or point as the tests see it
     auto place = [&](const float* c, float& r, bool posed) {
         float4 q = make_float4(c[0], c[1], D == 3 ? c[2] : 0.f, 0.f);
@@ -148,7 +155,7 @@ __device__ __forceinline__ bool find_reach(const ReachArgs& a, int group, uint32
         for (int s = 0; s < 4; ++s) {
             const float4 c = sh.sub[s];
             const float2 e = sh.sa[s];
-            const float T = sigk * fminf(aa, e.x) * fmaxf(L, e.y);
+            const float T = reach2(aa, L, e.x, e.y);
             const float rr = r + c.w, reach = fmaf(sqrt_fast(fmaxf(T, 0.f)), 1.f + 2e-6f, rr);
             const float d2 = dist2_f32<D>(q, c);
             const bool out = d2 * (1.f - 1e-5f) > reach * reach && d2 < 0.2f * d2max && rr * rr < 0.2f * d2max;
@@ -207,7 +214,7 @@ __device__ __forceinline__ bool find_reach(const ReachArgs& a, int group, uint32
                     for (int e = 0; e < kSub; ++e) {
                         const float4 c = sh.pt[g * kSub + e];
                         const float2 ca = sh.pa[g * kSub + e];
-                        const float T = sigk * fminf(s.a, ca.x) * fmaxf(L, c.w);
+                        const float T = reach2(s.a, L, ca.x, c.w);
                         const float d2 = dist2_f32<D>(q, c);
                         // (d - slack)^2 > T follows from d^2 > 1.001 T + 1001 slack^2
                         hit |= (m >> g & 1u) && !(d2 > fmaf(T, 1.002f, slack + ca.y) && d2 < d2max);

@@ -39,7 +39,6 @@ __global__ void __launch_bounds__(128, 6) sparse_kernel(SparseArgs a, const int*
 
 // out[v] = sum of rows[i][v]: per-block partials over contiguous slices, then the block that finishes
 // last adds the partials, all in fixed order (deterministic).  host_out as in reduce_items_kernel.
-constexpr int kRowBlocks = 256;
 __global__ void __launch_bounds__(256) reduce_rows_kernel(const double* rows, int n, int nv, double* part, int* ticket,
                                                           double* out, double* host_out, const int* err,
                                                           const int* go)
@@ -85,6 +84,16 @@ __global__ void __launch_bounds__(256) reduce_rows_kernel(const double* rows, in
         if (host_out) host_out[v] = s;
     }
     if (threadIdx.x == 0 && host_out) host_out[nv] = (double)*err;
+}
+
+// the rows c.scratch holds (N x 8) into out_dev; the blocks' partials go behind them
+int reduce_rows(Context& c, int nv, double* out_dev, cudaStream_t s, double* host_out, const int* go)
+{
+    double* rows = c.scratch;
+    DUGMA_CK(launch_dependent(c.pdl, reduce_rows_kernel, std::min(kRowBlocks, (c.N + 255) / 256), 256, 0, s,
+                              (const double*)rows, c.N, nv, rows + (size_t)c.N * 8, c.counter + 1, out_dev, host_out,
+                              (const int*)c.err, go));
+    return DUGMA_OK;
 }
 
 // Which of a context's evaluations go this way: one whose sigma is below this.  The reach of a pair is
@@ -134,11 +143,7 @@ static int sparse_impl(Context& c, const double* pose_dev, int tile_rec, int chu
     DUGMA_RET(timing_begin(c, s));
     DUGMA_CK(launch_dependent(c.pdl, sparse_kernel<D, GRAD>, grid, 128, kSparseFixed + sizeof(uint32_t) * a.words, s, a, go));
     DUGMA_RET(timing_end(c, s));
-    const int nv = GRAD ? 1 + (D == 3 ? 6 : 3) : 1;
-    DUGMA_CK(launch_dependent(c.pdl, reduce_rows_kernel, std::min(kRowBlocks, (c.N + 255) / 256), 256, 0, s,
-                              (const double*)a.rows, c.N, nv, c.scratch + rows, c.counter + 1, out_dev, host_out,
-                              (const int*)c.err, go));
-    return DUGMA_OK;
+    return reduce_rows(c, GRAD ? 1 + (D == 3 ? 6 : 3) : 1, out_dev, s, host_out, go);
 }
 
 int sparse_launch(Context& c, const double* pose_dev, bool grad, int tile_rec, int chunk_rec, double* out_dev,

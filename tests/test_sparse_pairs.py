@@ -37,6 +37,9 @@ def _problem(kind, n, m, seed):
     elif kind == "mixed_scales":
         XC *= np.exp(rng.uniform(-4, 4, n))[:, None, None]
         YC *= np.exp(rng.uniform(-4, 4, m))[:, None, None]
+    elif kind == "nearly_singular":   # flat covariances, some along the same plane: the FP64 path
+        flat = np.diag([1e-3, 1e-3, 1e-11][:D])
+        XC[::2], YC[::3] = flat, P.R_G.T @ flat @ P.R_G
     elif kind == "not_finite":
         Y[3, 0] = np.inf
     elif kind == "huge":
@@ -49,6 +52,8 @@ ENERGY = {"grad": lambda h, R, t, sig: api.energy_grad(h, R, t, sig)[:2],
           "grad_dx": lambda h, R, t, sig: api.energy_grad(h, R, t, sig, with_dx=True),
           "energy": lambda h, R, t, sig: (api.energy(h, R, t, sig),),
           "fd": lambda h, R, t, sig: (api.energy_fd_grad(h, R, t, sig)[0],)}
+CONV = {"conv_grad": lambda h, R, t, sig: api.energy_grad(h, R, t, sig, model=1, with_dx=True),
+        "conv_energy": lambda h, R, t, sig: (api.energy(h, R, t, sig, model=1),)}
 COEF = {"compi": lambda h, R, t, sig: (api.compi(h, R, t, sig=sig),)}
 
 
@@ -96,6 +101,13 @@ def _compare(monkeypatch, calls, kind, n, m, sigs):
 @pytest.mark.parametrize("kind", KINDS)
 def test_energy_same_sums_as_all_pairs(kind, n, m, monkeypatch):
     _compare(monkeypatch, ENERGY, kind, n, m, (2e-4, 4e-3, 3e-2))
+
+
+@pytest.mark.filterwarnings("ignore")
+@pytest.mark.parametrize("n,m", [(2049, 2001), (5000, 901), (1025, 4097)])
+@pytest.mark.parametrize("kind", KINDS + ["nearly_singular"])
+def test_conv_same_sums_as_all_pairs(kind, n, m, monkeypatch):
+    _compare(monkeypatch, CONV, kind, n, m, (2e-4, 2e-3, 8e-3))
 
 
 @pytest.mark.filterwarnings("ignore")
