@@ -618,7 +618,7 @@ int dugma_batch_create(int n_problems, int D, const int* N, const int* M, const 
         b->ctx.push_back(find_context(&b->ptrs[6 * (size_t)p]));
         if (b->ctx.back()->x_indef > 0) b->chol = false;
     }
-    for (const Context* c : b->ctx) b->below.push_back(b->chol ? sparse_sigma(*c) : 0.0);
+    for (const Context* c : b->ctx) b->below.push_back(b->chol ? sparse_sigma(*c, SparseUse::batch) : 0.0);
     if (cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking) != cudaSuccess) {
         for (int k = 0; k < n_problems; ++k) dugma_fr_m(&b->ptrs[6 * (size_t)k]);
         delete b;

@@ -1635,14 +1635,10 @@ static int coef_impl(Context& c, double* pose_dev, double* moments_dev, cudaStre
     // the Cholesky form of every matrix when every weighted point's inverse covariance has a factor,
     // else the Horner form throughout
     const bool chol = c.ux && c.x_indef == 0 && c.y_indef == 0;
-    // The sparse pass by the rule of the energy's (sparse_sigma).  A call and an EM step at the same
-    // sigma go the same way (their coefficients are the same bits); in the EM step, where only the device
-    // knows sigma, both passes are enqueued and the prologue's flag lets one run, so the pass is taken up
-    // from kSparseCoefMinPairs pairs, where the launch that returns at once is lost in the other.
-    const double below = fused && chol && c.coef_kernel == 0 && c.N <= kSparseMaxTargets &&
-                                 (double)c.N * c.M >= kSparseCoefMinPairs
-                             ? sparse_sigma(c)
-                             : 0.0;
+    // The sparse pass by sparse_sigma's rule.  A call and an EM step at the same sigma go the same way
+    // (their coefficients are the same bits); in the EM step, where only the device knows sigma, both
+    // passes are enqueued and the prologue's flag lets one run.
+    const double below = fused && chol && c.coef_kernel == 0 ? sparse_sigma(c, SparseUse::coef) : 0.0;
     const double sig = o.pose_value ? o.pose_value[kPoseSig] : 0.0;
     const bool both = !(sig > 0.0) && below > 0.0;
     const bool sparse = both || (sig > 0.0 && sig < below);

@@ -45,6 +45,7 @@ struct KernelShape {
     int max_chunk = 0;   // most streamed records one work item may cover (0: no limit)
     int min_chunk = 0;   // fewest streamed records per work item (0: no limit); bounds the
                          // per-chunk partial buffers of the coefficient passes
+    int fixed_tiles = 0; // tiles per chunk when they are given (0: pair_split's rule)
     bool valid() const { return ipt > 0; }
     bool same(const KernelShape& o) const { return ipt == o.ipt && nt == o.nt && tj == o.tj && pack == o.pack; }
 };
@@ -189,11 +190,12 @@ int timing_end(Context& c, cudaStream_t s);
 // The REF energy or adjoint over the pairs above the FP32 flush (sparse.cu), from the records of the
 // packed kernels' prologue: the same sums as the all-pairs kernel with tiles of tile_rec and chunks of
 // chunk_rec records.  go (nullable, device): nothing is done unless it is set.
-constexpr double kSparseMinPairs = 4e6, kSparseMinPairsAuto = 64e6, kSparseCoefMinPairs = 24e6;
+constexpr double kSparseMinPairsAuto = 256e6, kSparseCoefMinPairs = 24e6;
 constexpr int kSparseMaxTargets = 1 << 20;
 constexpr int kRowBlocks = 256;
 int reduce_rows(Context& c, int nv, double* out_dev, cudaStream_t s, double* host_out, const int* go);
-double sparse_sigma(const Context& c);   // evaluations with a sigma below this go that way
+enum class SparseUse { energy, coef, conv, batch };
+double sparse_sigma(const Context& c, SparseUse use);   // evaluations with a sigma below this go that way
 int sparse_launch(Context& c, const double* pose_dev, bool grad, int tile_rec, int chunk_rec, double* out_dev,
                   double* dEdx_dev, cudaStream_t s, double* host_out, const int* go);
 // Nearest-neighbour prologue: only the target records of the search (c.yp32), y' = R y + t as the

@@ -1093,8 +1093,7 @@ int conv_launch(Context& c, const double* pose_dev, bool grad, int i0, int i1, d
     const int nv = grad ? 1 + (c.D == 3 ? 6 : 3) : 1;
     if (packed && !force && i0 == 0 && i1 == c.N && sig > 0.0) {
         const double cut = 2.0 + std::max(285.0, 150.0 + 0.5 * c.D * std::log2(std::max(1.0, 0.5 * c.cscale * c.inv_trace)));
-        // the reach's rule as the energy's (sparse_sigma), with this cut and two variances
-        if (c.nonpd == 0 && sig < sparse_sigma(c) * kFlushExp / (2.0 * cut))
+        if (c.nonpd == 0 && sig < sparse_sigma(c, SparseUse::conv))
             return c.D == 3 ? (grad ? conv_sparse_launch<3, true>(c, v->fn, v->shape, pose_dev, out_dev, dEdx_dev, s, cut)
                                     : conv_sparse_launch<3, false>(c, v->fn, v->shape, pose_dev, out_dev, nullptr, s, cut))
                             : (grad ? conv_sparse_launch<2, true>(c, v->fn, v->shape, pose_dev, out_dev, dEdx_dev, s, cut)

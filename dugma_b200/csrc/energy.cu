@@ -142,6 +142,18 @@ static const Variant& energy_fallback()
     return v;
 }
 
+// small_shape's kernels: one source per thread, or two (energies), with the tiles of the default shapes
+template <int D, bool GRAD, bool CHOL>
+static KernelFn small_kernel(int ipt)
+{
+    if constexpr (GRAD)
+        return pair_kernel<PackedBody<D, 1, true, CHOL>, 64, 64>;
+    else
+        return ipt == 1 ? pair_kernel<PackedBody<D, 1, false, CHOL>, 64, 32> : pair_kernel<PackedBody<D, 2, false, CHOL>, 64, 32>;
+}
+
+static void small_shape(const Context& c, bool grad, bool chol, int rows, KernelFn* fn, KernelShape* sh);
+
 std::vector<KernelShape> adjoint_shapes()
 {
     std::vector<KernelShape> s;
@@ -178,6 +190,11 @@ void pair_split(const Context& c, KernelFn fn, const KernelShape& sh, int rows, 
     const int n_ib = (rows + BI - 1) / BI;
     const int total_tiles = (int)(yrec_size / sh.tj);
     const int resident = c.num_sms * occupancy_blocks(fn, sh.nt);
+    if (sh.fixed_tiles > 0) {
+        *jc_tiles_out = std::min(sh.fixed_tiles, total_tiles);
+        *n_jc_out = (total_tiles + *jc_tiles_out - 1) / *jc_tiles_out;
+        return;
+    }
     const int target = 4 * resident;
     int n_jc = std::max(1, std::min(total_tiles, (target + n_ib - 1) / n_ib));
     // small problems: rather than many one-tile items (each pays the per-item set-up, FP64
@@ -189,6 +206,35 @@ void pair_split(const Context& c, KernelFn fn, const KernelShape& sh, int rows, 
     n_jc = std::min(n_jc, total_tiles);
     *jc_tiles_out = (total_tiles + n_jc - 1) / n_jc;
     *n_jc_out = (total_tiles + *jc_tiles_out - 1) / *jc_tiles_out;
+}
+
+// Small problems take fewer sources per thread than the default shapes, on the default's own tiles and
+// chunks (so each source's FP32 sums stay what they are; only FP64 additions regroup): with four a
+// thread the items are too few, or too uneven, for 148 SMs.  One B200, us a call, 4 / 2 / 1 sources:
+//   adjoint  1000: 49 / 37 / 33;  2000: 47 / 36 / 36;  4500: 90 / 76 / 69;  7000: 119 / 121 / 112;  9000: 180 / 184 / 172;
+//            12000: 265 / 272 / 276;  65536: 6337 / 6460 / 6870
+//   energy   1000: 30 / 26.5 / 25.6;  2000: 29.5 / 29.9 / 30.6;  3000: 34.2 / 35.6 / 38;  4500: 52 / 49.5 / 52;  7000:
+//            79 / 74.5 / 83;  9000: 119 / 109 / 127;  12000: 174 / 174 / 188
+static void small_shape(const Context& c, bool grad, bool chol, int rows, KernelFn* fn, KernelShape* sh)
+{
+    if (sh->ipt != 4 || sh->tj != (grad ? 64 : 32)) return;
+    const double pairs = (double)rows * c.M;
+    int ipt = 0;
+    if (grad)
+        ipt = pairs < 8.2e7 ? 1 : 0;
+    else
+        ipt = pairs < 2.5e6 ? 1 : (pairs >= 1.1e7 && pairs < 8.2e7 ? 2 : 0);
+    if (ipt == 0) return;
+    int n_jc = 0;
+    pair_split(c, *fn, *sh, rows, (size_t)c.M_pad / 2, &sh->fixed_tiles, &n_jc);
+    sh->ipt = ipt;
+    sh->nt = 64;
+    if (c.D == 3)
+        *fn = grad ? (chol ? small_kernel<3, true, true>(ipt) : small_kernel<3, true, false>(ipt))
+                   : (chol ? small_kernel<3, false, true>(ipt) : small_kernel<3, false, false>(ipt));
+    else
+        *fn = grad ? (chol ? small_kernel<2, true, true>(ipt) : small_kernel<2, true, false>(ipt))
+                   : (chol ? small_kernel<2, false, true>(ipt) : small_kernel<2, false, false>(ipt));
 }
 
 int timing_begin(Context& c, cudaStream_t s)
@@ -301,6 +347,9 @@ int launch_pairs(Context& c, const double* pose_dev, int model, bool grad, int i
                      : (grad ? &adjoint_fallback<2>() : &energy_fallback<2>());
         xchol = false;
     }
+    KernelFn fn = v->fn;
+    KernelShape shape = v->shape;
+    if (!force && shape.pack == 2) small_shape(c, grad, xchol, i1 - i0, &fn, &shape);
     // record layout: 0 scalar adjoint, 1 scalar Horner energy, 2 / 3 their packed-pair forms
     const int layout = (grad ? 0 : 1) + (v->shape.pack == 2 ? 2 : 0);
     if (io && (io->pv || io->pose_src) && !io->pose_out)
@@ -309,7 +358,7 @@ int launch_pairs(Context& c, const double* pose_dev, int model, bool grad, int i
     // the others (sparse.cu).  Where only the device knows sigma (a pose in device memory, a captured
     // graph) both ways are enqueued and the prologue's flag lets one of them run; that costs an
     // all-pairs evaluation two launches that return at once, so it takes kSparseMinPairsAuto pairs.
-    const double below = !force && xchol && i0 == 0 && i1 == c.N ? sparse_sigma(c) : 0.0;
+    const double below = !force && xchol && i0 == 0 && i1 == c.N ? sparse_sigma(c, SparseUse::energy) : 0.0;
     const double sig = io ? (io->pv ? io->pv->v[kPoseSig] : io->sig) : 0.0;
     const bool known = sig > 0.0;
     const bool both = !known && below > 0.0 && (double)c.N * c.M >= kSparseMinPairsAuto;
@@ -323,8 +372,8 @@ int launch_pairs(Context& c, const double* pose_dev, int model, bool grad, int i
     double* host_out = io ? io->host_out : nullptr;
     const int* flag = both ? c.counter + 4 : nullptr;
     if (!sparse)
-        DUGMA_RET(launch_pair_variant(c, v->fn, v->shape, c.xrec, c.yrec, (size_t)c.M_pad / v->shape.pack, nv, c.Lmax_y,
-                                      pose, i0, i1, out_dev, grad ? dEdx_dev : nullptr, nullptr, 0, nullptr, s, nullptr,
+        DUGMA_RET(launch_pair_variant(c, fn, shape, c.xrec, c.yrec, (size_t)c.M_pad / shape.pack, nv, c.Lmax_y, pose,
+                                      i0, i1, out_dev, grad ? dEdx_dev : nullptr, nullptr, 0, nullptr, s, nullptr,
                                       true, host_out, flag));
     if (sparse || both) {
         int jc_tiles = 0, n_jc = 0;

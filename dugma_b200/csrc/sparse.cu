@@ -96,17 +96,34 @@ int reduce_rows(Context& c, int nv, double* out_dev, cudaStream_t s, double* hos
     return DUGMA_OK;
 }
 
-// Which of a context's evaluations go this way: one whose sigma is below this.  The reach of a pair is
-// sqrt(127.5 sig v / |k|) for the mean variance v; up to 0.63 of the smaller cloud's radius (a tenth of
-// a surface) the search and the marked records cost less than all pairs, beyond the records are as
-// many as make the all-pairs kernel, with four sources a thread, the better one.
-double sparse_sigma(const Context& c)
+// Which of a context's evaluations go this way: those with a sigma below this (0: none).  With f the share
+// of a surface that a pair of mean variance v reaches, f = 127.5 sig v / (4 |k| r^2) for clouds of radius
+// r (r^2: mean squared distance to the mean, of the smaller one), an evaluation is sparse where f is
+// under `most`, a line drawn from timings of both ways at 1000 - 32000 points on six kinds of cloud, f
+// from 5e-4 to 0.2 (one B200, us a call, all pairs / sparse; the outliers' clouds, whose variances differ
+// most, cross first):
+//   energy_grad 3000: 46 / 47-52 at any f;  4500: 91 / 52-82 at 6e-3, 91 / 69-145 at 0.02;  16000:
+//     487 / 94-304 at 6e-3, 487 / 146-611 at 0.02;  32000: 1608 / 162-736, 1608 / 319-1740
+//   compi 4500: 96 / 68-83 at 2e-3, 96 / 77-106 at 6e-3;  6500: 141 / 104-140 at 6e-3;  16000: 622 /
+//     154-432 at 6e-3, 622 / 246-877 at 0.02
+//   CONV 4500: 121 / 83-96 at 5e-4;  6500: 171 / 121-145 at 2e-3;  16000: 762 / 198-427 at 2e-3,
+//     762 / 281-828 at 6e-3
+//   batches, many problems at once: 700 points 246 / 162-213 at 6e-3, 246 / 192-267 at 0.02;  1000: 417 /
+//     264-362 at 0.02, 417 / 340-552 at 0.06;  8000: 837 / 276-561 at 0.02
+double sparse_sigma(const Context& c, SparseUse use)
 {
-    // (the same rule for the coefficients' sparse pass, coef.cu)
-    if (c.x_indef > 0 || c.y_indef > 0 || !c.ux || !c.xpt || c.no_alloc || c.all_pairs) return 0.0;
-    if ((double)c.N * c.M < kSparseMinPairs || c.M > kSparseMaxTargets) return 0.0;
+    if (c.x_indef > 0 || c.y_indef > 0 || !c.ux || !c.xpt || c.no_alloc || c.all_pairs || c.M > kSparseMaxTargets)
+        return 0.0;
+    const double pairs = (double)c.N * c.M, grow = std::pow(std::max(1.0, pairs / 4e7), 1.0 / 6);
+    double most = 0.0;
+    switch (use) {
+    case SparseUse::energy: most = pairs < 12e6 ? 0.0 : (pairs < 2e7 ? 2e-3 : 6e-3 * grow); break;
+    case SparseUse::coef: most = pairs < kSparseCoefMinPairs || c.N > kSparseMaxTargets ? 0.0 : (pairs < 4e7 ? 2e-3 : 6e-3 * grow); break;
+    case SparseUse::conv: most = pairs < 2e7 ? 0.0 : (pairs < 4e7 ? 5e-4 : 2e-3 * grow); break;
+    case SparseUse::batch: most = pairs < 4e5 ? 0.0 : (pairs < 1e6 ? 6e-3 : 2e-2); break;
+    }
     const double v = (c.trace_x + c.trace_y) / (2.0 * c.D), r2 = std::min(c.rho2_x, c.rho2_y);
-    const double s = 0.1 * 4.0 * r2 * -K_EXP2 / ((double)kFlushExp * v);
+    const double s = most * 4.0 * r2 * -K_EXP2 / ((double)kFlushExp * v);
     return s > 0 && std::isfinite(s) ? s : 0.0;
 }
 
