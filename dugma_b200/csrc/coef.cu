@@ -77,7 +77,7 @@ __global__ void coef_prologue_kernel(const PoseBlock pv, int use_pv, double* __r
                                      const float* __restrict__ xinv, const float* __restrict__ lwx, int N, int N_pad,
                                      Rec128* __restrict__ xr, Rec256* __restrict__ xr2, int* __restrict__ reset_counter,
                                      int* __restrict__ reset_err, const double* __restrict__ ux,
-                                     const float* __restrict__ wx, double inv_wmax_x, double sparse_below)
+                                     const float* __restrict__ wx, double Lmax_x, double sparse_below)
 {
     pdl_trigger();   // the one-pass kernel may be scheduled now; it waits for this kernel's writes
     constexpr int NS = Sym<D>::N, NF = Feat<D>::N;
@@ -133,7 +133,7 @@ __global__ void coef_prologue_kernel(const PoseBlock pv, int use_pv, double* __r
             xr[i] = r;
             // for the sparse pass the pairs carry fw = (w / 2^Lmax_x) f(x), as the one pass forms it
             if (wx) {
-                const double ws = i < N ? (double)wx[i] * inv_wmax_x : 0.0;
+                const double ws = i < N ? (double)wx[i] * exp2(-Lmax_x) : 0.0;
                 for (int q = 0; q < NF; ++q) r.g[q] = __double2float_rn(ws * (double)r.g[q]);
             }
             write_pair_half(xr2, i, r);
@@ -366,8 +366,7 @@ struct FusedCoefArgs {
     const Rec256* yrec;    // target pair records
     const float* wx;       // |Sigma_x|^-1/2
     const double* pose;
-    double wmax_x, wmax_y, inv_wmax_x;   // 2^Lmax of either side (a block has no time for FP64 pow and exp2:
-                                         // its set-up was 5 us of the 40 us of an item at 4.5K points)
+    double Lmax_x, Lmax_y;
     int N, M, n_ib, SB, n_grp, n_jc, jc_tiles, total_tiles;
     double* h2_part;       // [n_jc][N][16]
     double* h1_part;       // [n_grp][M][16]
@@ -422,10 +421,10 @@ __global__ void __launch_bounds__(128, 3) coef_fused_kernel(FusedCoefArgs a)
     }
     __syncthreads();
     const double sgm = 1.0 / a.pose[kPoseSig];
-    const double Gs = D == 3 ? sgm * sgm * sgm : sgm * sgm;
-    const double G2 = Gs * a.wmax_y;               // H2_i = w_i G2 sum_j p g_j
-    const double G1 = Gs * a.wmax_x * a.wmax_y;    // H1_j = G1 sum_i fw_i p_ij
-    const double inv_wmax = a.inv_wmax_x;
+    const double Gs = pow(sgm, (double)D);
+    const double G2 = Gs * exp2(a.Lmax_y);               // H2_i = w_i G2 sum_j p g_j
+    const double G1 = Gs * exp2(a.Lmax_x + a.Lmax_y);    // H1_j = G1 sum_i fw_i p_ij
+    const double inv_wmax = exp2(-a.Lmax_x);
     const Rec256* yg = a.yrec;
     const int n_items = a.n_grp * a.n_jc;
     uint32_t tcount = 0;
@@ -908,10 +907,10 @@ __global__ void __launch_bounds__(128, 4 / IPT) coef_tc_kernel(FusedCoefArgs a)
     const uint32_t tbase = *s_tmem;
     const uint32_t tlane = 32u * warp;   // this warp's TMEM lanes (its rows of every M-block)
     const double sgm = 1.0 / a.pose[kPoseSig];
-    const double Gs = D == 3 ? sgm * sgm * sgm : sgm * sgm;
-    const double G2 = Gs * a.wmax_y;
-    const double G1 = Gs * a.wmax_x * a.wmax_y;
-    const double inv_wmax = a.inv_wmax_x;
+    const double Gs = pow(sgm, (double)D);
+    const double G2 = Gs * exp2(a.Lmax_y);
+    const double G1 = Gs * exp2(a.Lmax_x + a.Lmax_y);
+    const double inv_wmax = exp2(-a.Lmax_x);
     const Rec256* yg = a.yrec;
     const int n_items = a.n_grp * a.n_jc;
     uint32_t tcount = 0;   // tiles this block has run (ring and MMA barrier phases)
@@ -1333,9 +1332,7 @@ __global__ void moments_reduce_kernel(const double* __restrict__ a, int na, cons
     const int mi = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     if (mi >= nm) return;
     double v = 0.0;
-#pragma unroll 8
     for (int k = lane; k < na; k += 32) v += a[(size_t)k * nm + mi];
-#pragma unroll 8
     for (int k = lane; k < nb; k += 32) v += b[(size_t)k * nm + mi];
     v = warp_sum(v);
     if (lane == 0) {
@@ -1547,9 +1544,8 @@ static int coef_fused_launch(Context& c, const double* pose_dev, double* moments
     a.yrec = static_cast<const Rec256*>(c.yrec256);
     a.wx = c.wx;
     a.pose = pose_dev;
-    a.wmax_x = std::exp2(c.Lmax_x);
-    a.wmax_y = std::exp2(c.Lmax_y);
-    a.inv_wmax_x = std::exp2(-c.Lmax_x);
+    a.Lmax_x = c.Lmax_x;
+    a.Lmax_y = c.Lmax_y;
     a.N = c.N;
     a.M = c.M;
     a.n_ib = n_ib;
@@ -1649,7 +1645,7 @@ static int coef_impl(Context& c, double* pose_dev, double* moments_dev, cudaStre
                                 static_cast<Rec256*>(c.yrec256), c.x, c.xinv, c.lwx, c.N, c.N_pad, c.xrec128,
                                 static_cast<Rec256*>(c.xrec256), fused ? c.counter : nullptr,
                                 o.reset_err ? c.err : nullptr, (const double*)c.ux, sparse ? (const float*)c.wx : nullptr,
-                                std::exp2(-c.Lmax_x), both ? below : 0.0);
+                                c.Lmax_x, both ? below : 0.0);
     DUGMA_CK(cudaGetLastError());
     if (fused)
         return chol ? coef_fused_launch<D, true>(c, pose_dev, moments_dev, s, o.host_moments, sparse, flag)
