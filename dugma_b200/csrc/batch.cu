@@ -216,8 +216,8 @@ __global__ void __launch_bounds__(NT) batch_pairs_kernel(const PQDesc* __restric
 }
 
 // The sparse pairs of a slab: tile blockIdx.x of the sources of pair pq0 + blockIdx.y (sparse.cu).
-template <int D>
-__global__ void __launch_bounds__(128, 6) batch_sparse_kernel(const PQDesc* __restrict__ desc, int pq0, int tile_shift,
+template <int D, int NW>
+__global__ void __launch_bounds__(32 * NW, 24 / NW) batch_sparse_kernel(const PQDesc* __restrict__ desc, int pq0, int tile_shift,
                                                               int chunk_rec, double* __restrict__ rows)
 {
     extern __shared__ __align__(16) unsigned char smem[];
@@ -235,9 +235,9 @@ __global__ void __launch_bounds__(128, 6) batch_sparse_kernel(const PQDesc* __re
     a.tile_shift = tile_shift;
     a.chunk_rec = chunk_rec;
     a.rows = rows + (size_t)pd.row0 * 8;
-    uint32_t* bits = reinterpret_cast<uint32_t*>(smem + kSparseFixed);
-    for (int w = threadIdx.x; w < a.words; w += 128) bits[w] = 0;
-    sparse_tile<D, true>(a, blockIdx.x, smem);
+    uint32_t* bits = reinterpret_cast<uint32_t*>(smem + SparseShape<NW>::kFixed);
+    for (int w = threadIdx.x; w < a.words; w += 32 * NW) bits[w] = 0;
+    sparse_tile<D, true, NW>(a, blockIdx.x, smem);
 }
 
 // out[pq][v] = sum of the pair's item partials, in the fixed order of its item index list, or of its
@@ -513,11 +513,15 @@ static int batch_enqueue(Batch& b, cudaStream_t s)
     }
     int shift = 0;
     while (1 << shift < var.sh.tj) ++shift;
-    const size_t smem = kSparseFixed + sizeof(uint32_t) * b.max_words;
-    DUGMA_CK(cudaFuncSetAttribute(batch_sparse_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    // two warps a tile where the batch's tiles fill the GPU that way (24 x 8: 367 us with two, 392 with four,
+    // 670 with eight: the work that each warp repeats counts), eight where they do not
+    const bool two = (size_t)b.max_tiles * n_pq > (size_t)6 * sms;
+    auto sparse = two ? batch_sparse_kernel<D, 2> : batch_sparse_kernel<D, 8>;
+    const size_t smem = (two ? SparseShape<2>::kFixed : SparseShape<8>::kFixed) + sizeof(uint32_t) * b.max_words;
+    DUGMA_CK(cudaFuncSetAttribute(sparse, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     for (size_t k = 0; k + 1 < b.slab.size(); ++k) {
         const int q0 = b.slab[k], nq = b.slab[k + 1] - q0;
-        batch_sparse_kernel<D><<<dim3(b.max_tiles, nq), 128, smem, s>>>(b.desc, q0, shift, var.sh.chunk, b.rows);
+        sparse<<<dim3(b.max_tiles, nq), two ? 64 : 256, smem, s>>>(b.desc, q0, shift, var.sh.chunk, b.rows);
         DUGMA_CK(cudaGetLastError());
         batch_reduce_kernel<<<nq, 256, 0, s>>>(b.desc, q0, b.partials, b.pq_start, b.pq_items, b.rows, b.nv, b.out);
         DUGMA_CK(cudaGetLastError());

@@ -635,17 +635,18 @@ struct CoefSparseArgs {
     const int* go;                 // nullable: nothing is done unless set
 };
 
+template <int NW>
 struct CoefSparseShape {
     static constexpr int BATCH = 4, UNITS = 16;   // records loaded together; units listed together per warp
-    static constexpr size_t kRec = 4 * 2 * BATCH * sizeof(Rec256), kList = 4 * UNITS * 64 * sizeof(uint16_t),
-                            kSums = 4 * 10 * 32 * sizeof(double);
+    static constexpr size_t kRec = NW * 2 * BATCH * sizeof(Rec256), kList = NW * UNITS * 64 * sizeof(uint16_t),
+                            kSums = NW * 10 * 32 * sizeof(double);
     static constexpr size_t kFixed = (sizeof(ReachShared) + 15) / 16 * 16 + kRec + kList + kSums;
 };
 
-template <int D, int SIDE>
+template <int D, int SIDE, int NW>
 __device__ __forceinline__ void coef_sparse_side(const CoefSparseArgs& a, int group, unsigned char* smem)
 {
-    using S = CoefSparseShape;
+    using S = CoefSparseShape<NW>;
     constexpr int NF = Feat<D>::N, NS = Sym<D>::N;
     ReachShared& sh = *reinterpret_cast<ReachShared*>(smem);
     unsigned char* work = smem + (sizeof(ReachShared) + 15) / 16 * 16;
@@ -664,7 +665,7 @@ __device__ __forceinline__ void coef_sparse_side(const CoefSparseArgs& a, int gr
     reach.sm = SIDE == 0 ? a.y : a.x;
     reach.pose = a.pose;
     reach.inv_trace = a.inv_trace;
-    const bool marked = find_reach<D, SIDE == 0>(reach, group, bits, sh);
+    const bool marked = find_reach<D, NW, SIDE == 0>(reach, group, bits, sh);
     if (!__syncthreads_or(marked)) {   // nothing reaches these points
         if (warp == 0 && in)
 #pragma unroll
@@ -711,8 +712,8 @@ __device__ __forceinline__ void coef_sparse_side(const CoefSparseArgs& a, int gr
     };
     const float2* recs = reinterpret_cast<const float2*>(SIDE == 0 ? a.ypair : a.xpair);
     const int n_units = a.n_units[SIDE];
-    // 64 units at a time, 16 of them this warp's (side 1: four blocks of four units)
-    for (int ubase = 0; ubase < n_units; ubase += 4 * S::UNITS) {
+    // 16 units a warp at a time (side 1: four blocks of four units)
+    for (int ubase = 0; ubase < n_units; ubase += NW * S::UNITS) {
         // lane's unit: its records [r0, r1) and their marks
         auto first_rec = [&](int u) {
             if (SIDE == 1) return 32 * u;
@@ -720,7 +721,7 @@ __device__ __forceinline__ void coef_sparse_side(const CoefSparseArgs& a, int gr
             return 16 * (c * a.jc_tiles + 4 * m);
         };
         auto unit_of = [&](int l) {
-            return ubase + (SIDE == 0 ? 4 * l + warp : 16 * (l >> 2) + 4 * warp + (l & 3));
+            return ubase + (SIDE == 0 ? NW * l + warp : 4 * NW * (l >> 2) + 4 * warp + (l & 3));
         };
         const int base = first_rec(ubase);
         const int u = unit_of(lane);
@@ -801,26 +802,27 @@ __device__ __forceinline__ void coef_sparse_side(const CoefSparseArgs& a, int gr
     for (int q = 0; q < NF; ++q) {
         double t = sums[0][q][lane];
 #pragma unroll
-        for (int k = 1; k < 4; ++k) t += sums[k][q][lane];
+        for (int k = 1; k < NW; ++k) t += sums[k][q][lane];
         o[q] = w * t;
     }
 }
 
-template <int D>
-__global__ void __launch_bounds__(128, 5) coef_sparse_kernel(CoefSparseArgs a)
+constexpr int kCoefWarps = 4;   // 16384 x 15000: 35 us with two, 31 with four and with eight
+template <int D, int NW>
+__global__ void __launch_bounds__(32 * NW, 20 / NW) coef_sparse_kernel(CoefSparseArgs a)
 {
-    using S = CoefSparseShape;
+    using S = CoefSparseShape<NW>;
     extern __shared__ __align__(128) unsigned char smem[];
     const int side = (int)blockIdx.x < a.n_st0 ? 0 : 1;
     uint32_t* bits = reinterpret_cast<uint32_t*>(smem + S::kFixed);
     pdl_trigger();   // a dependent of the coefficient prologue, and the moments kernel one of this
-    for (int w = threadIdx.x; w < a.words[side]; w += 128) bits[w] = 0;
+    for (int w = threadIdx.x; w < a.words[side]; w += 32 * NW) bits[w] = 0;
     pdl_wait();
     if (a.go && !*a.go) return;
     if (side == 0)
-        coef_sparse_side<D, 0>(a, blockIdx.x, smem);
+        coef_sparse_side<D, 0, NW>(a, blockIdx.x, smem);
     else
-        coef_sparse_side<D, 1>(a, blockIdx.x - a.n_st0, smem);
+        coef_sparse_side<D, 1, NW>(a, blockIdx.x - a.n_st0, smem);
 }
 
 // ---------------------------------------------------------------------------
@@ -1501,8 +1503,8 @@ static int coef_sparse_setup(int dev)
     static bool done[64];
     std::lock_guard<std::mutex> lk(mu);
     if (dev >= 64 || !done[dev]) {
-        DUGMA_CK(cudaFuncSetAttribute(coef_sparse_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      (int)(CoefSparseShape::kFixed + kSparseMaxTargets / 64 * sizeof(uint32_t))));
+        DUGMA_CK(cudaFuncSetAttribute(coef_sparse_kernel<D, kCoefWarps>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      (int)(CoefSparseShape<kCoefWarps>::kFixed + kSparseMaxTargets / 64 * sizeof(uint32_t))));
         if (dev < 64) done[dev] = true;
     }
     return DUGMA_OK;
@@ -1599,8 +1601,10 @@ static int coef_fused_launch(Context& c, const double* pose_dev, double* moments
         sa.h2 = rows2;
         sa.h1 = rows1;
         sa.go = flag;
-        const size_t bytes = CoefSparseShape::kFixed + sizeof(uint32_t) * std::max(sa.words[0], sa.words[1]);
-        DUGMA_CK(launch_dependent(c.pdl, coef_sparse_kernel<D>, sa.n_st0 + (c.M + kTile - 1) / kTile, 128, bytes, s, sa));
+        using S = CoefSparseShape<kCoefWarps>;
+        const int tiles = sa.n_st0 + (c.M + kTile - 1) / kTile;
+        const size_t bits = sizeof(uint32_t) * std::max(sa.words[0], sa.words[1]);
+        DUGMA_CK(launch_dependent(c.pdl, coef_sparse_kernel<D, kCoefWarps>, tiles, 32 * kCoefWarps, S::kFixed + bits, s, sa));
     }
     DUGMA_RET(timing_end(c, s));
     const int nblk = std::max(1, std::min(2 * c.num_sms, (std::max(c.N, c.M) + 31) / 32));

@@ -876,7 +876,7 @@ __global__ void __launch_bounds__(128, 3) conv_sparse_kernel(ConvSparseArgs a)
     const int pos = blockIdx.x * kTile + lane;
     const bool in = pos < a.reach.st.n;
     const int i = a.reach.st.pt[in ? pos : 0].idx;
-    const bool marked = find_reach<D, true, true>(a.reach, blockIdx.x, bits, sh);
+    const bool marked = find_reach<D, 4, true, true>(a.reach, blockIdx.x, bits, sh);
     double acc[NV], dx[3] = {0, 0, 0};
 #pragma unroll
     for (int v = 0; v < NV; ++v) acc[v] = 0.0;

@@ -33,7 +33,6 @@ struct ReachArgs {
                            // is left out (conv.cu)
 };
 
-// one block of 4 warps
 struct ReachShared {
     float4 pt[kTile];      // position, L
     float2 pa[kTile];      // a, slack
@@ -106,12 +105,13 @@ __device__ __forceinline__ float dist2_f32(const float4& p, const float4& q)
 }
 
 // The records that reach tile `group` of the stationary side, into bits (shared, one per record; all
-// 128 threads; the caller zeroes bits before and synchronises after).  True for a lane that marked any.  POSE_SM: the streamed side is
+// 32 NW threads; the caller zeroes bits before and synchronises after).  True for a lane that marked any.  POSE_SM: the streamed side is
 // the targets' (moved by the pose), else the stationary side is.
-template <int D, bool POSE_SM, bool CONV = false>
+template <int D, int NW, bool POSE_SM, bool CONV = false>
 __device__ __forceinline__ bool find_reach(const ReachArgs& a, int group, uint32_t* bits, ReachShared& sh)
 {
-    constexpr int NW = 4, TPW = kSuper / NW;
+    constexpr int TPW = kSuper / NW;
+    static_assert(NW == 2 || NW == 4 || NW == 8, "36 threads and more set the tile up");
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const PoseF P = pose_f32<D>(a.pose);
     const float sigk = (float)(a.pose[kPoseSig] * (1.0 / -K_EXP2)) * (1.f + 1e-6f);

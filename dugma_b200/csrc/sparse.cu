@@ -3,12 +3,12 @@
 // Where the covariances follow the point spacing, all but a few of a source's pairs have both
 // exponentials below the FP32 flush (reach.cuh), and the all-pairs kernels spend their time adding
 // zeros.  Here a block takes one tile of 32 sources in spatial order (one per lane, the same in its
-// four warps), marks the target records that can reach one of them, and evaluates those alone.
+// warps), marks the target records that can reach one of them, and evaluates those alone.
 //
 // The sums are those of the all-pairs kernels, term for term: a source's records are taken in index
 // order, its energy summed in FP32 over each of their tiles and its moments over each of their chunks,
 // by the same body on the same records; the terms left out are exact zeros.  Chunks are split over
-// the warps (chunk c to warp c mod 4), the chunks' sums added in FP64 per source, and the sources'
+// the warps (chunk c to warp c mod their number), the chunks' sums added in FP64 per source, and the sources'
 // contributions to E and the gradient go to rows by source index that a second kernel adds in fixed
 // order, so neither the spatial order nor the schedule shows in a result.
 //
@@ -25,16 +25,20 @@
 
 namespace dugma {
 
-template <int D, bool GRAD>
-__global__ void __launch_bounds__(128, 6) sparse_kernel(SparseArgs a, const int* go)
+// Eight warps a tile: one problem's few heavy tiles (outliers, edges of a depth map) end the launch.  2 / 4 / 8
+// warps, adjoint kernel on one B200: 65536 x 65536 73 / 54 / 48 us; 240000 depth 627 / 490 / 411; 6000 with
+// outliers - / 23 / 17.5; 2D 20011 - / 18.5 / 16.
+constexpr int kSparseWarps = 8;
+template <int D, bool GRAD, int NW>
+__global__ void __launch_bounds__(32 * NW, 24 / NW) sparse_kernel(SparseArgs a, const int* go)
 {
     extern __shared__ __align__(16) unsigned char smem[];
-    uint32_t* bits = reinterpret_cast<uint32_t*>(smem + kSparseFixed);
+    uint32_t* bits = reinterpret_cast<uint32_t*>(smem + SparseShape<NW>::kFixed);
     pdl_trigger();   // a dependent of the prologue; the rows' sum is one of this kernel
-    for (int w = threadIdx.x; w < a.words; w += 128) bits[w] = 0;
+    for (int w = threadIdx.x; w < a.words; w += 32 * NW) bits[w] = 0;
     pdl_wait();
     if (go && !*go) return;   // (nullable: nothing is done unless set)
-    sparse_tile<D, GRAD>(a, blockIdx.x, smem);
+    sparse_tile<D, GRAD, NW>(a, blockIdx.x, smem);
 }
 
 // out[v] = sum of rows[i][v]: per-block partials over contiguous slices, then the block that finishes
@@ -131,13 +135,15 @@ template <int D, bool GRAD>
 static int sparse_impl(Context& c, const double* pose_dev, int tile_rec, int chunk_rec, double* out_dev,
                        double* dEdx_dev, cudaStream_t s, double* host_out, const int* go)
 {
+    constexpr int NW = kSparseWarps;
     static std::mutex mu;
     static bool done[64];
-    const size_t most = kSparseFixed + kSparseMaxTargets / 64 * sizeof(uint32_t);
+    const size_t most = SparseShape<NW>::kFixed + kSparseMaxTargets / 64 * sizeof(uint32_t);
     {
         std::lock_guard<std::mutex> lk(mu);
         if (c.dev < 64 && !done[c.dev]) {
-            DUGMA_CK(cudaFuncSetAttribute(sparse_kernel<D, GRAD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most));
+            DUGMA_CK(cudaFuncSetAttribute(sparse_kernel<D, GRAD, NW>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                          (int)most));
             done[c.dev] = true;
         }
     }
@@ -158,7 +164,8 @@ static int sparse_impl(Context& c, const double* pose_dev, int tile_rec, int chu
     a.dx = dEdx_dev;
     const int grid = (c.N + kTile - 1) / kTile;
     DUGMA_RET(timing_begin(c, s));
-    DUGMA_CK(launch_dependent(c.pdl, sparse_kernel<D, GRAD>, grid, 128, kSparseFixed + sizeof(uint32_t) * a.words, s, a, go));
+    DUGMA_CK(launch_dependent(c.pdl, sparse_kernel<D, GRAD, NW>, grid, 32 * NW,
+                              SparseShape<NW>::kFixed + sizeof(uint32_t) * a.words, s, a, go));
     DUGMA_RET(timing_end(c, s));
     return reduce_rows(c, GRAD ? 1 + (D == 3 ? 6 : 3) : 1, out_dev, s, host_out, go);
 }
@@ -168,11 +175,9 @@ int sparse_launch(Context& c, const double* pose_dev, bool grad, int tile_rec, i
 {
     if (chunk_rec > kSparseChunk || chunk_rec % 32 || tile_rec < 32 || (tile_rec & (tile_rec - 1)))
         return set_error(DUGMA_ERR_STATE, "sparse evaluation: chunks of %d records, tiles of %d", chunk_rec, tile_rec);
-    if (c.D == 3)
-        return grad ? sparse_impl<3, true>(c, pose_dev, tile_rec, chunk_rec, out_dev, dEdx_dev, s, host_out, go)
-                    : sparse_impl<3, false>(c, pose_dev, tile_rec, chunk_rec, out_dev, dEdx_dev, s, host_out, go);
-    return grad ? sparse_impl<2, true>(c, pose_dev, tile_rec, chunk_rec, out_dev, dEdx_dev, s, host_out, go)
-                : sparse_impl<2, false>(c, pose_dev, tile_rec, chunk_rec, out_dev, dEdx_dev, s, host_out, go);
+    auto fn = c.D == 3 ? (grad ? sparse_impl<3, true> : sparse_impl<3, false>)
+                       : (grad ? sparse_impl<2, true> : sparse_impl<2, false>);
+    return fn(c, pose_dev, tile_rec, chunk_rec, out_dev, dEdx_dev, s, host_out, go);
 }
 
 }  // namespace dugma

@@ -24,31 +24,33 @@ struct SparseArgs {
 constexpr int kSparseChunk = 1024;  // most records a chunk may have (32 words of the bitmap)
 constexpr int kSparseBatch = 8;     // records loaded together
 // shared memory: reach tests, then per warp two batches of records, the chunk's list and the FP64 sums
-// (there, and not in registers, so that six blocks fit an SM: 67 us at 64K against 78 with four)
-constexpr size_t kSparseRec = 4 * 2 * kSparseBatch * sizeof(YRec2);
-constexpr size_t kSparseList = 4 * kSparseChunk * sizeof(uint16_t);
-constexpr size_t kSparseSums = 4 * 13 * 32 * sizeof(double);
-constexpr size_t kSparseWork = kSparseRec + kSparseList + kSparseSums;
-constexpr size_t kSparseFixed = (sizeof(ReachShared) + 15) / 16 * 16 + kSparseWork;
+// (there, and not in registers, so that 24 warps fit an SM: 67 us at 64K against 78 with 16 of them)
+template <int NW>
+struct SparseShape {
+    static constexpr size_t kRec = NW * 2 * kSparseBatch * sizeof(YRec2), kList = NW * kSparseChunk * sizeof(uint16_t),
+                            kSums = NW * 13 * 32 * sizeof(double);
+    static constexpr size_t kFixed = (sizeof(ReachShared) + 15) / 16 * 16 + kRec + kList + kSums;
+};
 
-// The tile `group` of 32 sources, by the block's 128 threads; the caller has zeroed the bitmap behind
-// kSparseFixed bytes of smem.
-template <int D, bool GRAD>
+// The tile `group` of 32 sources, by the block's NW warps; the caller has zeroed the bitmap behind
+// SparseShape::kFixed bytes of smem.
+template <int D, bool GRAD, int NW>
 __device__ __forceinline__ void sparse_tile(const SparseArgs& a, int group, unsigned char* smem)
 {
+    using S = SparseShape<NW>;
     using Body = PackedBody<D, 1, GRAD, true>;
     constexpr int NS = Sym<D>::N, NV = Body::NV;
     ReachShared& sh = *reinterpret_cast<ReachShared*>(smem);
     unsigned char* work = smem + (sizeof(ReachShared) + 15) / 16 * 16;
-    uint32_t* bits = reinterpret_cast<uint32_t*>(work + kSparseWork);
+    uint32_t* bits = reinterpret_cast<uint32_t*>(smem + S::kFixed);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     float(*rec)[kSparseBatch * 32] = reinterpret_cast<float(*)[kSparseBatch * 32]>(work) + 2 * warp;
-    uint16_t* list = reinterpret_cast<uint16_t*>(work + kSparseRec) + kSparseChunk * warp;
+    uint16_t* list = reinterpret_cast<uint16_t*>(work + S::kRec) + kSparseChunk * warp;
 
     const int pos = group * kTile + lane;
     const bool in = pos < a.reach.st.n;
     const int i = a.reach.st.pt[in ? pos : 0].idx;
-    const bool marked = find_reach<D, true>(a.reach, group, bits, sh);
+    const bool marked = find_reach<D, NW, true>(a.reach, group, bits, sh);
     if (!__syncthreads_or(marked)) {   // nothing reaches these sources
         if (warp == 0 && in) {
 #pragma unroll
@@ -70,11 +72,11 @@ __device__ __forceinline__ void sparse_tile(const SparseArgs& a, int group, unsi
     }
     body.zero_all();
     // E, sum e1 u, sum e2 z, sum e2 z z^T per source
-    double(*sums)[13][32] = reinterpret_cast<double(*)[13][32]>(work + kSparseRec + kSparseList);
+    double(*sums)[13][32] = reinterpret_cast<double(*)[13][32]>(work + S::kRec + S::kList);
 #pragma unroll
     for (int q = 0; q < 13; ++q) sums[warp][q][lane] = 0.0;
     const float* recs = reinterpret_cast<const float*>(a.yrec);
-    for (int base = warp * a.chunk_rec; base < a.n_rec; base += 4 * a.chunk_rec) {
+    for (int base = warp * a.chunk_rec; base < a.n_rec; base += NW * a.chunk_rec) {
         // the chunk's marked records, ascending
         const int nw = (min(a.chunk_rec, a.n_rec - base) + 31) / 32;
         uint32_t w = lane < nw ? bits[base / 32 + lane] : 0u;
@@ -140,7 +142,7 @@ __device__ __forceinline__ void sparse_tile(const SparseArgs& a, int group, unsi
     auto total = [&](int q) {
         double s = sums[0][q][lane];
 #pragma unroll
-        for (int u = 1; u < 4; ++u) s += sums[u][q][lane];
+        for (int u = 1; u < NW; ++u) s += sums[u][q][lane];
         return s;
     };
     const double sg = 1.0 / a.pose[kPoseSig];
