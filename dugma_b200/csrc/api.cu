@@ -890,6 +890,7 @@ int dugma_timing(float* Ptr[6], int mode, double* total_ms, int* launches)
     GET_CTX(c, Ptr);
     if (mode == 1) {
         c->timing = true;
+        c->timing_open = c->timing_hold = false;
         c->tused = 0;
         return DUGMA_OK;
     }

@@ -134,6 +134,8 @@ struct Context {
     std::mutex mu;                            // one host call at a time per context
     // optional timing of the main pairwise kernel (dugma_timing)
     bool timing = false;
+    bool timing_open = false;                 // an interval has begun
+    bool timing_hold = false;                 // the next kernel belongs to the same interval
     std::vector<std::pair<cudaEvent_t, cudaEvent_t>> tevents;
     size_t tused = 0;
 
@@ -184,7 +186,8 @@ int launch_pair_variant(Context& c, KernelFn fn, const KernelShape& sh, const vo
 // How that launch splits `rows` x `total` streamed records (tiles of sh.tj): tiles per chunk, chunks.
 void pair_split(const Context& c, KernelFn fn, const KernelShape& sh, int rows, size_t yrec_size, int* jc_tiles,
                 int* n_jc);
-// CUDA events around the main pairwise kernel when timing is on (dugma_timing)
+// CUDA events around the main pairwise kernel when timing is on (dugma_timing); while c.timing_hold is set
+// the interval stays open
 int timing_begin(Context& c, cudaStream_t s);
 int timing_end(Context& c, cudaStream_t s);
 // The REF energy or adjoint over the pairs above the FP32 flush (sparse.cu), from the records of the

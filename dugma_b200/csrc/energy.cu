@@ -239,7 +239,8 @@ static void small_shape(const Context& c, bool grad, bool chol, int rows, Kernel
 
 int timing_begin(Context& c, cudaStream_t s)
 {
-    if (!c.timing) return DUGMA_OK;
+    if (!c.timing || c.timing_open) return DUGMA_OK;
+    c.timing_open = true;
     if (c.tused == c.tevents.size()) {
         cudaEvent_t e0, e1;
         DUGMA_CK(cudaEventCreate(&e0));
@@ -252,7 +253,8 @@ int timing_begin(Context& c, cudaStream_t s)
 
 int timing_end(Context& c, cudaStream_t s)
 {
-    if (!c.timing) return DUGMA_OK;
+    if (!c.timing || !c.timing_open || c.timing_hold) return DUGMA_OK;
+    c.timing_open = false;
     DUGMA_CK(cudaEventRecord(c.tevents[c.tused].second, s));
     ++c.tused;
     return DUGMA_OK;
@@ -371,10 +373,12 @@ int launch_pairs(Context& c, const double* pose_dev, int model, bool grad, int i
     const double* pose = io && io->pose_out ? io->pose_out : pose_dev;
     double* host_out = io ? io->host_out : nullptr;
     const int* flag = both ? c.counter + 4 : nullptr;
+    c.timing_hold = both;   // (one timed interval for the two pair kernels)
     if (!sparse)
         DUGMA_RET(launch_pair_variant(c, fn, shape, c.xrec, c.yrec, (size_t)c.M_pad / shape.pack, nv, c.Lmax_y, pose,
                                       i0, i1, out_dev, grad ? dEdx_dev : nullptr, nullptr, 0, nullptr, s, nullptr,
                                       true, host_out, flag));
+    c.timing_hold = false;
     if (sparse || both) {
         int jc_tiles = 0, n_jc = 0;
         pair_split(c, v->fn, v->shape, c.N, (size_t)c.M_pad / 2, &jc_tiles, &n_jc);

@@ -646,7 +646,9 @@ static int nn_run(Context& c, double* pose_dev, int k, int* idx_dev, float* d2_d
         const bool wide = nx <= 2 * c.num_sms;
         auto fn = wide ? (c.D == 3 ? prune_kernel<3, 8>(K) : prune_kernel<2, 8>(K))
                        : (c.D == 3 ? prune_kernel<3, 4>(K) : prune_kernel<2, 4>(K));
+        DUGMA_RET(timing_begin(c, s));
         DUGMA_CK(launch_dependent(c.pdl, fn, nx, wide ? 256 : 128, 0, s, a));
+        DUGMA_RET(timing_end(c, s));
         return DUGMA_OK;
     }
     const KernelShape want = force ? *force : c.shape_nn;
