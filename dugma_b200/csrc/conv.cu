@@ -36,9 +36,13 @@ template <int D>
 __global__ void conv_prologue_kernel(const double* __restrict__ pose, const float* __restrict__ y,
                                      const float* __restrict__ ycov, int M, int M_pad, YRec* __restrict__ yrec,
                                      const float* __restrict__ x, const float* __restrict__ xcov, int N, int N_pad,
-                                     XRec* __restrict__ xrec)
+                                     XRec* __restrict__ xrec, int* __restrict__ counter, double sparse_below)
 {
     constexpr int NS = Sym<D>::N;
+    if (blockIdx.x == 0 && threadIdx.x == 0) {   // work counters, and whether the sparse pass runs
+        counter[0] = counter[1] = 0;
+        counter[4] = pose[kPoseSig] < sparse_below;
+    }
     double R[9], t[3];
     for (int k = 0; k < D * D; ++k) R[k] = pose[k];
     for (int a = 0; a < D; ++a) t[a] = pose[kPoseT + a];
@@ -857,7 +861,7 @@ struct ConvSparseShape {
 };
 
 template <int D, bool GRAD>
-__global__ void __launch_bounds__(128, 3) conv_sparse_kernel(ConvSparseArgs a)
+__global__ void __launch_bounds__(128, 3) conv_sparse_kernel(ConvSparseArgs a, const int* go)
 {
     using S = ConvSparseShape;
     using Body = PackedConvBody<D, 1, GRAD, 128>;
@@ -873,6 +877,7 @@ __global__ void __launch_bounds__(128, 3) conv_sparse_kernel(ConvSparseArgs a)
     pdl_trigger();
     for (int w = threadIdx.x; w < a.words; w += 128) bits[w] = 0;
     pdl_wait();
+    if (go && !*go) return;   // (nullable: nothing is done unless set)
     const int pos = blockIdx.x * kTile + lane;
     const bool in = pos < a.reach.st.n;
     const int i = a.reach.st.pt[in ? pos : 0].idx;
@@ -1018,7 +1023,7 @@ std::vector<KernelShape> conv_shapes(bool grad)
 
 template <int D, bool GRAD>
 static int conv_sparse_launch(Context& c, KernelFn fn, const KernelShape& sh, const double* pose_dev, double* out_dev,
-                              double* dEdx_dev, cudaStream_t s, double cut)
+                              double* dEdx_dev, cudaStream_t s, double cut, const int* go)
 {
     using S = ConvSparseShape;
     static std::mutex mu;
@@ -1053,12 +1058,11 @@ static int conv_sparse_launch(Context& c, KernelFn fn, const KernelShape& sh, co
     if (a.chunk_rec > S::CHUNK) return set_error(DUGMA_ERR_STATE, "sparse CONV: chunks of %d records", a.chunk_rec);
     a.rows = c.scratch;
     a.dx = dEdx_dev;
-    DUGMA_CK(cudaMemsetAsync(c.counter, 0, 2 * sizeof(int), s));
     DUGMA_RET(timing_begin(c, s));
-    conv_sparse_kernel<D, GRAD><<<(c.N + kTile - 1) / kTile, 128, S::kFixed + sizeof(uint32_t) * a.words, s>>>(a);
+    conv_sparse_kernel<D, GRAD><<<(c.N + kTile - 1) / kTile, 128, S::kFixed + sizeof(uint32_t) * a.words, s>>>(a, go);
     DUGMA_CK(cudaGetLastError());
     DUGMA_RET(timing_end(c, s));
-    return reduce_rows(c, GRAD ? 1 + (D == 3 ? 6 : 3) : 1, out_dev, s, nullptr, nullptr);
+    return reduce_rows(c, GRAD ? 1 + (D == 3 ? 6 : 3) : 1, out_dev, s, nullptr, go);
 }
 
 int conv_launch(Context& c, const double* pose_dev, bool grad, int i0, int i1, double* out_dev, double* dEdx_dev,
@@ -1070,16 +1074,22 @@ int conv_launch(Context& c, const double* pose_dev, bool grad, int i0, int i1, d
     for (auto& cand : vars)
         if (cand.shape.same(want)) v = &cand;
     const bool packed = v->shape.pack == 2;
+    // all rows by the packed kernels: the sparse pass below sparse_sigma's line; where only the device knows
+    // sigma both are enqueued and the prologue's flag lets one run (as the REF model's, energy.cu)
+    const double below = packed && !force && i0 == 0 && i1 == c.N && c.nonpd == 0 ? sparse_sigma(c, SparseUse::conv) : 0.0;
+    const bool both = !(sig > 0.0) && below > 0.0 && (double)c.N * c.M >= kSparseMinPairsAuto;
+    const bool sparse = sig > 0.0 && sig < below;
+    const int* flag = both ? c.counter + 4 : nullptr;
     // source records always; target records scalar (YRec) or paired (YRec2, same bytes)
     const int n = std::max(c.M_pad, c.N_pad);
     const int g = std::min((n + 255) / 256, c.num_sms * 4);
     const int my = packed ? 0 : c.M, myp = packed ? 0 : c.M_pad;
     if (c.D == 3)
         conv_prologue_kernel<3><<<g, 256, 0, s>>>(pose_dev, c.y, c.ycov, my, myp, c.yrec, c.x, c.xcov, c.N, c.N_pad,
-                                                  c.xrec);
+                                                  c.xrec, c.counter, both ? below : 0.0);
     else
         conv_prologue_kernel<2><<<g, 256, 0, s>>>(pose_dev, c.y, c.ycov, my, myp, c.yrec, c.x, c.xcov, c.N, c.N_pad,
-                                                  c.xrec);
+                                                  c.xrec, c.counter, both ? below : 0.0);
     DUGMA_CK(cudaGetLastError());
     if (packed) {
         YRec2* y2 = reinterpret_cast<YRec2*>(c.yrec);
@@ -1091,16 +1101,17 @@ int conv_launch(Context& c, const double* pose_dev, bool grad, int i0, int i1, d
         DUGMA_CK(cudaGetLastError());
     }
     const int nv = grad ? 1 + (c.D == 3 ? 6 : 3) : 1;
-    if (packed && !force && i0 == 0 && i1 == c.N && sig > 0.0) {
-        const double cut = 2.0 + std::max(285.0, 150.0 + 0.5 * c.D * std::log2(std::max(1.0, 0.5 * c.cscale * c.inv_trace)));
-        if (c.nonpd == 0 && sig < sparse_sigma(c, SparseUse::conv))
-            return c.D == 3 ? (grad ? conv_sparse_launch<3, true>(c, v->fn, v->shape, pose_dev, out_dev, dEdx_dev, s, cut)
-                                    : conv_sparse_launch<3, false>(c, v->fn, v->shape, pose_dev, out_dev, nullptr, s, cut))
-                            : (grad ? conv_sparse_launch<2, true>(c, v->fn, v->shape, pose_dev, out_dev, dEdx_dev, s, cut)
-                                    : conv_sparse_launch<2, false>(c, v->fn, v->shape, pose_dev, out_dev, nullptr, s, cut));
-    }
-    return launch_pair_variant(c, v->fn, v->shape, c.xrec, c.yrec, (size_t)c.M_pad / v->shape.pack, nv, c.cscale,
-                               pose_dev, i0, i1, out_dev, grad ? dEdx_dev : nullptr, nullptr, 0, nullptr, s);
+    c.timing_hold = both;
+    if (!sparse)
+        DUGMA_RET(launch_pair_variant(c, v->fn, v->shape, c.xrec, c.yrec, (size_t)c.M_pad / v->shape.pack, nv, c.cscale,
+                                      pose_dev, i0, i1, out_dev, grad ? dEdx_dev : nullptr, nullptr, 0, nullptr, s,
+                                      nullptr, true, nullptr, flag));
+    c.timing_hold = false;
+    if (!sparse && !both) return DUGMA_OK;
+    const double cut = 2.0 + std::max(285.0, 150.0 + 0.5 * c.D * std::log2(std::max(1.0, 0.5 * c.cscale * c.inv_trace)));
+    auto run = c.D == 3 ? (grad ? conv_sparse_launch<3, true> : conv_sparse_launch<3, false>)
+                        : (grad ? conv_sparse_launch<2, true> : conv_sparse_launch<2, false>);
+    return run(c, v->fn, v->shape, pose_dev, out_dev, grad ? dEdx_dev : nullptr, s, cut, flag);
 }
 
 }  // namespace dugma

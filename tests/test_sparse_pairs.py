@@ -153,3 +153,29 @@ def test_batch_same_sums_as_all_pairs(monkeypatch):
     for u, v in zip(*out):
         assert np.all(np.linalg.norm((u - v).reshape(len(probs), 3, -1), axis=2)
                       <= 1e-12 * np.linalg.norm(v.reshape(len(probs), 3, -1), axis=2))
+
+
+@pytest.mark.parametrize("model", [0, 1])
+def test_device_pose_is_host_pose(model):
+    """Where only the device knows sigma (a pose in device memory) a flag picks the pass that a host pose
+    picks on the host: the same bits, below the rule's line (3e-4) and above it (1)."""
+    import torch
+    from dugma_b200 import _lib
+    X, XC, Y, YC, R, t = _problem("sphere", 16385, 16001, 2)
+    _, h = api.init(X, XC, Y, YC)
+    s = torch.cuda.Stream()
+    pose, out = torch.zeros(16, dtype=torch.float64, device="cuda"), torch.zeros(8, dtype=torch.float64, device="cuda")
+    dx = torch.zeros(len(X), 3, dtype=torch.float64, device="cuda")
+    for sig in (3e-4, 1.0, 3e-4):
+        pose[:9] = torch.tensor(np.asarray(R).T.reshape(-1))
+        pose[9:12] = torch.tensor(t + 0.01)
+        pose[12] = sig
+        torch.cuda.synchronize()
+        assert _lib.load().dugma_energy_grad_async(h.arr, pose.data_ptr(), model, out.data_ptr(), dx.data_ptr(),
+                                                   s.cuda_stream) == 0
+        torch.cuda.synchronize()
+        E, g, d = api.energy_grad(h, R, t + 0.01, sig, model=model, with_dx=True)
+        got = out.cpu().numpy()
+        assert got[0] == E and np.array_equal(got[1:7], np.asarray(g).reshape(-1))
+        assert np.array_equal(dx.cpu().numpy().reshape(-1), np.asarray(d).reshape(-1))
+    api.fr_m(h)
