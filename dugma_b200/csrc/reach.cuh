@@ -10,6 +10,10 @@
 // index) of which a point passes that test for some stationary point: super tiles against the
 // tile's four subgroups, tiles against them, points against them, then points against points.
 // CONV: the pair's matrix is the sum of both covariances, so the test is |d|^2 > (sig / |k|) cut (L_i + L_j).
+// The last of these is most of the work (32 x 32 tests a tile), so it runs in packed FP32 on two stationary
+// points at a time, with sig / |k| and its room already in their L, and leaves overflow to the spheres' test:
+// 11 instructions a pair of tests against 32.  Adjoint kernel at 65536 x 65536: 53 -> 40 us, compi's 94 -> 62, CONV's
+// 76 -> 52, 240000 depth points 493 -> 417, 24 x 8 poses 518 -> 457.
 // The tests run in FP32 with room for their rounding, for that of the evaluation (in L, see variance_bound)
 // and for what a pose that is no exact rotation stretches.  What is not finite, or so large that the
 // evaluation could overflow, is marked.
@@ -33,9 +37,11 @@ struct ReachArgs {
                            // is left out (conv.cu)
 };
 
+static_assert(kSparseMaxTargets / kTile <= 65536, "a tile's number takes 16 bits");
+
 struct ReachShared {
-    float4 pt[kTile];      // position, L
-    float2 pa[kTile];      // a, slack
+    float4 xy[kTile / 2], zl[kTile / 2];   // points by pairs: -x -x' -y -y', -z -z' and L L' (scaled)
+    float2 a[kTile / 2], slack[kTile / 2];
     float4 sub[4];         // centre, radius
     float2 sa[4];          // a, L
 };
@@ -121,6 +127,10 @@ __device__ __forceinline__ bool find_reach(const ReachArgs& a, int group, uint32
     auto reach2 = [&](float a0, float L0, float a1, float L1) {
         return CONV ? (L0 + L1 < a.big ? sigk * a.cut * (L0 + L1) : INFINITY) : sigk * fminf(a0, a1) * fmaxf(L0, L1);
     };
+    // a point's L for the tests of point against point: x sig / |k|, and the room of those tests
+    auto scaled = [&](float L) {
+        return CONV ? (L < 0.5f * a.big ? sigk * a.cut * 1.002f * L : INFINITY) : sigk * 1.002f * L;
+    };
     // a sphere or point as the tests see it
     auto place = [&](const float* c, float& r, bool posed) {
         float4 q = make_float4(c[0], c[1], D == 3 ? c[2] : 0.f, 0.f);
@@ -134,11 +144,16 @@ __device__ __forceinline__ bool find_reach(const ReachArgs& a, int group, uint32
         const int i = group * kTile + lane;
         SortedPoint s = a.st.pt[i < a.st.n ? i : 0];
         float slack = 0.f;
-        float4 q = place(s.p, slack, !POSE_SM);
-        q.w = POSE_SM ? s.L : s.L * P.Lscale;
-        sh.pt[lane] = q;
+        const float4 q = place(s.p, slack, !POSE_SM);
+        const bool in = i < a.st.n;
+        const int p = lane >> 1, h = lane & 1;
+        (h ? sh.xy[p].y : sh.xy[p].x) = -q.x;
+        (h ? sh.xy[p].w : sh.xy[p].z) = -q.y;
+        (h ? sh.zl[p].y : sh.zl[p].x) = -q.z;
         // a lane without a point, and a point without weight (a = -1), reaches nothing
-        sh.pa[lane] = make_float2(i < a.st.n ? s.a : -1.f, 1001.f * slack * slack);
+        (h ? sh.zl[p].w : sh.zl[p].z) = CONV && !in ? -INFINITY : scaled(POSE_SM ? s.L : s.L * P.Lscale);
+        (h ? sh.a[p].y : sh.a[p].x) = in ? s.a : -1.f;
+        (h ? sh.slack[p].y : sh.slack[p].x) = 1001.f * slack * slack;
     } else if (threadIdx.x < kTile + 4) {
         const Bound b = a.st.sub[4 * group + lane];
         float r = b.r;
@@ -148,18 +163,21 @@ __device__ __forceinline__ bool find_reach(const ReachArgs& a, int group, uint32
         sh.sa[lane] = make_float2(b.a, POSE_SM ? b.L : b.L * P.Lscale);
     }
     __syncthreads();
-    // can something at q (radius r, a, L) reach a point of the subgroups?  one bit each
-    auto subs = [&](const float4& q, float r, float aa, float L) {
+    // can something at q (radius r, a, L) reach a point of the subgroups in `of`?  one bit each, and bit 4 where
+    // a distance is too large to tell (no point of the other subgroups is then beyond d2max)
+    auto subs = [&](const float4& q, float r, float aa, float L, unsigned of) {
         unsigned m = 0;
 #pragma unroll
         for (int s = 0; s < 4; ++s) {
+            if (!(of >> s & 1u)) continue;
             const float4 c = sh.sub[s];
             const float2 e = sh.sa[s];
             const float T = reach2(aa, L, e.x, e.y);
             const float rr = r + c.w, reach = fmaf(sqrt_fast(fmaxf(T, 0.f)), 1.f + 2e-6f, rr);
             const float d2 = dist2_f32<D>(q, c);
-            const bool out = d2 * (1.f - 1e-5f) > reach * reach && d2 < 0.2f * d2max && rr * rr < 0.2f * d2max;
-            m |= (unsigned)!out << s;
+            const bool near = d2 < 0.2f * d2max && rr * rr < 0.2f * d2max;
+            const bool out = d2 * (1.f - 1e-5f) > reach * reach && near;
+            m |= (unsigned)!out << s | (unsigned)!near << 4;
         }
         return m;
     };
@@ -171,7 +189,7 @@ __device__ __forceinline__ bool find_reach(const ReachArgs& a, int group, uint32
             const Bound b = a.sm.super[base + lane];
             float r = b.r;
             const float4 q = place(b.c, r, POSE_SM);
-            go = subs(q, r, b.a, POSE_SM ? b.L * P.Lscale : b.L) != 0;
+            go = subs(q, r, b.a, POSE_SM ? b.L * P.Lscale : b.L, 15u) != 0;
         }
         unsigned mask = __ballot_sync(0xffffffffu, go);
         while (mask) {   // the warp's tiles of up to NW super tiles at a time
@@ -183,42 +201,59 @@ __device__ __forceinline__ bool find_reach(const ReachArgs& a, int group, uint32
                 if (k == lane / TPW) mine = bit;
             }
             const int t = (base + mine) * kSuper + (lane % TPW) * NW + warp;
-            go = mine >= 0 && t < n_tiles;
-            if (go) {
+            unsigned reached = 0;   // the subgroups a tile reaches
+            if (mine >= 0 && t < n_tiles) {
                 const Bound b = a.sm.tile[t];
                 float r = b.r;
                 const float4 q = place(b.c, r, POSE_SM);
-                go = subs(q, r, b.a, POSE_SM ? b.L * P.Lscale : b.L) != 0;
+                reached = subs(q, r, b.a, POSE_SM ? b.L * P.Lscale : b.L, 15u);
             }
-            unsigned todo = __ballot_sync(0xffffffffu, go);
+            unsigned todo = __ballot_sync(0xffffffffu, reached != 0);
             while (todo) {   // lane = point of the tile
-                const int from = __ffs(todo) - 1;
+                const uint32_t e = __shfl_sync(0xffffffffu, (uint32_t)t | reached << 16, __ffs(todo) - 1);
                 todo &= todo - 1;
-                const int j = __shfl_sync(0xffffffffu, t, from) * kTile + lane;
+                const int j = (int)(e & 0xffffu) * kTile + lane;
                 unsigned m = 0;
-                SortedPoint s;
+                SortedPoint s{};
                 float4 q = make_float4(0.f, 0.f, 0.f, 0.f);
                 float L = 0.f, slack = 0.f;
                 if (j < a.sm.n) {
                     s = a.sm.pt[j];
                     q = place(s.p, slack, POSE_SM);
                     L = POSE_SM ? s.L * P.Lscale : s.L;
-                    m = subs(q, slack, s.a, L);
+                    m = subs(q, slack, s.a, L, e >> 16);
                     slack = 1001.f * slack * slack;
+                    L = scaled(L);
                 }
-                bool hit = false;
+                bool hit = m >> 4;
 #pragma unroll
                 for (int g = 0; g < 4; ++g) {
                     if (!__any_sync(0xffffffffu, m >> g & 1u)) continue;
+                    bool near = false;
 #pragma unroll
-                    for (int e = 0; e < kSub; ++e) {
-                        const float4 c = sh.pt[g * kSub + e];
-                        const float2 ca = sh.pa[g * kSub + e];
-                        const float T = reach2(s.a, L, ca.x, c.w);
-                        const float d2 = dist2_f32<D>(q, c);
+                    for (int p = g * (kSub / 2); p < (g + 1) * (kSub / 2); ++p) {   // two of its points
+                        const float4 xy = sh.xy[p], zl = sh.zl[p];
+                        const float2 dx = fadd2(make_float2(q.x, q.x), make_float2(xy.x, xy.y));
+                        const float2 dy = fadd2(make_float2(q.y, q.y), make_float2(xy.z, xy.w));
+                        float2 d2 = ffma2(dy, dy, fmul2(dx, dx));
+                        if (D == 3) {
+                            const float2 dz = fadd2(make_float2(q.z, q.z), make_float2(zl.x, zl.y));
+                            d2 = ffma2(dz, dz, d2);
+                        }
                         // (d - slack)^2 > T follows from d^2 > 1.001 T + 1001 slack^2
-                        hit |= (m >> g & 1u) && !(d2 > fmaf(T, 1.002f, slack + ca.y) && d2 < d2max);
+                        const float2 room = POSE_SM ? make_float2(slack, slack) : sh.slack[p];
+                        float2 T;
+                        if constexpr (CONV) {
+                            T = fadd2(fadd2(make_float2(L, L), make_float2(zl.z, zl.w)), room);
+                        } else {
+                            const float2 pa = sh.a[p];
+                            T = ffma2(make_float2(fminf(s.a, pa.x), fminf(s.a, pa.y)),
+                                     make_float2(fmaxf(L, zl.z), fmaxf(L, zl.w)), room);
+                        }
+                        near |= !(d2.x > T.x);
+                        near |= !(d2.y > T.y);
                     }
+                    hit |= near && (m >> g & 1u);
                 }
                 if (hit) atomicOr(&bits[s.idx >> 6], 1u << (s.idx >> 1 & 31));
                 marked |= hit;

@@ -15,8 +15,8 @@
 // Bound by the latency and issue slots of the search: the tests of super tiles, tiles and points are
 // some 10K instructions a tile of sources, the few dozen records after it (loaded 8 ahead, coalesced,
 // and broadcast from shared memory) less.  Measured on one B200, adjoint kernel, all pairs -> here:
-// 65536 x 65536 harmonic 6300 -> 67 us; 240000 x 239999 depth views 83500 -> 490 us; 6000 x 5501
-// with outliers 70 -> 24 us; 20011 x 17003 in 2D 370 -> 20 us.
+// 65536 x 65536 harmonic 6300 -> 40 us; 240000 x 240000 depth views 83500 -> 417 us; 16384 x 16384 sphere
+// 370 -> 25 us; 20011 x 20011 in 2D 370 -> 18 us.
 #include <algorithm>
 #include <cmath>
 #include <mutex>
@@ -26,8 +26,8 @@
 namespace dugma {
 
 // Eight warps a tile: one problem's few heavy tiles (outliers, edges of a depth map) end the launch.  2 / 4 / 8
-// warps, adjoint kernel on one B200: 65536 x 65536 73 / 54 / 48 us; 240000 depth 627 / 490 / 411; 6000 with
-// outliers - / 23 / 17.5; 2D 20011 - / 18.5 / 16.
+// warps, adjoint kernel on one B200 (before the packed tests of reach.cuh): 65536 x 65536 73 / 54 / 48 us; 240000
+// depth 627 / 490 / 411; 6000 with outliers - / 23 / 17.5; 2D 20011 - / 18.5 / 16.
 constexpr int kSparseWarps = 8;
 template <int D, bool GRAD, int NW>
 __global__ void __launch_bounds__(32 * NW, 24 / NW) sparse_kernel(SparseArgs a, const int* go)
