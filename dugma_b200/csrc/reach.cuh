@@ -37,6 +37,10 @@ struct ReachArgs {
                            // is left out (conv.cu)
 };
 
+// Super tiles (of 1024 points) beyond which the block shares their tests.  Adjoint kernel on one B200, each warp
+// all / shared: 240000 depth points (235) 418 -> 354 us, compi 673 -> 623; 65536 points (64) 40 us either way; below,
+// the two barriers cost up to 1 us of 25.
+constexpr int kReachShare = 64;
 static_assert(kSparseMaxTargets / kTile <= 65536, "a tile's number takes 16 bits");
 
 struct ReachShared {
@@ -44,6 +48,8 @@ struct ReachShared {
     float2 a[kTile / 2], slack[kTile / 2];
     float4 sub[4];         // centre, radius
     float2 sa[4];          // a, L
+    int n_super;
+    uint16_t super[256];   // super tiles that reach the tile, of the 32 NW tested together
 };
 
 // R y + t in FP32 (stretch, Lscale: how much R can stretch a length and a variance)
@@ -161,6 +167,8 @@ __device__ __forceinline__ bool find_reach(const ReachArgs& a, int group, uint32
         q.w = r;
         sh.sub[lane] = q;
         sh.sa[lane] = make_float2(b.a, POSE_SM ? b.L : b.L * P.Lscale);
+    } else if (threadIdx.x == kTile + 4) {
+        sh.n_super = 0;
     }
     __syncthreads();
     // can something at q (radius r, a, L) reach a point of the subgroups in `of`?  one bit each, and bit 4 where
@@ -183,22 +191,46 @@ __device__ __forceinline__ bool find_reach(const ReachArgs& a, int group, uint32
     };
     bool marked = false;
     const int n_tiles = (a.sm.n + kTile - 1) / kTile, n_super = (n_tiles + kSuper - 1) / kSuper;
-    for (int base = 0; base < n_super; base += 32) {
-        bool go = base + lane < n_super;
+    // Each warp tests all super tiles; where they are many a thread tests one, and the block goes on with a list of
+    // those that reach (two barriers).
+    const bool share = n_super > kReachShare;
+    for (int base = 0; base < n_super; base += share ? 32 * NW : 32) {
+        const int u = base + (share ? (int)threadIdx.x : lane);
+        bool go = u < n_super;
         if (go) {
-            const Bound b = a.sm.super[base + lane];
+            const Bound b = a.sm.super[u];
             float r = b.r;
             const float4 q = place(b.c, r, POSE_SM);
             go = subs(q, r, b.a, POSE_SM ? b.L * P.Lscale : b.L, 15u) != 0;
         }
         unsigned mask = __ballot_sync(0xffffffffu, go);
-        while (mask) {   // the warp's tiles of up to NW super tiles at a time
+        int listed = 0;
+        if (share) {
+            if (base) {   // (the last list has been read)
+                __syncthreads();
+                if (threadIdx.x == 0) sh.n_super = 0;
+                __syncthreads();
+            }
+            int at = 0;
+            if (lane == 0 && mask) at = atomicAdd(&sh.n_super, __popc(mask));
+            at = __shfl_sync(0xffffffffu, at, 0) + __popc(mask & ((1u << lane) - 1u));
+            if (go) sh.super[at] = (uint16_t)threadIdx.x;
+            __syncthreads();
+            listed = sh.n_super;
+            mask = 0;
+        }
+        // the warp's tiles of up to NW super tiles at a time
+        for (int first = 0; mask || first < listed; first += NW) {
             int mine = -1;
+            if (share) {
+                if (first + lane / TPW < listed) mine = sh.super[first + lane / TPW];
+            } else {
 #pragma unroll
-            for (int k = 0; k < NW; ++k) {
-                const int bit = __ffs(mask) - 1;   // -1: none left
-                mask &= mask - 1;
-                if (k == lane / TPW) mine = bit;
+                for (int k = 0; k < NW; ++k) {
+                    const int bit = __ffs(mask) - 1;   // -1: none left
+                    mask &= mask - 1;
+                    if (k == lane / TPW) mine = bit;
+                }
             }
             const int t = (base + mine) * kSuper + (lane % TPW) * NW + warp;
             unsigned reached = 0;   // the subgroups a tile reaches

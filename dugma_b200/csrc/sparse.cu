@@ -15,7 +15,7 @@
 // Bound by the latency and issue slots of the search: the tests of super tiles, tiles and points are
 // some 10K instructions a tile of sources, the few dozen records after it (loaded 8 ahead, coalesced,
 // and broadcast from shared memory) less.  Measured on one B200, adjoint kernel, all pairs -> here:
-// 65536 x 65536 harmonic 6300 -> 40 us; 240000 x 240000 depth views 83500 -> 417 us; 16384 x 16384 sphere
+// 65536 x 65536 harmonic 6300 -> 40 us; 240000 x 240000 depth views 83500 -> 354 us; 16384 x 16384 sphere
 // 370 -> 25 us; 20011 x 20011 in 2D 370 -> 18 us.
 #include <algorithm>
 #include <cmath>
