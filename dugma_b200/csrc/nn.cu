@@ -273,10 +273,10 @@ __global__ void __launch_bounds__(32 * NW) nn_prune_kernel(PruneArgs a)
 {
     constexpr int KL = K > 0 ? K : 1;
     constexpr unsigned long long kNone = (unsigned long long)0x7f800000u << 32 | 0x7fffffffu;
-    __shared__ int s_bound[kTile];                      // bounds on the lanes' k-th distances (float bits)
+    __shared__ __align__(8) int s_bound[kTile];         // bounds on the lanes' k-th distances (float bits)
     __shared__ int s_best[kTile];                       // K = 0: the squared distances
     __shared__ int s_first[NW];
-    __shared__ float s_x[3][kTile];
+    __shared__ __align__(8) float s_x[3][kTile];        // minus the sources
     __shared__ __align__(16) float4 s_rec[NW][2][kTile];   // two tiles of records per warp
     __shared__ unsigned long long s_list[K > 0 ? NW - 1 : 1][KL][kTile];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -297,7 +297,7 @@ __global__ void __launch_bounds__(32 * NW) nn_prune_kernel(PruneArgs a)
     if (warp == 0) {
         s_best[lane] = s_bound[lane] = __float_as_int(bound);
 #pragma unroll
-        for (int q = 0; q < 3; ++q) s_x[q][lane] = s.p[q];
+        for (int q = 0; q < 3; ++q) s_x[q][lane] = in ? -s.p[q] : 1e18f;   // (out of every sphere's reach)
     }
     pdl_wait();
     __syncthreads();
@@ -354,14 +354,27 @@ __global__ void __launch_bounds__(32 * NW) nn_prune_kernel(PruneArgs a)
     };
 
     const float4* super = a.sphere + a.n_tiles;
-    // lane = sphere: can any source still need it?  (many spheres at a time, one test each per source)
+    // lane = sphere: can any source still need it?  (many spheres at a time, one test each per source, in packed FP32
+    // on two sources: update_sig 65536 x 65536 33.5 -> 29.5 us, 240000 depth points 135 -> 116, k = 8 at 30000 83 -> 75)
     auto filter = [&](float4 c, bool go) {
         bool any = false;
+        const float2 w2 = make_float2(c.w, c.w), less = make_float2(1.f - 1e-5f, 1.f - 1e-5f);
 #pragma unroll 4
-        for (int q = 0; q < kTile; ++q) {
-            const float x[3] = {s_x[0][q], s_x[1][q], s_x[2][q]};
-            const float b = __int_as_float(*(volatile int*)&s_bound[q]);
-            any |= b >= 0.f && !beyond(dist2<D>(x, c), c.w, b);
+        for (int q = 0; q < kTile; q += 2) {
+            const long long b2 = *(const volatile long long*)&s_bound[q];
+            const int2 b = make_int2((int)b2, (int)(b2 >> 32));
+            const float2 d0 = fadd2(make_float2(c.x, c.x), *(const float2*)&s_x[0][q]);
+            const float2 d1 = fadd2(make_float2(c.y, c.y), *(const float2*)&s_x[1][q]);
+            float2 d = ffma2(d1, d1, fmul2(d0, d0));
+            if (D == 3) {
+                const float2 d2 = fadd2(make_float2(c.z, c.z), *(const float2*)&s_x[2][q]);
+                d = ffma2(d2, d2, d);
+            }
+            d = fmul2(d, less);   // (beyond, twice)
+            const float2 r = fadd2(w2, make_float2(__int_as_float(b.x), __int_as_float(b.y)));
+            const float2 rr = fmul2(r, r);
+            any |= !(d.x > rr.x);
+            any |= !(d.y > rr.y);
         }
         return __ballot_sync(0xffffffffu, go && any);
     };
