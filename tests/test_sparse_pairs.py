@@ -179,3 +179,10 @@ def test_device_pose_is_host_pose(model):
         assert got[0] == E and np.array_equal(got[1:7], np.asarray(g).reshape(-1))
         assert np.array_equal(dx.cpu().numpy().reshape(-1), np.asarray(d).reshape(-1))
     api.fr_m(h)
+
+
+@pytest.mark.parametrize("kind,m", [("sphere", 70001), ("sphere", 300001), ("not_finite", 270000)])
+def test_many_super_tiles(kind, m, monkeypatch):
+    """Targets beyond 64 super tiles (65536 points), whose tests the block shares, and beyond the 128 or 256
+    that it tests together: the same sums as all pairs."""
+    _compare(monkeypatch, {**ENERGY, **CONV, **COEF}, kind, 501, m, (2e-4, 4e-3))
