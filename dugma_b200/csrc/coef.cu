@@ -1212,7 +1212,7 @@ struct MomSide {
     const float* p;       // the side's points, D per row
     const float* cinv;    // its inverse covariances, D x D per row
     double* out;          // [nblk][moments] block partials
-    const int* sparse;    // nullable: when set, h1 holds the rows, one copy
+    const int* sparse;    // (PICK) when set, h1 holds the rows, one copy
     const double* h1;
 };
 
@@ -1220,8 +1220,9 @@ struct MomSide {
 // split its rows.  Each pass stages kMomRows rows -- H summed over its copies (one (row, feature)
 // entry per thread, coalesced), the row's matrix and monomials -- in shared memory; each thread
 // then owns one moment of the side and sums its products over the staged rows.  Per-block
-// partials in fixed order (deterministic).
-template <int D>
+// partials in fixed order (deterministic).  PICK: the rows are chosen on the device (a choice of pointers for every
+// call cost the 2D kernel its load schedule: 3868 x 4925 81.3 us a call against 76.4).
+template <int D, bool PICK>
 __global__ void __launch_bounds__(kMomThreads) moments_kernel(const MomSide s0, const MomSide s1,
                                                               const double* __restrict__ pose)
 {
@@ -1232,8 +1233,8 @@ __global__ void __launch_bounds__(kMomThreads) moments_kernel(const MomSide s0, 
     const float* __restrict__ p = ms.p;
     const float* __restrict__ cinv = ms.cinv;
     double* __restrict__ block_out = ms.out;
-    const int n_jc = ms.sparse && *ms.sparse ? 1 : ms.copies, n = ms.n, side = ms.side;
-    const double* __restrict__ hpart = ms.sparse && *ms.sparse ? ms.h1 : ms.h;
+    const int n_jc = PICK && *ms.sparse ? 1 : ms.copies, n = ms.n, side = ms.side;
+    const double* __restrict__ hpart = PICK && *ms.sparse ? ms.h1 : ms.h;
     constexpr int NS = Sym<D>::N, NF = Feat<D>::N;
     constexpr int NM = D == 3 ? kNumMoments3D : kNumMoments2D;
     const signed char(*tab)[4] = D == 3 ? c_moment3 : c_moment2;
@@ -1612,7 +1613,7 @@ static int coef_fused_launch(Context& c, const double* pose_dev, double* moments
     const MomSide m0{dense ? a.h2_part : rows2, dense ? n_jc : 1, c.N, nb0, 0, c.x, c.xinv, c.mom_part, flag, rows2};
     const MomSide m1{dense ? a.h1_part : rows1, dense ? n_grp : 1, c.M, nb1, 1, c.y, c.yinv,
                      c.mom_part + (size_t)nblk * NM, flag, rows1};
-    DUGMA_CK(launch_dependent(c.pdl, moments_kernel<D>, dim3(std::max(nb0, nb1), 2), kMomThreads, 0, s, m0, m1,
+    DUGMA_CK(launch_dependent(c.pdl, flag ? moments_kernel<D, true> : moments_kernel<D, false>, dim3(std::max(nb0, nb1), 2), kMomThreads, 0, s, m0, m1,
                               (const double*)pose_dev));
     DUGMA_CK(launch_dependent(c.pdl, moments_reduce_kernel, (NM + 7) / 8, 256, 0, s, (const double*)c.mom_part, nb0,
                               (const double*)(c.mom_part + (size_t)nblk * NM), nb1, NM, moments_dev,
@@ -1702,7 +1703,7 @@ static int coef_impl(Context& c, double* pose_dev, double* moments_dev, cudaStre
         const MomSide ms = side == 0 ? MomSide{hp, n_jc, rows, nb, 0, c.x + o1, c.xinv + o2, mom, nullptr, nullptr}
                                      : MomSide{hp, n_jc, rows, nb, 1, c.y + o1, c.yinv + o2, mom + (size_t)nblk * NM,
                                                nullptr, nullptr};
-        moments_kernel<D><<<dim3(nb, 1), kMomThreads, 0, s>>>(ms, ms, pose_dev);
+        moments_kernel<D, false><<<dim3(nb, 1), kMomThreads, 0, s>>>(ms, ms, pose_dev);
         if (cudaGetLastError() != cudaSuccess) rc = set_error(DUGMA_ERR_CUDA, "moments kernel launch failed");
     }
     if (rc == DUGMA_OK) {
