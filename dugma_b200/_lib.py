@@ -59,6 +59,8 @@ EXPORTS = {
                                c_int, dp, dp, dp]),
     "dugma_version": (ctypes.c_char_p, []),
     "dugma_timing": (c_int, [PtrArray, c_int, dp, ip]),
+    "dugma_last_pass": (c_int, [PtrArray, ip]),
+    "dugma_batch_last_pass": (c_int, [c_void_p, ip]),
     "dugma_shapes": (c_int, [c_int, ip, c_int]),
     "dugma_knn_covariance": (c_int, [dp, c_int, c_int, c_int, c_double, c_double, dp]),
     "dugma_minimise_surrogate": (c_int, [c_int, dp, dp, dp, dp, ip]),

@@ -217,6 +217,14 @@ def set_shape(h: Handles, what, shape):
     check(_lib.load().dugma_set_shape(h.arr, int(what), *[int(v) for v in shape]))
 
 
+def last_pass(h: Handles) -> tuple:
+    """How the last evaluations went: (0 all pairs, 1 only those above the FP32 flush, 2 the device decides;
+    an energy's sources per thread over all pairs, 0 for none; 1 for a pruned neighbour search)."""
+    buf = (ctypes.c_int * 3)()
+    check(_lib.load().dugma_last_pass(h.arr, buf))
+    return tuple(buf)
+
+
 class Batch:
     """Many registration problems (uneven sizes) evaluated together: one persistent launch
     per evaluation over every (problem, pose) pair, replayed as a CUDA graph after the first."""
@@ -276,6 +284,13 @@ class Batch:
         ms, n = ctypes.c_double(0), ctypes.c_int(0)
         check(_lib.load().dugma_batch_timing(self.b, int(mode), ctypes.byref(ms), ctypes.byref(n)))
         return ms.value, n.value
+
+    def last_pass(self) -> tuple:
+        """Of the last evaluation: ((problem, pose)s evaluated over the pairs above the FP32 flush only, the
+        launches they were split into, warps per tile of sources there)."""
+        s = (ctypes.c_int * 3)()
+        check(_lib.load().dugma_batch_last_pass(self.b, s))
+        return tuple(s)
 
     @staticmethod
     def shapes():

@@ -883,6 +883,16 @@ int dugma_set_shape(float* Ptr[6], int what, int ipt, int nt, int tj, int pack)
     return set_error(DUGMA_ERR_ARG, "set_shape: (%d, %d, %d, %d) is not a compiled shape", ipt, nt, tj, pack);
 }
 
+int dugma_last_pass(float* Ptr[6], int info[3])
+{
+    GET_CTX(c, Ptr);
+    if (!info) return set_error(DUGMA_ERR_ARG, "last_pass: null argument");
+    info[0] = c->last_pass;
+    info[1] = c->last_ipt;
+    info[2] = c->last_search;
+    return DUGMA_OK;
+}
+
 // mode 1: start recording (clears), 0: stop, 2: synchronise and report the total duration
 // (ms) and count of the main pairwise-kernel launches recorded since mode 1.
 int dugma_timing(float* Ptr[6], int mode, double* total_ms, int* launches)

@@ -334,6 +334,7 @@ struct Batch {
     int max_tiles = 0, max_words = 0; // source tiles, target bitmap words of the largest problem
     bool all_pairs = false;           // no pair sparse (while the dense shapes are timed)
     bool any_dense = true, any_sparse = false;   // of the evaluation at hand
+    int n_sparse = 0, sparse_warps = 0;          // its sparse pairs, and the warps per tile they take
     bool chol = true;                 // every problem's weighted sources have Cholesky factors
     cudaGraphExec_t exec = nullptr;
     cudaGraph_t graph = nullptr;
@@ -517,6 +518,7 @@ static int batch_enqueue(Batch& b, cudaStream_t s)
     // 670 with eight: the work that each warp repeats counts), eight where they do not
     const bool two = (size_t)b.max_tiles * n_pq > (size_t)6 * sms;
     auto sparse = two ? batch_sparse_kernel<D, 2> : batch_sparse_kernel<D, 8>;
+    b.sparse_warps = two ? 2 : 8;
     const size_t smem = (two ? SparseShape<2>::kFixed : SparseShape<8>::kFixed) + sizeof(uint32_t) * b.max_words;
     DUGMA_CK(cudaFuncSetAttribute(sparse, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     for (size_t k = 0; k + 1 < b.slab.size(); ++k) {
@@ -571,6 +573,7 @@ static int batch_eval(Batch& b, int n_poses, const double* poses, double* out)
     DUGMA_RET(batch_prepare(b, n_poses));
     const int n_pq = b.P * n_poses, D = b.D;
     b.any_dense = b.any_sparse = false;
+    b.n_sparse = 0;
     for (int k = 0; k < n_pq; ++k) {
         double* h = b.host + 16 * (size_t)k;
         for (int q = 0; q < 16; ++q) h[q] = 0.0;
@@ -582,6 +585,7 @@ static int batch_eval(Batch& b, int n_poses, const double* poses, double* out)
         const bool sparse = !b.all_pairs && src[12] < b.below[k / n_poses];
         h[kPoseSparse] = sparse ? 1.0 : 0.0;
         (sparse ? b.any_sparse : b.any_dense) = true;
+        b.n_sparse += sparse;
     }
     DUGMA_CK(cudaMemcpyAsync(b.poses, b.host, sizeof(double) * 16 * n_pq, cudaMemcpyHostToDevice, b.stream));
     DUGMA_RET(batch_launch(b));
@@ -677,6 +681,16 @@ int dugma_batch_get_shape(void* batch, int shape[4])
     shape[1] = sh.nt;
     shape[2] = sh.tj;
     shape[3] = sh.chunk;
+    return DUGMA_OK;
+}
+
+int dugma_batch_last_pass(void* batch, int info[3])
+{
+    Batch* b = static_cast<Batch*>(batch);
+    if (!b || !info) return set_error(DUGMA_ERR_ARG, "batch_last_pass: null argument");
+    info[0] = b->n_sparse;
+    info[1] = b->n_sparse ? (int)b->slab.size() - 1 : 0;
+    info[2] = b->n_sparse ? b->sparse_warps : 0;
     return DUGMA_OK;
 }
 

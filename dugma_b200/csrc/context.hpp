@@ -103,6 +103,11 @@ struct Context {
     Bound *xtile = nullptr, *ytile = nullptr, *xsub = nullptr, *ysub = nullptr;
     Bound *xsuper = nullptr, *ysuper = nullptr;
     float4* ysphere = nullptr;                // the target tiles' and super tiles' spheres at a pose
+    // how the last evaluations went (dugma_last_pass)
+    int last_pass = 0;                        // energies, CONV, coefficients: 0 all pairs, 1 sparse, 2 both
+                                              // enqueued and the device's sigma decides
+    int last_ipt = 0;                         // sources per thread of that all-pairs kernel (0: none launched)
+    int last_search = 0;                      // nearest neighbours: 0 all pairs, 1 pruned
     bool nn_pinned = false;                   // a nearest-neighbour kernel shape was pinned: no pruning
     double* dedx = nullptr;                   // dE/dx rows (allocated on first request)
     void* nn_out = nullptr;                   // dugma_nn's results under a pinned shape (on request)

@@ -1079,6 +1079,8 @@ int conv_launch(Context& c, const double* pose_dev, bool grad, int i0, int i1, d
     const double below = packed && !force && i0 == 0 && i1 == c.N && c.nonpd == 0 ? sparse_sigma(c, SparseUse::conv) : 0.0;
     const bool both = !(sig > 0.0) && below > 0.0 && (double)c.N * c.M >= kSparseMinPairsAuto;
     const bool sparse = sig > 0.0 && sig < below;
+    c.last_pass = sparse ? 1 : (both ? 2 : 0);
+    c.last_ipt = sparse ? 0 : v->shape.ipt;
     const int* flag = both ? c.counter + 4 : nullptr;
     // source records always; target records scalar (YRec) or paired (YRec2, same bytes)
     const int n = std::max(c.M_pad, c.N_pad);

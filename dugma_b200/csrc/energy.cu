@@ -332,6 +332,8 @@ int launch_pairs(Context& c, const double* pose_dev, int model, bool grad, int i
         if (grad)
             return set_error(DUGMA_ERR_ARG, "the FP64 reference-precision model has no adjoint (use the "
                                             "finite-difference gradient)");
+        c.last_pass = 0;
+        c.last_ipt = 1;
         return ref64_launch(c, pose_dev, i0, i1, out_dev, s);
     }
     if (model != DUGMA_MODEL_REF) return set_error(DUGMA_ERR_ARG, "unknown model %d", model);
@@ -365,6 +367,8 @@ int launch_pairs(Context& c, const double* pose_dev, int model, bool grad, int i
     const bool known = sig > 0.0;
     const bool both = !known && below > 0.0 && (double)c.N * c.M >= kSparseMinPairsAuto;
     const bool sparse = known && sig < below;
+    c.last_pass = sparse ? 1 : (both ? 2 : 0);
+    c.last_ipt = sparse ? 0 : shape.ipt;
     if (io && io->pose_src) DUGMA_RET(launch_pose_in(c, io->pose_src, io->pose_out, s, true));
     const double* pose_read = io && io->pose_src ? io->pose_out : pose_dev;
     DUGMA_RET(launch_prologue(c, pose_read, layout, s, xchol, c.counter, io ? io->pv : nullptr,

@@ -646,6 +646,7 @@ static int nn_run(Context& c, double* pose_dev, int k, int* idx_dev, float* d2_d
         reset_err = false;
     }
     const bool pruned = nn_pruned(c, force, rows);
+    c.last_search = pruned;
     DUGMA_RET(launch_nn_prologue(c, pose_dev, s, pv, c.counter, reset_err ? c.err : nullptr, pruned));
     if (pruned) {
         const int K = !idx_dev ? 0 : (k <= 1 ? 1 : (k <= 8 ? 8 : 16));

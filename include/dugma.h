@@ -221,6 +221,10 @@ int dugma_batch_autotune(void* batch, int n_poses, const double* poses, char* re
  * synchronise and report the summed duration in ms and the number of evaluations. */
 int dugma_batch_timing(void* batch, int mode, double* total_ms, int* launches);
 
+/* How the last batched evaluation went: info[0] (problem, pose)s evaluated over the pairs above the FP32
+ * flush only, info[1] launches they were split into, info[2] warps per tile of sources there. */
+int dugma_batch_last_pass(void* batch, int info[3]);
+
 /* ---------------- registration driver ---------------- */
 
 enum {
@@ -243,6 +247,12 @@ int dugma_register(const double* X, const double* X_C, const double* Y, const do
  * (mode 1: start and clear, 0: stop, 2: synchronise and return the summed duration in ms
  * and the number of launches since mode 1). */
 int dugma_timing(float* Ptr[6], int mode, double* total_ms, int* launches);
+
+/* How this context's last evaluations went: info[0] energy, gradient (any model) or coefficients: 0 all
+ * pairs, 1 only the pairs whose terms are not below the FP32 flush, 2 both enqueued, the sigma on the
+ * device decides; info[1] source points per thread of an energy's or gradient's all-pairs kernel (0:
+ * none launched); info[2] nearest neighbours and sigma: 0 all pairs, 1 the pruned search. */
+int dugma_last_pass(float* Ptr[6], int info[3]);
 
 /* Measured peak of a GPU pipe on the current device: what = 0 FP32 fused multiply-add,
  * 1 SFU ex2, 2 packed f32x2 fused multiply-add; returns lane operations per second (and the

@@ -1,0 +1,99 @@
+"""Which way an evaluation goes (api.last_pass): the comparisons of the sparse passes with all pairs do
+compare two different passes, and inputs on which they can differ -- points that overflow FP32 beside
+finite statistics, batches of several slabs -- against all pairs (DUGMA_ALL_PAIRS=1 at init) to the
+rounding of FP64 additions, 1e-12."""
+import numpy as np
+import pytest
+
+from dugma_b200 import api
+from tests.test_sparse_pairs import COEF, CONV, ENERGY, _problem
+
+pytestmark = pytest.mark.gpu
+
+
+def _run(monkeypatch, calls, prob, R, t, sig, all_pairs):
+    """{name: (the pass taken, outputs or error code)}"""
+    if all_pairs:
+        monkeypatch.setenv("DUGMA_ALL_PAIRS", "1")
+    else:
+        monkeypatch.delenv("DUGMA_ALL_PAIRS", raising=False)
+    _, h = api.init(*prob[:4])
+    out = {}
+    try:
+        for name, fn in calls.items():
+            try:
+                got = [np.asarray(v) for v in fn(h, R, t, sig)]
+            except api.DugmaError as e:
+                got = e.code
+            out[name] = (api.last_pass(h)[0], got)
+    finally:
+        api.fr_m(h)
+    return out
+
+
+def _same(a, b, name):
+    if isinstance(a, int) or isinstance(b, int):
+        assert isinstance(a, int) and isinstance(b, int) and a == b, (name, a, b)
+        return
+    for u, v in zip(a, b):
+        assert np.array_equal(np.isfinite(u), np.isfinite(v)), name
+        u, v = u[np.isfinite(u)], v[np.isfinite(v)]
+        assert np.linalg.norm(u - v) <= 1e-12 * np.linalg.norm(v), (name, u, v)
+
+
+SPARSE = [(ENERGY, 6001, 5100), (ENERGY, 20001, 4001), (CONV, 7001, 6301), (CONV, 20001, 5025), (COEF, 6001, 5901)]
+
+
+@pytest.mark.filterwarnings("ignore")
+@pytest.mark.parametrize("calls,n,m", SPARSE)
+@pytest.mark.parametrize("kind", ["sphere", "outliers", "harmonic", "curve", "coincident"])
+def test_sparse_pass_is_taken(kind, calls, n, m, monkeypatch):
+    prob = _problem(kind, n, m, 3)
+    R, t = prob[4], prob[5] + 0.01
+    for all_pairs in (False, True):
+        for name, (took, _) in _run(monkeypatch, calls, prob, R, t, 2e-5, all_pairs).items():
+            assert took == (0 if all_pairs else 1), (name, took)
+
+
+@pytest.mark.filterwarnings("ignore")
+@pytest.mark.parametrize("calls,n,m", SPARSE)
+@pytest.mark.parametrize("what", ["inf_target", "inf_source", "inf_corner"])
+def test_points_beyond_fp32(what, calls, n, m, monkeypatch):
+    """A coordinate that is finite in FP64 and infinite in FP32: the other cloud's radius keeps the
+    evaluation sparse."""
+    X, XC, Y, YC, R, t = _problem("harmonic", n, m, 4)
+    if what == "inf_target":
+        Y[3, 0] = 1e39
+    elif what == "inf_source":
+        X[n // 2, 1] = -1e39
+    else:
+        Y[m - 1] = 1e39
+    prob = (X, XC, Y, YC)
+    for sig in (2e-5, 2e-3):
+        a = _run(monkeypatch, calls, prob, R, t + 0.01, sig, False)
+        b = _run(monkeypatch, calls, prob, R, t + 0.01, sig, True)
+        for name in b:
+            assert b[name][0] == 0 and (sig > 1e-4 or a[name][0] == 1), (name, a[name][0])
+            _same(a[name][1], b[name][1], name)
+
+
+def test_batch_of_several_slabs(monkeypatch):
+    """More source rows than one sparse launch takes (4M), among sparse and dense poses."""
+    probs = [_problem(k, 20001, 1301, s) for s, k in enumerate(("sphere", "harmonic", "sphere", "outliers", "sphere"))]
+    Q = 48
+    R = np.array([[p[4]] * Q for p in probs])
+    t = np.array([[p[5] + 0.001 * q for q in range(Q)] for p in probs])
+    sig = np.array([[1e-4] * (Q - 1) + [10.0]] * len(probs))
+    out = []
+    for all_pairs in (False, True):
+        if all_pairs:
+            monkeypatch.setenv("DUGMA_ALL_PAIRS", "1")
+        b = api.Batch([p[:4] for p in probs])
+        out.append(b.energy_grad(R, t, sig))
+        took = b.last_pass()
+        assert took[:2] == ((0, 0) if all_pairs else (len(probs) * (Q - 1), 2)), took
+        b.close()
+    for u, v in zip(*out):
+        for p in range(len(probs)):
+            for q in range(Q):
+                _same([u[p, q]], [v[p, q]], (p, q))
