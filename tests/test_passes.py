@@ -97,3 +97,35 @@ def test_batch_of_several_slabs(monkeypatch):
         for p in range(len(probs)):
             for q in range(Q):
                 _same([u[p, q]], [v[p, q]], (p, q))
+
+
+def _needles(n, m, seed):
+    """Half of each cloud on a line with needle covariances along it (condition 5e4: their pairs fail the
+    FP32 path's test, yet have a bound on their reach), the sources' on one side and the targets' on the
+    other, half beside the whole line with round ones."""
+    rng = np.random.default_rng(seed)
+    u = np.array([0.48, -0.6, 0.64])
+
+    def cloud(k, side):
+        s, needle = rng.uniform(-1, 1, k), rng.uniform(size=k) < 0.5
+        P = np.outer(np.where(needle, side * (0.1 + 0.9 * np.abs(s)), s), u)
+        P += np.where(needle, 1e-4, 0.02)[:, None] * rng.standard_normal((k, 3))
+        v = u + 1e-3 * rng.standard_normal((k, 3))
+        v *= rng.uniform(0.9, 1.1, (k, 1)) / np.linalg.norm(v, axis=1)[:, None]
+        flat = 1e-3 * v[:, :, None] * v[:, None, :] + 2e-8 * np.eye(3)
+        return P, np.where(needle[:, None, None], flat, 1e-3 * np.eye(3))
+
+    return (*cloud(n, -1.0), *cloud(m, 1.0), np.eye(3), np.zeros(3))
+
+
+@pytest.mark.parametrize("n,m", [(7001, 6301), (12001, 5001)])
+def test_conv_of_needles(n, m, monkeypatch):
+    """A pair that fails the FP32 path's test is evaluated in FP64; what the FP32 path made of it has no
+    say in which term is the largest, whether or not the pass comes upon that pair."""
+    prob = _needles(n, m, 5)
+    for sig in (3e-3, 8e-3):
+        a = _run(monkeypatch, CONV, prob, prob[4], prob[5] + 1e-3, sig, False)
+        b = _run(monkeypatch, CONV, prob, prob[4], prob[5] + 1e-3, sig, True)
+        for name in b:
+            assert (a[name][0], b[name][0]) == (1, 0), (name, a[name][0])
+            _same(a[name][1], b[name][1], name)
