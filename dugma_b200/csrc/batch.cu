@@ -331,7 +331,7 @@ struct Batch {
     int max_span = 0;
     double* rows = nullptr;           // a slab's source rows (sparse pairs)
     std::vector<int> slab;            // the slabs' first pairs, and n_pq
-    int max_tiles = 0, max_words = 0; // source tiles, target bitmap words of the largest problem
+    int max_tiles = 0, max_words = 0; // source tiles, target bitmap words of the largest problem that can be sparse
     bool all_pairs = false;           // no pair sparse (while the dense shapes are timed)
     bool any_dense = true, any_sparse = false;   // of the evaluation at hand
     int n_sparse = 0, sparse_warps = 0;          // its sparse pairs, and the warps per tile they take
@@ -402,8 +402,10 @@ static int batch_prepare(Batch& b, int n_poses)
         row0[pq] = (int)slab_rows;
         slab_rows += c.N;
         most_rows = std::max(most_rows, slab_rows);
-        b.max_tiles = std::max(b.max_tiles, (c.N + kTile - 1) / kTile);
-        b.max_words = std::max(b.max_words, (c.M_pad / 2 + 31) / 32);
+        if (b.below[pq / n_poses] > 0) {
+            b.max_tiles = std::max(b.max_tiles, (c.N + kTile - 1) / kTile);
+            b.max_words = std::max(b.max_words, (c.M_pad / 2 + 31) / 32);
+        }
     }
     b.slab.push_back(n_pq);
     std::vector<int> order(items.size());

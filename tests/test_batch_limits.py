@@ -1,0 +1,34 @@
+"""Problems of very different sizes in one batch: every problem that can be evaluated alone can be evaluated
+beside one of any other size."""
+import numpy as np
+import pytest
+
+from dugma_b200 import api
+from tests.test_sparse_pairs import _problem
+
+pytestmark = pytest.mark.gpu
+
+
+def _poses(probs, Q, sig):
+    R = np.array([[p[4]] * Q for p in probs])
+    t = np.array([[p[5] + 0.001 * q for q in range(Q)] for p in probs])
+    return R, t, np.full((len(probs), Q), sig)
+
+
+def test_sparse_problem_beside_a_huge_one():
+    """A problem of more targets than the sparse pass takes: it is evaluated over all pairs, and the
+    launch of the sparse one beside it does not grow with it."""
+    n, m = 16, 3700000
+    rng = np.random.default_rng(8)
+    small = _problem("sphere", 3001, 3000, 2)
+    eye = lambda k: np.broadcast_to(1e-3 * np.eye(3), (k, 3, 3))  # noqa: E731
+    big = (rng.uniform(-1, 1, (n, 3)), eye(n), rng.uniform(-1, 1, (m, 3)), eye(m), np.eye(3), np.zeros(3))
+    out = []
+    for k, probs in enumerate(([small], [small, big], [big])):
+        b = api.Batch([p[:4] for p in probs])
+        out.append(b.energy_grad(*_poses(probs, 2, 1e-4)))
+        assert b.last_pass()[0] == (0 if k == 2 else 2), b.last_pass()
+        b.close()
+    for k in range(2):
+        assert np.allclose(out[1][k][0], out[0][k][0], rtol=1e-12, atol=0)
+        assert np.allclose(out[1][k][1], out[2][k][0], rtol=1e-12, atol=0)
