@@ -17,6 +17,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <mutex>
 #include <numeric>
 #include <string>
 #include <vector>
@@ -491,6 +492,24 @@ static int batch_prepare(Batch& b, int n_poses)
     return DUGMA_OK;
 }
 
+// The sparse kernels' dynamic shared memory limit: once per device, and the most a launch can take (the
+// attribute belongs to the function, so every batch of the process shares it).
+template <int D>
+static int batch_sparse_setup(int dev)
+{
+    static std::mutex mu;
+    static bool done[64];
+    std::lock_guard<std::mutex> lk(mu);
+    if (dev < 64 && done[dev]) return DUGMA_OK;
+    constexpr size_t bits = kSparseMaxTargets / 64 * sizeof(uint32_t);
+    DUGMA_CK(cudaFuncSetAttribute(batch_sparse_kernel<D, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  (int)(SparseShape<2>::kFixed + bits)));
+    DUGMA_CK(cudaFuncSetAttribute(batch_sparse_kernel<D, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  (int)(SparseShape<8>::kFixed + bits)));
+    if (dev < 64) done[dev] = true;
+    return DUGMA_OK;
+}
+
 template <int D>
 static int batch_enqueue(Batch& b, cudaStream_t s)
 {
@@ -522,7 +541,7 @@ static int batch_enqueue(Batch& b, cudaStream_t s)
     auto sparse = two ? batch_sparse_kernel<D, 2> : batch_sparse_kernel<D, 8>;
     b.sparse_warps = two ? 2 : 8;
     const size_t smem = (two ? SparseShape<2>::kFixed : SparseShape<8>::kFixed) + sizeof(uint32_t) * b.max_words;
-    DUGMA_CK(cudaFuncSetAttribute(sparse, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    DUGMA_RET(batch_sparse_setup<D>(b.ctx[0]->dev));
     for (size_t k = 0; k + 1 < b.slab.size(); ++k) {
         const int q0 = b.slab[k], nq = b.slab[k + 1] - q0;
         sparse<<<dim3(b.max_tiles, nq), two ? 64 : 256, smem, s>>>(b.desc, q0, shift, var.sh.chunk, b.rows);

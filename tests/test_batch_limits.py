@@ -1,9 +1,11 @@
-"""Problems of very different sizes in one batch: every problem that can be evaluated alone can be evaluated
-beside one of any other size."""
+"""Batches beside one another and problems of very different sizes in one batch: every batch that can be
+evaluated alone can be evaluated while others are, and beside a problem of any other size."""
+import threading
+
 import numpy as np
 import pytest
 
-from dugma_b200 import api
+from dugma_b200 import _lib, api
 from tests.test_sparse_pairs import _problem
 
 pytestmark = pytest.mark.gpu
@@ -13,6 +15,38 @@ def _poses(probs, Q, sig):
     R = np.array([[p[4]] * Q for p in probs])
     t = np.array([[p[5] + 0.001 * q for q in range(Q)] for p in probs])
     return R, t, np.full((len(probs), Q), sig)
+
+
+def test_batches_in_threads():
+    """Sparse batches whose largest problems differ, from a thread each: their launches need different
+    amounts of shared memory, and none takes another's."""
+    L = _lib.load()
+    work = []
+    for s, (n, m) in enumerate([(1001, 900), (5001, 60000)] * 3):
+        probs = [_problem("sphere", n, m, s)]
+        b = api.Batch([p[:4] for p in probs])
+        pose = _poses(probs, 1, 1e-4)
+        E, g = b.energy_grad(*pose)
+        assert b.last_pass() == (1, 1, 8)
+        work.append((b, b._poses(*pose)[0], np.concatenate([E.ravel(), g.ravel()]), np.zeros(7)))
+    failed, start = [], threading.Barrier(len(work))
+
+    def run(b, rec, want, out):
+        start.wait(60)
+        for _ in range(4000):
+            if L.dugma_batch_energy_grad(b.b, 1, api._ptr(rec), 0, api._ptr(out)):
+                failed.append(L.dugma_last_error().decode())
+            elif not np.array_equal(out, want):
+                failed.append("another result")
+
+    threads = [threading.Thread(target=run, args=w) for w in work]
+    for th in threads:
+        th.start()
+    for th in threads:
+        th.join(600)
+    for w in work:
+        w[0].close()
+    assert not failed, (len(failed), failed[0])
 
 
 def test_sparse_problem_beside_a_huge_one():
