@@ -330,7 +330,9 @@ struct Batch {
     std::vector<std::pair<cudaEvent_t, cudaEvent_t>> tevents;
     size_t tused = 0;
     int max_span = 0;
-    double* rows = nullptr;           // a slab's source rows (sparse pairs)
+    double* rows = nullptr;           // a slab's source rows (sparse pairs; null until the first of them)
+    size_t row_bytes = 0;
+    void* rows_mem = nullptr;         // their own allocation, where mem was made without them
     std::vector<int> slab;            // the slabs' first pairs, and n_pq
     int max_tiles = 0, max_words = 0; // source tiles, target bitmap words of the largest problem that can be sparse
     bool all_pairs = false;           // no pair sparse (while the dense shapes are timed)
@@ -345,18 +347,31 @@ struct Batch {
         if (exec) cudaGraphExecDestroy(exec);
         if (graph) cudaGraphDestroy(graph);
         if (mem) cudaFree(mem);
+        if (rows_mem) cudaFree(rows_mem);
         if (host) cudaFreeHost(host);
         exec = nullptr;
         graph = nullptr;
-        mem = nullptr;
+        mem = rows_mem = nullptr;
+        rows = nullptr;
         host = nullptr;
         n_poses = 0;
     }
 };
 
-static int batch_prepare(Batch& b, int n_poses)
+// The state of a pose count and shape; with room for the sparse pairs' rows (up to 256 MB) where the
+// evaluation at hand has any, in the same allocation, or in one of their own if the state is there already.
+static int batch_prepare(Batch& b, int n_poses, bool sparse)
 {
-    if (b.n_poses == n_poses && b.prepared_shape == b.shape) return DUGMA_OK;
+    if (b.n_poses == n_poses && b.prepared_shape == b.shape) {
+        if (!sparse || b.rows) return DUGMA_OK;
+        if (cudaMalloc(&b.rows_mem, b.row_bytes) != cudaSuccess) {
+            cudaGetLastError();
+            b.rows_mem = nullptr;
+            return set_error(DUGMA_ERR_NOMEM, "batch: cannot allocate %zu bytes", b.row_bytes);
+        }
+        b.rows = static_cast<double*>(b.rows_mem);
+        return DUGMA_OK;
+    }
     cudaStreamSynchronize(b.stream);
     b.release_pose_state();
     const int D = b.D, NG = D == 3 ? 6 : 3;
@@ -396,12 +411,13 @@ static int batch_prepare(Batch& b, int n_poses)
     b.max_tiles = b.max_words = 0;
     for (int pq = 0; pq < n_pq; ++pq) {
         const Context& c = *b.ctx[pq / n_poses];
-        if (slab_rows + c.N > kSlabRows && slab_rows > 0) {
+        const size_t n = b.below[pq / n_poses] > 0 ? c.N : 0;
+        if (slab_rows + n > kSlabRows && slab_rows > 0) {
             b.slab.push_back(pq);
             slab_rows = 0;
         }
         row0[pq] = (int)slab_rows;
-        slab_rows += c.N;
+        slab_rows += n;
         most_rows = std::max(most_rows, slab_rows);
         if (b.below[pq / n_poses] > 0) {
             b.max_tiles = std::max(b.max_tiles, (c.N + kTile - 1) / kTile);
@@ -429,7 +445,8 @@ static int batch_prepare(Batch& b, int n_poses)
                  s_items = up(sizeof(BatchItem) * sorted.size()), s_start = up(sizeof(int) * (n_pq + 1)),
                  s_list = up(sizeof(int) * sorted.size()), s_ctr = 256, s_part = up(sizeof(double) * 8 * sorted.size()),
                  s_out = up(sizeof(double) * b.nv * n_pq), s_y = up(ybytes), s_x = up(xbytes),
-                 s_rows = up(sizeof(double) * 8 * most_rows);
+                 s_rows = sparse ? up(sizeof(double) * 8 * most_rows) : 0;
+    b.row_bytes = sizeof(double) * 8 * most_rows;
     const size_t total = s_poses + s_desc + s_items + s_start + s_list + s_ctr + s_part + s_out + s_y + s_x + s_rows;
     if (cudaMalloc(&b.mem, total) != cudaSuccess) {
         cudaGetLastError();
@@ -448,7 +465,7 @@ static int batch_prepare(Batch& b, int n_poses)
     b.out = reinterpret_cast<double*>(m); m += s_out;
     char* ybase = m; m += s_y;
     char* xbase = m; m += s_x;
-    b.rows = reinterpret_cast<double*>(m);
+    b.rows = sparse ? reinterpret_cast<double*>(m) : nullptr;
     std::vector<PQDesc> desc(n_pq);
     for (int p = 0; p < b.P; ++p) {
         const Context& c = *b.ctx[p];
@@ -591,10 +608,12 @@ static int batch_launch(Batch& b)
 
 static int batch_eval(Batch& b, int n_poses, const double* poses, double* out)
 {
-    DUGMA_RET(batch_prepare(b, n_poses));
     const int n_pq = b.P * n_poses, D = b.D;
-    b.any_dense = b.any_sparse = false;
     b.n_sparse = 0;
+    for (int k = 0; k < n_pq; ++k) b.n_sparse += !b.all_pairs && poses[13 * (size_t)k + 12] < b.below[k / n_poses];
+    b.any_sparse = b.n_sparse > 0;
+    b.any_dense = b.n_sparse < n_pq;
+    DUGMA_RET(batch_prepare(b, n_poses, b.any_sparse));
     for (int k = 0; k < n_pq; ++k) {
         double* h = b.host + 16 * (size_t)k;
         for (int q = 0; q < 16; ++q) h[q] = 0.0;
@@ -603,10 +622,7 @@ static int batch_eval(Batch& b, int n_poses, const double* poses, double* out)
         for (int a = 0; a < D; ++a) h[kPoseT + a] = src[9 + a];
         h[kPoseSig] = src[12];
         if (!(src[12] > 0)) return set_error(DUGMA_ERR_ARG, "batch_energy_grad: sig of pose %d is not positive", k);
-        const bool sparse = !b.all_pairs && src[12] < b.below[k / n_poses];
-        h[kPoseSparse] = sparse ? 1.0 : 0.0;
-        (sparse ? b.any_sparse : b.any_dense) = true;
-        b.n_sparse += sparse;
+        h[kPoseSparse] = !b.all_pairs && src[12] < b.below[k / n_poses] ? 1.0 : 0.0;
     }
     DUGMA_CK(cudaMemcpyAsync(b.poses, b.host, sizeof(double) * 16 * n_pq, cudaMemcpyHostToDevice, b.stream));
     DUGMA_RET(batch_launch(b));

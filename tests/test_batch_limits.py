@@ -66,3 +66,26 @@ def test_sparse_problem_beside_a_huge_one():
     for k in range(2):
         assert np.allclose(out[1][k][0], out[0][k][0], rtol=1e-12, atol=0)
         assert np.allclose(out[1][k][1], out[2][k][0], rtol=1e-12, atol=0)
+
+
+def test_rows_only_where_something_is_sparse():
+    """The sparse pass's rows (64 bytes a source and pose) are allocated by the first evaluation that has a
+    sparse pose, whatever came before it."""
+    import torch
+    probs = [_problem("sphere", 20001, 1301, s) for s in range(4)]
+    rows = 4 * 24 * 20001 * 64
+    out, used = [], []
+    for sigs in ((30.0, 1e-4), (1e-4, 30.0)):
+        b = api.Batch([p[:4] for p in probs])
+        got = []
+        for sig in sigs + sigs:
+            free = torch.cuda.mem_get_info()[0]
+            got.append(b.energy_grad(*_poses(probs, 24, sig)))
+            assert b.last_pass()[0] == (0 if sig > 1 else 96)
+            used.append(free - torch.cuda.mem_get_info()[0])
+        b.close()
+        assert all(np.array_equal(u, v) for k in range(2) for u, v in zip(got[k], got[k + 2]))
+        out.append(got)
+    assert all(np.array_equal(u, v) for k in range(2) for u, v in zip(out[0][k], out[1][1 - k]))
+    assert 0.9 * rows <= used[1] <= rows + (8 << 20) and used[4] >= used[0] + 0.9 * rows, (rows, used)
+    assert max(used[2:4] + used[5:]) <= 8 << 20, used
