@@ -801,12 +801,21 @@ int dugma_autotune(float* Ptr[6], int what, int model, char* report, size_t repo
         DUGMA_CK(cudaMalloc(&dd, sizeof(float) * c->N));
     }
     int rc = DUGMA_OK;
+    // The candidates are timed over all pairs (the sparse passes take their chunks from the shape, not their
+    // speed) as the calls then run them: for what = 0 and 1 in the context's slot and not pinned, so that a
+    // small problem's kernel stands in for the default shape here as it does there.
+    const KernelShape slot_was = shape_slot(*c, what);
+    const bool all_was = c->all_pairs, adj_was = c->adj_pinned, energy_was = c->energy_pinned;
+    c->all_pairs = true;
+    if (what == 0) c->adj_pinned = false;
+    if (what == 1) c->energy_pinned = false;
     for (auto& sh : cand) {
         auto run = [&]() {
             if (what == 2) return launch_nn(*c, c->pose, 1, di, dd, c->stream, &sh);
             if (what >= 3) return launch_pairs(*c, c->pose, DUGMA_MODEL_CONV, what == 3, 0, c->N, c->out, nullptr,
                                                c->stream, &sh);
-            return launch_pairs(*c, c->pose, model, what == 0, 0, c->N, c->out, nullptr, c->stream, &sh);
+            shape_slot(*c, what) = sh;
+            return launch_pairs(*c, c->pose, model, what == 0, 0, c->N, c->out, nullptr, c->stream);
         };
         rc = run();   // warm-up (also sizes scratch)
         if (rc != DUGMA_OK) break;
@@ -832,7 +841,13 @@ int dugma_autotune(float* Ptr[6], int what, int model, char* report, size_t repo
     cudaEventDestroy(e1);
     if (di) cudaFree(di);
     if (dd) cudaFree(dd);
-    if (rc != DUGMA_OK) return rc;
+    c->all_pairs = all_was;
+    if (rc != DUGMA_OK) {
+        shape_slot(*c, what) = slot_was;
+        c->adj_pinned = adj_was;
+        c->energy_pinned = energy_was;
+        return rc;
+    }
     shape_slot(*c, what) = best_shape;
     if (report && report_len) snprintf(report, report_len, "%s", rep.c_str());
     return DUGMA_OK;
@@ -878,6 +893,8 @@ int dugma_set_shape(float* Ptr[6], int what, int ipt, int nt, int tj, int pack)
         if (s.same(want)) {
             shape_slot(*c, what) = s;
             if (what == 2) c->nn_pinned = true;   // an all-pairs shape asked for: no pruned search
+            if (what == 0) c->adj_pinned = true;
+            if (what == 1) c->energy_pinned = true;
             return DUGMA_OK;
         }
     return set_error(DUGMA_ERR_ARG, "set_shape: (%d, %d, %d, %d) is not a compiled shape", ipt, nt, tj, pack);

@@ -136,6 +136,7 @@ struct Context {
     cudaStream_t stream = nullptr;
     int num_sms = 148;
     KernelShape shape_adj, shape_energy, shape_nn, shape_conv_adj, shape_conv_energy;
+    bool adj_pinned = false, energy_pinned = false;   // set by dugma_set_shape: no other shape for small problems
     std::mutex mu;                            // one host call at a time per context
     // optional timing of the main pairwise kernel (dugma_timing)
     bool timing = false;

@@ -208,8 +208,8 @@ void pair_split(const Context& c, KernelFn fn, const KernelShape& sh, int rows, 
     *n_jc_out = (total_tiles + *jc_tiles_out - 1) / *jc_tiles_out;
 }
 
-// Small problems take fewer sources per thread than the default shapes, on the default's own tiles and
-// chunks (so each source's FP32 sums stay what they are; only FP64 additions regroup): with four a
+// Small problems whose shape is not pinned take fewer sources per thread than the default shapes, on the
+// default's own tiles and chunks (so each source's FP32 sums stay what they are; only FP64 additions regroup): with four a
 // thread the items are too few, or too uneven, for 148 SMs.  One B200, us a call, 4 / 2 / 1 sources:
 //   adjoint  1000: 49 / 37 / 33;  2000: 47 / 36 / 36;  4500: 90 / 76 / 69;  7000: 119 / 121 / 112;  9000: 180 / 184 / 172;
 //            12000: 265 / 272 / 276;  65536: 6337 / 6460 / 6870
@@ -353,7 +353,8 @@ int launch_pairs(Context& c, const double* pose_dev, int model, bool grad, int i
     }
     KernelFn fn = v->fn;
     KernelShape shape = v->shape;
-    if (!force && shape.pack == 2) small_shape(c, grad, xchol, i1 - i0, &fn, &shape);
+    const bool pinned = force || (grad ? c.adj_pinned : c.energy_pinned);
+    if (!pinned && shape.pack == 2) small_shape(c, grad, xchol, i1 - i0, &fn, &shape);
     // record layout: 0 scalar adjoint, 1 scalar Horner energy, 2 / 3 their packed-pair forms
     const int layout = (grad ? 0 : 1) + (v->shape.pack == 2 ? 2 : 0);
     if (io && (io->pv || io->pose_src) && !io->pose_out)

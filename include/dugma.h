@@ -155,7 +155,9 @@ int dugma_energy_grad_noalloc(const float* x, const float* x_cov_inv, const floa
 
 /* Times the kernel shapes of `what` (0 = adjoint, 1 = energy, 2 = nearest neighbour, 3 = CONV
  * adjoint, 4 = CONV energy) on this context and keeps the fastest; writes a one-line report
- * into `report` (may be NULL).  `model` selects REF or CONV for what = 0 and 1. */
+ * into `report` (may be NULL).  `model` selects REF or CONV for what = 0 and 1.  Timed is what the calls
+ * run over all pairs: for small problems the default shape of what = 0 and 1 is run with fewer source
+ * points per thread.  Ends a pin of dugma_set_shape for what = 0 and 1. */
 int dugma_autotune(float* Ptr[6], int what, int model, char* report, size_t report_len);
 
 /* Kernel shapes available for `what` (0 adjoint, 1 energy, 2 nearest neighbour, 3 CONV adjoint,
@@ -169,7 +171,9 @@ int dugma_shapes(int what, int* shapes, int max);
  * target tiles of 32 per chunk, chunks}; items = groups x chunks.  Host-only (no device work). */
 int dugma_coef_work_grid(int N, int M, int resident, int grid[4]);
 
-/* Pins the kernel shape used for `what` on this context (one of dugma_shapes' tuples). */
+/* Pins the kernel shape used for `what` on this context (one of dugma_shapes' tuples): evaluations over all
+ * pairs run that kernel at every size, those over the pairs above the FP32 flush sum over its tiles and
+ * chunks, and a nearest-neighbour shape ends the pruned search. */
 int dugma_set_shape(float* Ptr[6], int what, int ipt, int nt, int tj, int pack);
 
 /* The kernel shape this context uses for `what`: shape[0..4) = {ipt, nt, tj, pack}. */
