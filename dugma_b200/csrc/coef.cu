@@ -1646,6 +1646,7 @@ static int coef_impl(Context& c, double* pose_dev, double* moments_dev, cudaStre
     const int* flag = both ? c.counter + 4 : nullptr;
     c.last_pass = both ? 2 : (sparse ? 1 : 0);
     c.last_ipt = 0;
+    TimingHold hold(c, false);
     const int pg = std::min((n + 127) / 128, c.num_sms * 8);
     auto prologue = chol ? coef_prologue_kernel<D, true> : coef_prologue_kernel<D, false>;
     prologue<<<pg, 128, 0, s>>>(pb, o.pose_value ? 1 : 0, pose_dev, c.y, c.yinv, c.lwy, c.M, c.M_pad, c.yrec128,

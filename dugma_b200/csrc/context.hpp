@@ -196,6 +196,14 @@ void pair_split(const Context& c, KernelFn fn, const KernelShape& sh, int rows, 
 // the interval stays open
 int timing_begin(Context& c, cudaStream_t s);
 int timing_end(Context& c, cudaStream_t s);
+// One evaluation's timing: the interval is held open over its kernels (when `on`) until release(), and one that an
+// error leaves open ends with the evaluation, not in the next one.
+struct TimingHold {
+    Context& c;
+    TimingHold(Context& ctx, bool on) : c(ctx) { c.timing_hold = on; }
+    void release() { c.timing_hold = false; }
+    ~TimingHold() { c.timing_hold = c.timing_open = false; }
+};
 // The REF energy or adjoint over the pairs above the FP32 flush (sparse.cu), from the records of the
 // packed kernels' prologue: the same sums as the all-pairs kernel with tiles of tile_rec and chunks of
 // chunk_rec records.  go (nullable, device): nothing is done unless it is set.

@@ -1121,12 +1121,12 @@ int conv_launch(Context& c, const double* pose_dev, bool grad, int i0, int i1, d
         DUGMA_CK(cudaGetLastError());
     }
     const int nv = grad ? 1 + (c.D == 3 ? 6 : 3) : 1;
-    c.timing_hold = both;
+    TimingHold hold(c, both);
     if (!sparse)
         DUGMA_RET(launch_pair_variant(c, v->fn, v->shape, c.xrec, c.yrec, (size_t)c.M_pad / v->shape.pack, nv, c.cscale,
                                       pose_dev, i0, i1, out_dev, grad ? dEdx_dev : nullptr, nullptr, 0, nullptr, s,
                                       nullptr, true, nullptr, flag));
-    c.timing_hold = false;
+    hold.release();
     if (!sparse && !both) return DUGMA_OK;
     const double cut = 2.0 + std::max(285.0, 150.0 + 0.5 * c.D * std::log2(std::max(1.0, 0.5 * c.cscale * c.inv_trace)));
     auto run = c.D == 3 ? (grad ? conv_sparse_launch<3, true> : conv_sparse_launch<3, false>)

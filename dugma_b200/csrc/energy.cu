@@ -378,12 +378,12 @@ int launch_pairs(Context& c, const double* pose_dev, int model, bool grad, int i
     const double* pose = io && io->pose_out ? io->pose_out : pose_dev;
     double* host_out = io ? io->host_out : nullptr;
     const int* flag = both ? c.counter + 4 : nullptr;
-    c.timing_hold = both;   // (one timed interval for the two pair kernels)
+    TimingHold hold(c, both);   // (one timed interval for the two pair kernels)
     if (!sparse)
         DUGMA_RET(launch_pair_variant(c, fn, shape, c.xrec, c.yrec, (size_t)c.M_pad / shape.pack, nv, c.Lmax_y, pose,
                                       i0, i1, out_dev, grad ? dEdx_dev : nullptr, nullptr, 0, nullptr, s, nullptr,
                                       true, host_out, flag));
-    c.timing_hold = false;
+    hold.release();
     if (sparse || both) {
         int jc_tiles = 0, n_jc = 0;
         pair_split(c, v->fn, v->shape, c.N, (size_t)c.M_pad / 2, &jc_tiles, &n_jc);

@@ -660,6 +660,7 @@ static int nn_run(Context& c, double* pose_dev, int k, int* idx_dev, float* d2_d
         const bool wide = nx <= 2 * c.num_sms;
         auto fn = wide ? (c.D == 3 ? prune_kernel<3, 8>(K) : prune_kernel<2, 8>(K))
                        : (c.D == 3 ? prune_kernel<3, 4>(K) : prune_kernel<2, 4>(K));
+        TimingHold hold(c, false);
         DUGMA_RET(timing_begin(c, s));
         DUGMA_CK(launch_dependent(c.pdl, fn, nx, wide ? 256 : 128, 0, s, a));
         DUGMA_RET(timing_end(c, s));
@@ -688,6 +689,7 @@ static int nn_run(Context& c, double* pose_dev, int k, int* idx_dev, float* d2_d
     }
     double* hp = nullptr;
     int n_jc = 0;
+    TimingHold hold(c, false);
     DUGMA_RET(launch_pair_variant(c, fn, sh, c.x, c.yp32, (size_t)c.M_pad / 2, 1, 0.0, pose_dev, i0, i1, nullptr,
                                   nullptr, &hp, K, &n_jc, s, nullptr, true));
     const int g = std::min((rows + 255) / 256, c.num_sms * 8);
