@@ -324,8 +324,9 @@ __global__ void __launch_bounds__(32 * NW) nn_prune_kernel(PruneArgs a)
         r[lane] = v;
         __syncwarp();
         float2 nearest = make_float2(best, best);
-        // only what can still be among the K nearest (the others' lists count too)
-        const float cut = bound * bound * (1.f + 1e-5f);
+        // only what can still be among the K nearest (the others' lists count too); an infinite distance, as
+        // NaN, is none
+        const float cut = fminf(bound * bound * (1.f + 1e-5f), 3.402823466e38f);
 #pragma unroll 4
         for (int e = 0; e < kTile / 2; ++e) {
             const float4 ra = r[2 * e], rb = r[2 * e + 1];

@@ -103,7 +103,8 @@ int dugma_energy_fd_grad(float* Ptr[6], const double* R, const double* t, double
 
 /* k (1..16) nearest targets of every source point: idx (N*k, ascending distance, ties to the
  * lowest index) and squared distances d2 (N*k FP32, exactly
- * fmaf(dz,dz, fmaf(dy,dy, dx*dx)) with y' = float(FP64(R y + t))). */
+ * fmaf(dz,dz, fmaf(dy,dy, dx*dx)) with y' = float(FP64(R y + t))).  A distance that is not finite in
+ * FP32 is no neighbour's: where fewer than k are, the rest is index 0x7fffffff at distance +inf. */
 int dugma_nn(float* Ptr[6], const double* R, const double* t, int k, int* idx, float* d2);
 
 /* Data preparation: per-point covariance from the k (1..15) nearest other points (an exact
