@@ -350,7 +350,7 @@ __global__ void __launch_bounds__(32 * NW) nn_prune_kernel(PruneArgs a)
         if constexpr (K == 0) best = fminf(nearest.x, nearest.y);
         const float kth = K == 0 ? best : __uint_as_float((unsigned)(list[KL - 1] >> 32));
         // (distances order like their bits; -1 comes first)
-        if (in) atomicMin(&s_bound[lane], __float_as_int(sqrt_fast(kth) * (1.f + 1e-6f)));
+        if (in) atomicMin(&s_bound[lane], __float_as_int(fmaxf(sqrt_fast(kth) * (1.f + 1e-6f), kLeastReach)));
         bound = __int_as_float(*(volatile int*)&s_bound[lane]);
     };
 

@@ -41,6 +41,10 @@ struct __align__(16) Bound {
     float pad[2];
 };
 
+// Squares of less than this are below the normal FP32 numbers, and sqrt_fast makes 0 of them: a bound is at
+// least this much, and a radius wider by a few.
+constexpr float kLeastReach = 1.1e-19f;
+
 // sqrt on the SFU (PTX sqrt.approx.ftz.f32, relative error 2^-23)
 __device__ __forceinline__ float sqrt_fast(float x)
 {
@@ -69,7 +73,7 @@ __device__ __forceinline__ float pose_stretch(const double* R, int D)
 }
 
 // A bound's sphere under y' = R y + t: the centre rounded to FP32, the radius stretched and widened by
-// what that rounding and the FP32 distance tests can lose.
+// what that rounding, the FP32 distance tests and squares below the normal numbers (both spheres') can lose.
 template <int D>
 __device__ __forceinline__ float4 posed_sphere(const Bound& b, const double* R, const double* t, float stretch)
 {
@@ -83,7 +87,7 @@ __device__ __forceinline__ float4 posed_sphere(const Bound& b, const double* R, 
         c[a] = __double2float_rn(v);
         size += fabsf(c[a]) + fabsf(b.c[a]) + fabsf(__double2float_rn(t[a]));
     }
-    return make_float4(c[0], c[1], c[2], fmaf(b.r, stretch, 1e-6f * size));
+    return make_float4(c[0], c[1], c[2], fmaf(b.r, stretch, fmaf(1e-6f, size, 4.f * kLeastReach)));
 }
 
 // The place of a point's grid cell along a Hilbert curve through the 2^bits cells per axis (J. Skilling,

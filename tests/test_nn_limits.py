@@ -1,5 +1,6 @@
-"""The pruned search where FP32 ends: distances that overflow, points that are not finite.  Against the
-all-pairs kernels (a pinned shape): the same bits, also the mark of a neighbour that does not exist."""
+"""The pruned search where FP32 ends: distances that overflow, points that are not finite, distances below
+the smallest normal number.  Against the all-pairs kernels (a pinned shape): the same bits, also the mark
+of a neighbour that does not exist."""
 import numpy as np
 import pytest
 
@@ -36,3 +37,11 @@ def test_infinite_distances_are_no_neighbours(far, n, m, D):
     Y[3:] += 0.5 * far        # fewer targets in reach of a distance than neighbours asked for
     X[n // 2] = far
     _same(*_pinned(X, Y, np.eye(D), np.zeros(D), (1, 5, 16)))
+
+
+@pytest.mark.parametrize("D", [2, 3])
+@pytest.mark.parametrize("scale", [1e-18, 1e-19, 1e-20, 1e-21, 3e-22, 1e-24])
+def test_distances_below_the_normal_numbers(scale, D):
+    rng = np.random.default_rng(4)
+    X, Y = scale * rng.uniform(-1, 1, (2100, D)), scale * rng.uniform(-1, 1, (3000, D))
+    _same(*_pinned(X, Y, np.eye(D), 0.1 * scale * np.ones(D), (1, 8)))
