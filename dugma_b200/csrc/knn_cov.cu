@@ -1,6 +1,6 @@
 // knn_cov.cu -- per-point covariances from the k nearest neighbours (data preparation).
 //
-// For every point p_i: the k nearest other points by the brute-force kernel of nn.cu (a
+// For every point p_i: the k nearest other points by the search of nn.cu (a
 // self-join, k + 1 neighbours with the point itself first), their sample covariance
 // together with p_i (divided by k), and an eigenvalue clamp to [lo, hi] so that every
 // covariance is positive definite with a bounded condition number.  Eigen-decomposition
@@ -53,13 +53,14 @@ __global__ void knn_cov_kernel(const double* __restrict__ pts, const int* __rest
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         double mean[3] = {0, 0, 0};
         // the point itself plus the first k other points of its k + 1 nearest (itself is among
-        // them unless more than k others coincide with it)
+        // them unless more than k others coincide with it); fewer where fewer are at a finite
+        // distance (the search marks the rest with an index past the end)
         int list[17];
         int m = 0;
         list[m++] = i;
         for (int q = 0; q < kk && m < kk; ++q) {
             const int j = idx[(size_t)i * kk + q];
-            if (j != i) list[m++] = j;
+            if (j != i && j < n) list[m++] = j;
         }
         for (int q = 0; q < m; ++q)
             for (int a = 0; a < D; ++a) mean[a] += pts[(size_t)list[q] * D + a] / m;
@@ -68,7 +69,7 @@ __global__ void knn_cov_kernel(const double* __restrict__ pts, const int* __rest
             double c[3];
             for (int a = 0; a < D; ++a) c[a] = pts[(size_t)list[q] * D + a] - mean[a];
             for (int a = 0; a < D; ++a)
-                for (int b = 0; b < D; ++b) A[a][b] += c[a] * c[b] / (m - 1);
+                for (int b = 0; b < D; ++b) A[a][b] += c[a] * c[b] / max(m - 1, 1);
         }
         jacobi_sym<D>(A, V);
         double w[3];

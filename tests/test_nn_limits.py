@@ -45,3 +45,16 @@ def test_distances_below_the_normal_numbers(scale, D):
     rng = np.random.default_rng(4)
     X, Y = scale * rng.uniform(-1, 1, (2100, D)), scale * rng.uniform(-1, 1, (3000, D))
     _same(*_pinned(X, Y, np.eye(D), 0.1 * scale * np.ones(D), (1, 8)))
+
+
+@pytest.mark.parametrize("n", [40, 3000])
+def test_covariances_of_points_without_neighbours(n):
+    """A point with no finite distance to another has no neighbours: the others' covariances are what they
+    are without it, its own is the least one, or not finite like its coordinates."""
+    rng = np.random.default_rng(5)
+    P = rng.uniform(-1, 1, (n, 3))
+    Q = np.concatenate([P, [[1e39, 0.0, 0.0], [np.nan, 0.0, 0.0], [0.0, -1e39, 1.0]]])
+    got = api.knn_covariance(Q, 8, 1e-6, 1e-2)
+    assert np.array_equal(got[:n], api.knn_covariance(P, 8, 1e-6, 1e-2))
+    for k in (n, n + 2):
+        assert np.array_equal(got[k], 1e-6 * np.eye(3))
