@@ -463,7 +463,7 @@ int dugma_init(const double* X, const double* X_C, const double* Y, const double
         {(void**)&c->pose, sizeof(double) * kPoseDoubles * 2}, {(void**)&c->out, sizeof(double) * 64},
         {(void**)&c->poses, sizeof(double) * kPoseDoubles * kMaxPoses},
         {(void**)&c->err, sizeof(int) * 4},
-        {(void**)&c->counter, sizeof(int) * (kCounters + 2 * (size_t)c->cells)},
+        {(void**)&c->counter, sizeof(int) * (kCounters + 2 * (size_t)c->cells + kReachInts)},
         {(void**)&c->init_L, sizeof(float) * ((size_t)N + M)},
         {(void**)&c->init_part, sizeof(double) * 2 * kInitParts * 5},
         {(void**)&c->init_place, sizeof(int2) * ((size_t)N + M)},

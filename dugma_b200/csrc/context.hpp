@@ -52,9 +52,14 @@ struct KernelShape {
 
 constexpr int kCounters = 8;      // ints of Context::counter
 constexpr int kInitParts = 256;   // most blocks per cloud of init's statistics
-constexpr int kInitOut = 11;      // scalars init hands to the host: log2 of the largest weights, the CONV
-                                  // scale, det <= 0 and indefinite counts, mean traces, mean squared radii, largest
-                                  // inverse trace
+constexpr int kInitOut = 8;       // scalars init hands to the host: log2 of the largest weights, the CONV
+                                  // scale, det <= 0 and indefinite counts, largest inverse trace, the targets'
+                                  // sampled pairs nearer than a grid cell
+// init's samples of how far points reach (sample_reach): points, pairs of each, octaves of q, q's exponent field
+// in the first of them (2^-44 and less)
+constexpr int kReachPoints = 1024, kReachDraws = 64, kReachBins = 128, kReachExp = 127 - 44;
+constexpr int kReachInts = 4 * kReachBins + 1;
+constexpr int kSparseUses = 5;    // values of SparseUse
 
 struct SortedPoint;
 struct Bound;
@@ -73,8 +78,9 @@ struct Context {
     int x_indef = 0;                          // weighted sources whose sym(Sigma_x^-1) is not positive definite
     int y_indef = 0;                          // weighted targets whose sym(Sigma_y^-1) is not positive definite
     double Lmax_x = 0, Lmax_y = 0;
-    double trace_x = 0, trace_y = 0;          // mean covariance trace
-    double rho2_x = 0, rho2_y = 0;            // mean squared distance to the cloud's mean
+    int reach[2][2][kReachBins] = {};         // per cloud: sums of c and of c (c - 1) (sample_reach)
+    double near_y = 0;                        // share of the targets' pairs nearer than a grid cell
+    mutable double sparse_line[kSparseUses] = {-1, -1, -1, -1, -1};   // sparse_sigma, once asked for
     float inv_trace = 0;                      // largest trace of a weighted inverse covariance
     double cscale = 1.0;                      // CONV covariances are stored divided by this
     // per-evaluation records
@@ -92,7 +98,7 @@ struct Context {
     int* err = nullptr;                       // device error word
     int* counter = nullptr;                   // work-queue counters (kCounters: [0] items,
                                               // [1] blocks done, [2, 3] sigma's integer sum, [4] the
-                                              // evaluation is sparse), then hist
+                                              // evaluation is sparse), then hist and init's reach samples
     // the clouds in spatial order (spatial.cuh), made by init
     int cell_bits = 0, cells = 0;             // grid bits per axis, cells
     int* hist = nullptr;                      // 2 x cells
@@ -207,11 +213,14 @@ struct TimingHold {
 // The REF energy or adjoint over the pairs above the FP32 flush (sparse.cu), from the records of the
 // packed kernels' prologue: the same sums as the all-pairs kernel with tiles of tile_rec and chunks of
 // chunk_rec records.  go (nullable, device): nothing is done unless it is set.
-constexpr double kSparseMinPairsAuto = 256e6, kSparseCoefMinPairs = 24e6;
+// Pairs from which a pass may be sparse where the device decides (both ways enqueued: the one that does not run
+// costs a dense EM step 2.5 us); the coefficients also where the host does, so that a call and an EM step go
+// the same way; and a batch's problems.
+constexpr double kSparseMinPairsAuto = 256e6, kSparseCoefMinPairs = 24e6, kSparseBatchMinPairs = 4e5;
 constexpr int kSparseMaxTargets = 1 << 20;
 constexpr int kRowBlocks = 256;
 int reduce_rows(Context& c, int nv, double* out_dev, cudaStream_t s, double* host_out, const int* go);
-enum class SparseUse { energy, coef, conv, batch };
+enum class SparseUse { grad, energy, conv, coef, batch };
 double sparse_sigma(const Context& c, SparseUse use);   // evaluations with a sigma below this go that way
 int sparse_launch(Context& c, const double* pose_dev, bool grad, int tile_rec, int chunk_rec, double* out_dev,
                   double* dEdx_dev, cudaStream_t s, double* host_out, const int* go);

@@ -362,8 +362,10 @@ int launch_pairs(Context& c, const double* pose_dev, int model, bool grad, int i
     // All rows by the packed kernels and a sigma that leaves most pairs under the FP32 flush: only
     // the others (sparse.cu).  Where only the device knows sigma (a pose in device memory, a captured
     // graph) both ways are enqueued and the prologue's flag lets one of them run; that costs an
-    // all-pairs evaluation two launches that return at once, so it takes kSparseMinPairsAuto pairs.
-    const double below = !force && xchol && i0 == 0 && i1 == c.N ? sparse_sigma(c, SparseUse::energy) : 0.0;
+    // all-pairs evaluation two launches that return at once, and it takes kSparseMinPairsAuto pairs (a line
+    // with much room: below it such an evaluation is over all pairs also where a host's sigma would make it sparse).
+    const SparseUse use = grad ? SparseUse::grad : SparseUse::energy;
+    const double below = !force && xchol && i0 == 0 && i1 == c.N ? sparse_sigma(c, use) : 0.0;
     const double sig = io ? (io->pv ? io->pv->v[kPoseSig] : io->sig) : 0.0;
     const bool known = sig > 0.0;
     const bool both = !known && below > 0.0 && (double)c.N * c.M >= kSparseMinPairsAuto;

@@ -20,7 +20,7 @@ namespace dugma {
 //     covariance by the adjugate, in the order of the reference's formula, rounded to FP32; det <= 0:
 //     all entries 1e5, weight 0 (init.cu:48-57, 86-100).  Also the packed FP32 covariance of the CONV
 //     model, the largest weight, the Cholesky factors, and each point's grid cell and place in it.
-//   3 cell_scan_kernel    the cells' first positions
+//   3 cell_scan_kernel    the cells' first positions; beside it, samples of how far points reach
 //   4 sort_points_kernel  log2 weights relative to the largest, and the points in cell order
 //   5 split_kernel        runs of kRun points in that order split down to tiles at medians
 //   6 bounds_kernel       bounding spheres of subgroups, tiles and super tiles; the scalars for the host
@@ -44,7 +44,9 @@ struct InitArgs {
     int nb, bits;
     int* counter;          // [0] det <= 0, [2 + cloud] largest weight (float bits), [4 + cloud] weighted
                            // points without a Cholesky factor, [6] largest trace of an inverse covariance
+    int* reach;            // per cloud [2][kReachBins] (sample_reach), then the targets' pairs nearer than a grid cell
     double *out, *host;    // kInitOut scalars for the host (host: nullable, mapped)
+    double* out_reach;     // and the samples, which go to host + 16
 };
 
 // partial sums over contiguous slices, both in fixed order (deterministic): trace, coordinates, |p|^2
@@ -268,9 +270,86 @@ __global__ void __launch_bounds__(256) init_points_kernel(InitArgs ia)
     }
 }
 
-// hist[c] <- the points in the cells before c; one block of 1024 threads per cloud
+// Samples of how far a cloud's points reach, for the choice between all pairs and the sparse passes
+// (sparse_sigma): for each of kReachPoints points, a warp each, kReachDraws pairs of it with another
+// point of its cloud, standing for a target that lies there, and with the largest variance of a point
+// of the other cloud.  A pair is in reach where |k| |d|^2 / sig is less than the exponent to the flush
+// times that variance, so q = |d|^2 / the variance is binned by octaves, and per bin the sums over the
+// points of their pairs below its end, c, and of c (c - 1) are kept: how much a point reaches on average,
+// and how unevenly.  Points and pairs are chosen by index and the sums are whole numbers: the same in every init.
+template <int D>
+__device__ __forceinline__ void sample_reach(const InitArgs& a, int cloud, int block)
+{
+    __shared__ int count[32][kReachBins];
+    __shared__ int sums[2 * kReachBins + 1];
+    __shared__ double tot[2][5];
+    const InitCloud &c = a.cl[cloud], &o = a.cl[1 - cloud];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, tid = threadIdx.x;
+    for (int b = lane; b < kReachBins; b += 32) count[warp][b] = 0;
+    if (tid < 2 * kReachBins + 1) sums[tid] = 0;
+    init_stats_total(a, tot);   // (synchronises)
+    float lo[3];
+    const float inv = cell_grid(tot[cloud], c.n, D, a.bits, lo);
+    auto mix = [](uint32_t x) {   // multiplications by odd numbers and shifts: one to one, and far from regular
+        x *= 0x9e3779b1u;
+        x ^= x >> 15;
+        x *= 0x85ebca6bu;
+        return x ^ x >> 13;
+    };
+    const uint32_t s = 32 * block + warp;
+    const int i = (int)((long long)s * c.n / kReachPoints);
+    int near = 0;
+    if (c.n > 1)
+        for (int r = 0; r < kReachDraws / 32; ++r) {
+            const uint32_t h = mix(s * kReachDraws + 32 * r + lane + 1);
+            int j = i + 1 + (int)__umulhi(h, (uint32_t)c.n - 1);
+            if (j >= c.n) j -= c.n;
+            const int k = (int)__umulhi(mix(h ^ 0x5bd1e995u), (uint32_t)o.n);
+            float d2 = 0.f;
+#pragma unroll
+            for (int q = 0; q < D; ++q) {
+                const float d = c.p32[(size_t)i * D + q] - c.p32[(size_t)j * D + q];
+                d2 = d2 + d * d;
+            }
+            near += d2 * inv * inv < 1.f;
+            if (!(c.w[i] > 0.f && o.w[k] > 0.f)) continue;   // (without weight: reaches nothing)
+            const int e = (int)(__float_as_uint(d2 / fmaxf(c.L[i], o.L[k])) >> 23);
+            atomicAdd(&count[warp][min(max(e - kReachExp, 0), kReachBins - 1)], 1);
+        }
+    near = (int)__reduce_add_sync(0xffffffffu, (unsigned)near);
+    __syncwarp();
+    int v[kReachBins / 32], sum = 0;   // this lane's bins, and the bins before them
+#pragma unroll
+    for (int b = 0; b < kReachBins / 32; ++b) sum += v[b] = count[warp][kReachBins / 32 * lane + b];
+    int below = sum;
+#pragma unroll
+    for (int w = 1; w < 32; w <<= 1) {
+        const int u = __shfl_up_sync(0xffffffffu, below, w);
+        if (lane >= w) below += u;
+    }
+    below -= sum;
+#pragma unroll
+    for (int b = 0; b < kReachBins / 32; ++b) {
+        below += v[b];
+        if (below == 0) continue;
+        atomicAdd(&sums[kReachBins / 32 * lane + b], below);
+        atomicAdd(&sums[kReachBins + kReachBins / 32 * lane + b], below * (below - 1));
+    }
+    if (lane == 0) atomicAdd(&sums[2 * kReachBins], near);
+    __syncthreads();
+    if (tid < 2 * kReachBins && sums[tid]) atomicAdd(a.reach + 2 * kReachBins * cloud + tid, sums[tid]);
+    if (tid == 2 * kReachBins && cloud == 1 && sums[tid]) atomicAdd(a.reach + 4 * kReachBins, sums[tid]);
+}
+
+// hist[c] <- the points in the cells before c; one block of 1024 threads per cloud.  The blocks behind
+// them sample the reach, on SMs that the scan leaves idle.
+template <int D>
 __global__ void __launch_bounds__(1024) cell_scan_kernel(InitArgs a, int cells)
 {
+    if (blockIdx.x >= 2) {
+        sample_reach<D>(a, blockIdx.x & 1, (int)blockIdx.x / 2 - 1);
+        return;
+    }
     int* __restrict__ hist = a.cl[blockIdx.x].hist;
     __shared__ int sums[32];
     __shared__ int carry;
@@ -520,15 +599,17 @@ __global__ void __launch_bounds__(1024) bounds_kernel(InitArgs ia)
                 v = conv_scale(ia, tot, D);
             } else if (q < 6) {
                 v = (double)ia.counter[q == 3 ? 0 : q];
-            } else if (q < 8) {
-                v = tot[q - 6][0] / ia.cl[q - 6].n;   // mean covariance trace
-            } else if (q < 10) {
-                v = mean_radius2(tot[q - 8], ia.cl[q - 8].n, D);
-            } else {
+            } else if (q == 6) {
                 v = (double)__int_as_float(ia.counter[6]);
+            } else {
+                v = (double)ia.reach[4 * kReachBins];
             }
             ia.out[q] = v;
             if (ia.host) ia.host[q] = v;
+        }
+        for (int q = threadIdx.x; q < 4 * kReachBins; q += blockDim.x) {
+            ia.out_reach[q] = (double)ia.reach[q];
+            if (ia.host) ia.host[16 + q] = (double)ia.reach[q];
         }
     }
 }
@@ -553,8 +634,8 @@ int launch_init(Context& c, const double* X, const double* XC, const double* Y, 
     ck(cudaMemcpyAsync(tXC, XC, sizeof(double) * nd * D, cudaMemcpyHostToDevice, s), "copy X_C");
     ck(cudaMemcpyAsync(tY, Y, sizeof(double) * md, cudaMemcpyHostToDevice, s), "copy Y");
     ck(cudaMemcpyAsync(tYC, YC, sizeof(double) * md * D, cudaMemcpyHostToDevice, s), "copy Y_C");
-    // the work counters and, behind them, the cell histograms
-    ck(cudaMemsetAsync(c.counter, 0, sizeof(int) * (kCounters + 2 * (size_t)c.cells), s), "memset");
+    // the work counters and, behind them, the cell histograms and the samples of the reach
+    ck(cudaMemsetAsync(c.counter, 0, sizeof(int) * (kCounters + 2 * (size_t)c.cells + kReachInts), s), "memset");
     InitArgs a{};
     a.cl[0] = {tX, tXC, N, c.x, c.xinv, c.wx, c.xcov, c.lwx, c.ux, c.init_L, c.init_place, c.hist,
                c.xpt, c.xtile, c.xsub, c.xsuper};
@@ -565,8 +646,11 @@ int launch_init(Context& c, const double* X, const double* XC, const double* Y, 
     a.nb = std::min(kInitParts, std::max(1, (n + 255) / 256));
     a.bits = c.cell_bits;
     a.counter = c.counter;
+    a.reach = c.hist + 2 * (size_t)c.cells;
     a.out = c.out;
     a.host = c.host_dev;
+    static_assert(4 * kReachBins <= kMomSlots && 16 + 4 * kReachBins <= kHostDoubles, "staging of the samples");
+    a.out_reach = c.mom;
     const dim3 g(std::min((n + 255) / 256, c.num_sms * 8), 2);
     const dim3 gs((n + kTile * kSuper - 1) / (kTile * kSuper), 2);
     init_stats_kernel<<<dim3(a.nb, 2), 256, 0, s>>>(a, D);
@@ -574,18 +658,23 @@ int launch_init(Context& c, const double* X, const double* XC, const double* Y, 
         init_points_kernel<3><<<g, 256, 0, s>>>(a);
     else
         init_points_kernel<2><<<g, 256, 0, s>>>(a);
-    cell_scan_kernel<<<2, 1024, 0, s>>>(a, c.cells);
+    const int scan_blocks = 2 + 2 * kReachPoints / 32;
     if (D == 3) {
+        cell_scan_kernel<3><<<scan_blocks, 1024, 0, s>>>(a, c.cells);
         sort_points_kernel<3><<<g, 256, 0, s>>>(a);
         split_kernel<3><<<dim3((n + kRun - 1) / kRun, 2), kRun, 0, s>>>(a);
         bounds_kernel<3><<<gs, kTile * kSuper, 0, s>>>(a);
     } else {
+        cell_scan_kernel<2><<<scan_blocks, 1024, 0, s>>>(a, c.cells);
         sort_points_kernel<2><<<g, 256, 0, s>>>(a);
         split_kernel<2><<<dim3((n + kRun - 1) / kRun, 2), kRun, 0, s>>>(a);
         bounds_kernel<2><<<gs, kTile * kSuper, 0, s>>>(a);
     }
     ck(cudaGetLastError(), "init kernels");
-    if (!c.host_dev) ck(cudaMemcpyAsync(c.host, c.out, kInitOut * sizeof(double), cudaMemcpyDeviceToHost, s), "copy back");
+    if (!c.host_dev) {
+        ck(cudaMemcpyAsync(c.host, c.out, kInitOut * sizeof(double), cudaMemcpyDeviceToHost, s), "copy back");
+        ck(cudaMemcpyAsync(c.host + 16, c.mom, 4 * kReachBins * sizeof(double), cudaMemcpyDeviceToHost, s), "copy back");
+    }
     ck(cudaStreamSynchronize(s), "sync");
     if (rc != DUGMA_OK) return rc;
     c.Lmax_x = std::isfinite(c.host[0]) ? c.host[0] : 0.0;
@@ -594,11 +683,9 @@ int launch_init(Context& c, const double* X, const double* XC, const double* Y, 
     c.nonpd = (int)c.host[3];
     c.x_indef = c.ux ? (int)c.host[4] : N;
     c.y_indef = (int)c.host[5];
-    c.trace_x = c.host[6];
-    c.trace_y = c.host[7];
-    c.rho2_x = c.host[8];
-    c.rho2_y = c.host[9];
-    c.inv_trace = (float)c.host[10];
+    c.inv_trace = (float)c.host[6];
+    c.near_y = c.host[7] / (kReachPoints * kReachDraws);
+    for (int q = 0; q < 4 * kReachBins; ++q) (&c.reach[0][0][0])[q] = (int)c.host[16 + q];
     return DUGMA_OK;
 }
 

@@ -100,35 +100,109 @@ int reduce_rows(Context& c, int nv, double* out_dev, cudaStream_t s, double* hos
     return DUGMA_OK;
 }
 
-// Which of a context's evaluations go this way: those with a sigma below this (0: none).  With f the share
-// of a surface that a pair of mean variance v reaches, f = 127.5 sig v / (4 |k| r^2) for clouds of radius
-// r (r^2: mean squared distance to the mean, of the smaller one), an evaluation is sparse where f is
-// under `most`, a line drawn from timings of both ways at 1000 - 32000 points on six kinds of cloud, f
-// from 5e-4 to 0.2 (one B200, us a call, all pairs / sparse; the outliers' clouds, whose variances differ
-// most, cross first):
-//   energy_grad 3000: 46 / 47-52 at any f;  4500: 91 / 52-82 at 6e-3, 91 / 69-145 at 0.02;  16000:
-//     487 / 94-304 at 6e-3, 487 / 146-611 at 0.02;  32000: 1608 / 162-736, 1608 / 319-1740
-//   compi 4500: 96 / 68-83 at 2e-3, 96 / 77-106 at 6e-3;  6500: 141 / 104-140 at 6e-3;  16000: 622 /
-//     154-432 at 6e-3, 622 / 246-877 at 0.02
-//   CONV 4500: 121 / 83-96 at 5e-4;  6500: 171 / 121-145 at 2e-3;  16000: 762 / 198-427 at 2e-3,
-//     762 / 281-828 at 6e-3
-//   batches, many problems at once: 700 points 246 / 162-213 at 6e-3, 246 / 192-267 at 0.02;  1000: 417 /
-//     264-362 at 0.02, 417 / 340-552 at 0.06;  8000: 837 / 276-561 at 0.02
+// Which of a context's evaluations go this way: those with a sigma below a line (0: none) where the
+// modelled times of both ways meet.  All pairs: t0 + tp N M + tn (N + M).  The sparse pass, with f the
+// share of pairs in reach at that sigma (init's samples, sample_reach) and g the same of the points that
+// reach more (weighted by what they reach):
+//   s0 + sn (N + M) + |(a N C(f), b C(g))|,     C(f) = M (F + y G)
+//   F = min(1, u f, (f^(1/e) + (32/N)^(1/e))^e)                     records that one tile of 32 sources marks
+//   G = min(1, x (f^(1/e) + (32/N)^(1/e) + (32/M)^(1/e))^e)         tiles that it searches
+// a N C: all blocks at the GPU's rate; b C: one block alone, which is what few sources and uneven densities
+// come down to.  The coefficients search from both sides.  A batch's problems fill the GPU together: only
+// the terms in N and M count.
+// The constants are fits to calls timed both ways on one B200 (us): 12 kinds of cloud (surfaces, volumes,
+// curves, discs, outliers, points at one place, clusters of 1 % of the radius), 1000 - 64000 points, and 64
+// - 4000 against 20000 - 600000 either way round, f from 1e-4 to 0.35; batches of 8 and 192 evaluations,
+// 250 - 8000 points.  Of 2562 cases a use, slower than all pairs by more than 10 % with these lines: at most
+// gradient 40 (worst 1.6 times), energy 54 (2.5), CONV 29 (1.7), compi 41 (1.7), batch 13 of 702 (1.4),
+// nearly all of them clusters; by the mean variance over the mean squared radius alone, which knows neither of clusters nor
+// of few sources, 360 - 470 of 1575 (worst 92 times).
+struct SparseCost {
+    double t0, tp, tn;                        // all pairs
+    double s0, sn, a, b, y, x, u, e;          // the sparse pass
+    double margin;                            // sparse where its time is below this share of all pairs'
+};
+static const SparseCost& sparse_cost(SparseUse use, int D)
+{
+    static const SparseCost cost[kSparseUses][2] = {
+        {{31.2, 9.73e-7, 9.6e-5, 29.1, 3.6e-4, 2.32e-6, 0.0187, 0.0904, 5.01, 6.09, 2.0, 0.95},
+         {31.2, 1.59e-6, 9.6e-5, 30.0, 4.46e-4, 3.28e-6, 0.0186, 0.134, 3.33, 10.9, 3.0, 0.95}},
+        {{25.9, 5.83e-7, 1.48e-4, 28.6, 3.05e-4, 2.07e-6, 0.0173, 0.0871, 4.9, 4.48, 1.76, 1.0},
+         {25.9, 9.12e-7, 1.48e-4, 31.7, 3.63e-4, 2.96e-6, 0.0193, 0.0905, 3.44, 8.44, 3.0, 1.0}},
+        {{50.7, 1.54e-6, 1.64e-4, 50.2, 2.27e-4, 3.92e-6, 0.0245, 0.419, 1.95, 11.6, 2.71, 0.95},
+         {50.7, 2.75e-6, 1.64e-4, 54.6, 2.93e-4, 5.78e-6, 0.029, 0.526, 3.09, 11.1, 3.0, 0.95}},
+        {{43.2, 1.03e-6, 1.93e-3, 32.4, 1.06e-3, 1.5e-6, 0.0215, 0.129, 2.1, 9.37, 3.0, 0.9},
+         {43.2, 1.83e-6, 1.93e-3, 33.9, 2.03e-3, 3.36e-6, 0.0377, 0.0904, 3.41, 7.96, 3.0, 0.9}},
+        {{0, 7.76e-7, 1.54e-4, 0, 5.12e-5, 8.85e-7, 0, 2.0, 1.0, 1.0, 1.61, 0.85},
+         {0, 1.45e-6, 1.54e-4, 0, 3.53e-5, 3.19e-6, 0, 0.483, 2.36, 3.95, 1.88, 0.85}},
+    };
+    return cost[(int)use][D == 3];
+}
+
+// f and g where q < 2^x is in reach; the sampled sums are interpolated between octaves as powers of q
+static void reach_shares(const Context& c, double x, double* f, double* g)
+{
+    const double u = std::min(std::max(x + (127 - kReachExp) - 1.0, 0.0), kReachBins - 2.0);   // (bin b ends at 2^(b - 43))
+    const int b = (int)u;
+    double share[2], uneven = 0.0;
+    for (int k = 0; k < 2; ++k) {
+        double at[2], two[2];
+        for (int q = 0; q < 2; ++q) {
+            const int n = c.reach[k][0][b + q];
+            at[q] = std::log((n + 0.25) / (kReachPoints * kReachDraws));
+            two[q] = n > 0 ? c.reach[k][1][b + q] / ((kReachDraws - 1.0) * n) : 0.0;
+        }
+        share[k] = std::exp(at[0] + (u - b) * (at[1] - at[0]));
+        uneven = std::max(uneven, two[0] + (u - b) * (two[1] - two[0]));
+    }
+    *f = std::sqrt(share[0] * share[1]);   // (pairs of two clouds: at most this, by Cauchy-Schwarz)
+    *g = std::max(uneven, *f);
+}
+
+static double sparse_time(const SparseCost& t, SparseUse use, double f, double g, double N, double M)
+{
+    auto block = [&](double h, double n, double m) {   // C(h)
+        const double r = 1.0 / t.e, p = std::pow(h, r), pn = std::pow(std::min(1.0, 32.0 / n), r),
+                     pm = std::pow(std::min(1.0, 32.0 / m), r);
+        const double F = std::min({1.0, t.u * h, std::pow(p + pn, t.e)});
+        const double G = std::min(1.0, t.x * std::pow(p + pn + pm, t.e));
+        return m * (F + t.y * G);
+    };
+    double all = N * block(f, N, M), one = t.b > 0 ? block(g, N, M) : 0.0;
+    if (use == SparseUse::coef) {
+        all += M * block(f, M, N);
+        one = std::max(one, block(g, M, N));
+    }
+    return t.s0 + t.sn * (N + M) + std::hypot(t.a * all, t.b * one);
+}
+
 double sparse_sigma(const Context& c, SparseUse use)
 {
     if (c.x_indef > 0 || c.y_indef > 0 || !c.ux || !c.xpt || c.no_alloc || c.all_pairs || c.M > kSparseMaxTargets)
         return 0.0;
-    const double pairs = (double)c.N * c.M, grow = std::pow(std::max(1.0, pairs / 4e7), 1.0 / 6);
-    double most = 0.0;
-    switch (use) {
-    case SparseUse::energy: most = pairs < 12e6 ? 0.0 : (pairs < 2e7 ? 2e-3 : 6e-3 * grow); break;
-    case SparseUse::coef: most = pairs < kSparseCoefMinPairs || c.N > kSparseMaxTargets ? 0.0 : (pairs < 4e7 ? 2e-3 : 6e-3 * grow); break;
-    case SparseUse::conv: most = pairs < 2e7 ? 0.0 : (pairs < 4e7 ? 5e-4 : 2e-3 * grow); break;
-    case SparseUse::batch: most = pairs < 4e5 ? 0.0 : (pairs < 1e6 ? 6e-3 : 2e-2); break;
+    const double N = c.N, M = c.M;
+    if (use == SparseUse::coef && (N * M < kSparseCoefMinPairs || c.N > kSparseMaxTargets)) return 0.0;
+    if (use == SparseUse::batch && N * M < kSparseBatchMinPairs) return 0.0;
+    double& line = c.sparse_line[(int)use];
+    if (line >= 0) return line;
+    const SparseCost& t = sparse_cost(use, c.D);
+    const double limit = t.margin * (t.t0 + t.tp * N * M + t.tn * (N + M));
+    auto sparse_at = [&](double x) {
+        double f, g;
+        reach_shares(c, x, &f, &g);
+        return sparse_time(t, use, f, g, N, M) < limit;
+    };
+    double lo = kReachExp - 127 + 1.0, hi = lo + kReachBins - 2.0;   // log2 of q; the time grows with it
+    if (!sparse_at(lo)) return line = 0.0;
+    if (sparse_at(hi)) {
+        lo = hi;
+    } else {
+        for (int k = 0; k < 18; ++k) {
+            const double x = 0.5 * (lo + hi);
+            (sparse_at(x) ? lo : hi) = x;
+        }
     }
-    const double v = (c.trace_x + c.trace_y) / (2.0 * c.D), r2 = std::min(c.rho2_x, c.rho2_y);
-    const double s = most * 4.0 * r2 * -K_EXP2 / ((double)kFlushExp * v);
-    return s > 0 && std::isfinite(s) ? s : 0.0;
+    return line = std::exp2(lo) * -K_EXP2 / (double)kFlushExp;   // q < 127.5 sig / |k|
 }
 
 template <int D, bool GRAD>

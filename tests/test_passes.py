@@ -46,7 +46,7 @@ SPARSE = [(ENERGY, 6001, 5100), (ENERGY, 20001, 4001), (CONV, 7001, 6301), (CONV
 
 @pytest.mark.filterwarnings("ignore")
 @pytest.mark.parametrize("calls,n,m", SPARSE)
-@pytest.mark.parametrize("kind", ["sphere", "outliers", "harmonic", "curve", "coincident"])
+@pytest.mark.parametrize("kind", ["sphere", "outliers", "harmonic", "curve"])
 def test_sparse_pass_is_taken(kind, calls, n, m, monkeypatch):
     prob = _problem(kind, n, m, 3)
     R, t = prob[4], prob[5] + 0.01
@@ -123,7 +123,7 @@ def test_conv_of_needles(n, m, monkeypatch):
     """A pair that fails the FP32 path's test is evaluated in FP64; what the FP32 path made of it has no
     say in which term is the largest, whether or not the pass comes upon that pair."""
     prob = _needles(n, m, 5)
-    for sig in (3e-3, 8e-3):
+    for sig in (5e-5, 1e-4, 2e-4):
         a = _run(monkeypatch, CONV, prob, prob[4], prob[5] + 1e-3, sig, False)
         b = _run(monkeypatch, CONV, prob, prob[4], prob[5] + 1e-3, sig, True)
         for name in b:
