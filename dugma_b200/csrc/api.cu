@@ -707,11 +707,12 @@ int dugma_nn(float* Ptr[6], const double* R, const double* t, int k, int* idx, f
     GET_CTX(c, Ptr);
     if (k < 1 || k > 16 || k > c->M) return set_error(DUGMA_ERR_ARG, "nn: k = %d must be in [1, min(16, M)]", k);
     DUGMA_RET(upload_pose(*c, R, t, 1.0));
-    // results in the scratch, which the pruned search leaves alone (a pinned all-pairs shape keeps its
-    // lists there: then a buffer that stays with the context); allocating them per call took longer
-    // than the search
+    // results in the scratch, which the pruned search leaves alone (the all-pairs search keeps its lists
+    // there: then a buffer that stays with the context); allocating them per call took longer than the
+    // search
+    const bool pruned = nn_pruned(*c, k);
     const size_t n = (size_t)c->N * k, bytes = (sizeof(int) + sizeof(float)) * n;
-    if (c->nn_pinned && n > c->nn_slots) {
+    if (!pruned && n > c->nn_slots) {
         if (c->nn_out) cudaFree(c->nn_out);
         c->nn_out = nullptr;
         c->nn_slots = 0;
@@ -721,10 +722,10 @@ int dugma_nn(float* Ptr[6], const double* R, const double* t, int k, int* idx, f
             return set_error(DUGMA_ERR_NOMEM, "nn: cannot allocate %zu bytes", bytes);
         }
         c->nn_slots = n;
-    } else if (!c->nn_pinned) {
+    } else if (pruned) {
         DUGMA_RET(c->ensure_scratch(bytes));
     }
-    int* di = static_cast<int*>(c->nn_pinned ? c->nn_out : (void*)c->scratch);
+    int* di = static_cast<int*>(pruned ? (void*)c->scratch : c->nn_out);
     float* dd = reinterpret_cast<float*>(di + n);
     DUGMA_RET(launch_nn(*c, c->pose, k, di, dd, c->stream));
     DUGMA_CK(cudaMemcpyAsync(idx, di, sizeof(int) * n, cudaMemcpyDeviceToHost, c->stream));

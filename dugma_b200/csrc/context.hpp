@@ -116,7 +116,7 @@ struct Context {
     int last_search = 0;                      // nearest neighbours: 0 all pairs, 1 pruned
     bool nn_pinned = false;                   // a nearest-neighbour kernel shape was pinned: no pruning
     double* dedx = nullptr;                   // dE/dx rows (allocated on first request)
-    void* nn_out = nullptr;                   // dugma_nn's results under a pinned shape (on request)
+    void* nn_out = nullptr;                   // dugma_nn's results of an all-pairs search (on request)
     size_t nn_slots = 0;                      // its (index, distance) pairs
     double* mom = nullptr;                    // surrogate moments (512 doubles)
     double* mom_part = nullptr;               // per-block moment partials (with the 128-byte records)
@@ -264,6 +264,8 @@ int ref64_launch(Context& c, const double* pose_dev, int i0, int i1, double* out
 // Nearest neighbours: writes idx/d2 (device) and optionally the per-point minimum only.
 int launch_nn(Context& c, double* pose_dev, int k, int* idx_dev, float* d2_dev, cudaStream_t s,
               const KernelShape* force = nullptr);
+// Whether a search for k neighbours is the pruned one (all rows: rows < 0), which leaves c.scratch alone.
+bool nn_pruned(const Context& c, int k, const KernelShape* force = nullptr, int rows = -1);
 // Options of a sigma evaluation, for a call that issues no copy or memset:
 struct SigmaOpts {
     const PoseBlock* pose_value = nullptr;   // the pose by value to the first kernel (which also writes

@@ -8,8 +8,8 @@
 // Target records hold two targets each, coordinates negated (d = x + (-y') is the same FP32
 // value), interleaved so that the search kernels evaluate both with f32x2 operations.
 //   the k smallest (d2, j) in lexicographic order are kept in registers (ties -> lowest j)
-// All rows: the pruned search in spatial order (nn_prune_kernel).  Row ranges and pinned shapes: all
-// pairs, the targets streamed by bulk copy like the energy kernels and target chunks merged in
+// All rows: the pruned search in spatial order (nn_prune_kernel).  Row ranges, pinned shapes and very uneven
+// sizes (nn_pruned): all pairs, the targets streamed by bulk copy like the energy kernels and target chunks merged in
 // index order afterwards.  Either is exact and deterministic.  sigma is then
 //   exact:      sum_i d2min_i / (D N) in FP64
 //   quantised:  sum_i rn_u32(fl32(d2min_i / D) * 1e6) / 1e6 / N   (the reference's value)
@@ -623,18 +623,29 @@ static void (*prune_kernel(int K))(PruneArgs)
                             : (K == 8 ? nn_prune_kernel<D, 8, NW> : nn_prune_kernel<D, 16, NW>));
 }
 
-static bool nn_pruned(const Context& c, const KernelShape* force, int rows)
+// The pruned search takes all rows, but for one neighbour where its blocks are too few to fill the GPU while each
+// has a long chain of spheres and tiles (few sources), or where there is too little to prune for one block per 32
+// sources to pay (few targets).  update_sig on one B200, us a call, all pairs / pruned, points of a surface:
+//   targets  20000:  32 sources 49 / 60, 128 36 / 46, 512 38 / 32;   65000: 128 52 / 66, 512 53 / 43
+//            200000: 128 77 / 128, 512 80 / 73;   600000: 128 143 / 406, 512 146 / 214, 1000 203 / 176
+//   sources  200000: 32 targets 36 / 39, 128 38 / 42, 512 57 / 43;   600000: 32 54 / 66, 128 51 / 75, 512 103 / 77
+// Targets of which a quarter of the pairs share a grid cell are in a poor order, and few sources find their
+// tiles late: a cluster with 95 % of the points, 65000 targets: 1000 sources 60 / 98, 4000 96 / 80;  600000: 1000 205 / 836,
+// 2000 330 / 769, 4000 570 / 585.
+// With 8 neighbours the pruned search is the faster one at these sizes too (600000 targets: 2.8-14 times).
+bool nn_pruned(const Context& c, int k, const KernelShape* force, int rows)
 {
-    return !force && !c.nn_pinned && rows == c.N;
+    if (force || c.nn_pinned || (rows >= 0 && rows != c.N)) return false;
+    const bool few = c.N <= 256 || c.M / 800 >= c.N || (c.near_y > 0.25 && c.N < 4000);
+    return k > 1 || !((c.M >= 16384 && few) || (c.M <= 256 && c.N >= 262144));
 }
 
 // Runs the search; dmin_dev (nullable) receives the nearest squared distance per source.
 // Source rows [i0, i1) (i1 < 0: all); idx/d2 rows are relative to i0, dmin is indexed absolutely.
 // The search: the targets' search records (the nearest-neighbour prologue, which also zeroes the
 // work counters, and the error word when reset_err; the pose by value when pv, or read from
-// pose_src), then over all rows the pruned search in spatial order, and for a row range, or when a
-// kernel shape is asked for (force, nn_pinned), the all-pairs kernel and the merge of its per-chunk
-// lists.  quant: the pruned search also sums the quantised sigma (SigmaOpts) into out_dev[1].
+// pose_src), then the pruned search in spatial order or (nn_pruned) the all-pairs kernel and the
+// merge of its per-chunk lists.  quant: the pruned search also sums the quantised sigma (SigmaOpts) into out_dev[1].
 static int nn_run(Context& c, double* pose_dev, int k, int* idx_dev, float* d2_dev, float* dmin_dev,
                   cudaStream_t s, const KernelShape* force, int i0 = 0, int i1 = -1, const PoseBlock* pv = nullptr,
                   const double* pose_src = nullptr, bool reset_err = false, const SigmaOpts* quant = nullptr,
@@ -646,7 +657,7 @@ static int nn_run(Context& c, double* pose_dev, int k, int* idx_dev, float* d2_d
         DUGMA_RET(launch_pose_in(c, pose_src, pose_dev, s, reset_err));
         reset_err = false;
     }
-    const bool pruned = nn_pruned(c, force, rows);
+    const bool pruned = nn_pruned(c, k, force, rows);
     c.last_search = pruned;
     DUGMA_RET(launch_nn_prologue(c, pose_dev, s, pv, c.counter, reset_err ? c.err : nullptr, pruned));
     if (pruned) {
@@ -717,7 +728,7 @@ int launch_sigma(Context& c, double* pose_dev, double* out_dev, cudaStream_t s, 
     const bool whole = i1 < 0;
     if (whole) i1 = c.N;
     const int rows = i1 - i0;
-    const bool quant = !o.exact && whole && nn_pruned(c, nullptr, rows);
+    const bool quant = !o.exact && whole && nn_pruned(c, 1);
     DUGMA_RET(nn_run(c, pose_dev, 1, nullptr, nullptr, c.dmin, s, nullptr, i0, i1, o.pose_value, o.pose_src,
                      o.reset_err, quant ? &o : nullptr, out_dev));
     if (quant) return DUGMA_OK;

@@ -1,5 +1,6 @@
-"""Very uneven sizes and clouds with most points in one place: the way of an evaluation follows from how far the
-points reach, not from the clouds' mean variance and radius."""
+"""Very uneven sizes and clouds with most points in one place: what a rule made for even surfaces sends the
+slow way.  The searches give the bits of all pairs whichever way they go; the way of an evaluation follows
+from how far the points reach, not from the clouds' mean variance and radius."""
 import numpy as np
 import pytest
 
@@ -12,6 +13,33 @@ pytestmark = pytest.mark.gpu
 def _cluster(P, share, radius, rng):
     k = int(share * len(P))
     P[:k] = P[0] + radius * rng.standard_normal((k, P.shape[1]))
+
+
+@pytest.mark.parametrize("cluster", [False, True])
+@pytest.mark.parametrize("n,m,pruned", [(32, 16383, (1, 1)), (32, 16384, (0, 0)), (257, 20000, (1, 0)), (300, 240000, (0, 0)),
+                                        (3999, 16384, (1, 0)), (4000, 16384, (1, 1)), (262144, 256, (0, 0)),
+                                        (262144, 257, (1, 1))])
+def test_search_of_uneven_clouds(n, m, pruned, cluster):
+    rng = np.random.default_rng(n + m)
+    X, Y = rng.uniform(-1, 1, (n, 3)), rng.uniform(-1, 1, (m, 3))
+    if cluster:
+        _cluster(X, 0.9, 0.003, rng)
+        _cluster(Y, 0.9, 0.003, rng)
+    eye = lambda k: np.broadcast_to(np.eye(3), (k, 3, 3))  # noqa: E731
+    R, t = np.eye(3), np.array([0.01, -0.02, 0.0])
+    _, h = api.init(X, eye(n), Y, eye(m))
+    got = [api.update_sig(h, R, t), api.sigma(h, R, t)]
+    assert api.last_pass(h)[2] == pruned[cluster]
+    got += list(api.nn(h, R, t, 1))
+    assert api.last_pass(h)[2] == pruned[cluster]
+    got += list(api.nn(h, R, t, 5))
+    assert api.last_pass(h)[2] == 1
+    got.append(api.update_sig(h, R, t))
+    api.set_shape(h, 2, api.shapes(2)[0])
+    want = [api.update_sig(h, R, t), api.sigma(h, R, t), *api.nn(h, R, t, 1), *api.nn(h, R, t, 5), api.update_sig(h, R, t)]
+    assert api.last_pass(h)[2] == 0
+    assert all(np.array_equal(u, v) for u, v in zip(got, want))
+    api.fr_m(h)
 
 
 @pytest.mark.parametrize("call", ["grad", "energy", "conv", "compi"])
