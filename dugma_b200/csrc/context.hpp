@@ -167,9 +167,11 @@ const char* last_error();
 #define DUGMA_CK(call)                                                                    \
     do {                                                                                  \
         cudaError_t e_ = (call);                                                          \
-        if (e_ != cudaSuccess)                                                            \
+        if (e_ != cudaSuccess) {                                                          \
+            cudaGetLastError(); /* or the next check of a launch would report it again */ \
             return ::dugma::set_error(DUGMA_ERR_CUDA, "%s failed: %s (%s:%d)", #call,     \
                                       cudaGetErrorString(e_), __FILE__, __LINE__);        \
+        }                                                                                 \
     } while (0)
 
 #define DUGMA_RET(call)           \
