@@ -196,12 +196,14 @@ __global__ void __launch_bounds__(256) init_points_kernel(InitArgs ia)
         }
         float o[D * D];
         float wi;
+        bool valid;   // det > 0
         if (D == 3) {
             const double a11 = a_[0], a21 = a_[1], a31 = a_[2], a12 = a_[3], a22 = a_[4], a32 = a_[5],
                          a13 = a_[6], a23 = a_[7], a33 = a_[8];
             const double d = a11 * a22 * a33 - a11 * a23 * a32 - a12 * a21 * a33 + a12 * a23 * a31 +
                              a13 * a21 * a32 - a13 * a22 * a31;
-            if (d > 0) {
+            valid = d > 0;
+            if (valid) {
                 o[0] = __double2float_rn((a22 * a33 - a23 * a32) / d);
                 o[1] = __double2float_rn(-(a21 * a33 - a23 * a31) / d);
                 o[2] = __double2float_rn((a21 * a32 - a22 * a31) / d);
@@ -221,7 +223,8 @@ __global__ void __launch_bounds__(256) init_points_kernel(InitArgs ia)
         } else {
             const double a1 = a_[0], a2 = a_[1], a3 = a_[2], a4 = a_[3];
             const double d = a1 * a4 - a2 * a3;
-            if (d > 0) {
+            valid = d > 0;
+            if (valid) {
                 o[0] = __double2float_rn(a4 / d);
                 o[1] = __double2float_rn(-a2 / d);
                 o[2] = __double2float_rn(-a3 / d);
@@ -256,7 +259,8 @@ __global__ void __launch_bounds__(256) init_points_kernel(InitArgs ia)
         if (cl.ufac)
 #pragma unroll
             for (int k = 0; k < NS; ++k) cl.ufac[(size_t)i * NS + k] = wi > 0.0f ? u[k] : 0.0;
-        cl.L[i] = wi > 0.0f ? (ok ? variance_bound<D>(pk) : INFINITY) : 0.f;
+        // (a weight that is 0 in FP32 beside a positive determinant: no bound; the CONV model has such points' pairs)
+        cl.L[i] = wi > 0.0f ? (ok ? variance_bound<D>(pk) : INFINITY) : (valid ? INFINITY : 0.f);
         const int code = cell_code<D>(pf, lo, inv, ia.bits);
         cl.place[i] = make_int2(code, atomicAdd(cl.hist + code, 1));
     }

@@ -24,7 +24,8 @@ constexpr float kFlushExp = 127.5f;
 
 // A point in spatial order: coordinates, a = the exponent it can lose before the flush (kFlushExp +
 // log2 of its relative weight), L = a bound on 1 / (smallest eigenvalue of sym(Sigma^-1)) (the
-// largest variance; +inf when that matrix is not positive definite), and its index in the cloud.
+// largest variance; +inf when that matrix is not positive definite, or the weight 0 beside a positive
+// determinant; 0 when the point is neglected), and its index in the cloud.
 struct __align__(16) SortedPoint {
     float p[3];
     float a;

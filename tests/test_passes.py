@@ -129,3 +129,15 @@ def test_conv_of_needles(n, m, monkeypatch):
         for name in b:
             assert (a[name][0], b[name][0]) == (1, 0), (name, a[name][0])
             _same(a[name][1], b[name][1], name)
+
+
+def test_conv_with_a_boundless_covariance(monkeypatch):
+    """A covariance so large that its weight is 0 in FP32 (but its determinant positive): the CONV model still
+    has its pairs, and the sparse pass does not take it for a point without variance."""
+    X, XC, Y, YC, R, t = _problem("harmonic", 7001, 6301, 3)
+    XC[5] = YC[9] = 1e31 * np.eye(3)
+    a = _run(monkeypatch, CONV, (X, XC, Y, YC), R, t + 0.01, 1e-5, False)
+    b = _run(monkeypatch, CONV, (X, XC, Y, YC), R, t + 0.01, 1e-5, True)
+    for name in b:
+        assert (a[name][0], b[name][0]) == (1, 0) and b[name][1][0] > 0, (name, a[name][0], b[name][1][0])
+        _same(a[name][1], b[name][1], name)
