@@ -19,12 +19,12 @@ OUT = os.path.join(HERE, "_ref")
 # the reference tree: DUGMA_REFERENCE, else where this build environment mounts it (the one place
 # the path is named); absent on machines that only run the prebuilt objects
 REF = os.environ.get("DUGMA_REFERENCE", "/root/reference")
+PLUGINS = ("init", "update_sig", "compi")
 
 
 def reference_tree() -> str | None:
-    """The reference tree if it is present on this machine, else None."""
-    return REF if os.path.isdir(REF) else None
-PLUGINS = ("init", "update_sig", "compi")
+    """The reference tree if its plugins' sources are present on this machine, else None."""
+    return REF if all(os.path.isfile(os.path.join(REF, f"{name}.cu")) for name in PLUGINS) else None
 
 
 def build(ref: str = REF) -> list[str]:
