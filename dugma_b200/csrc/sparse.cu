@@ -159,22 +159,32 @@ static void reach_shares(const Context& c, double x, double* f, double* g)
     *g = std::max(uneven, *f);
 }
 
-static double sparse_time(const SparseCost& t, SparseUse use, double f, double g, double N, double M)
-{
-    auto block = [&](double h, double n, double m) {   // C(h)
-        const double r = 1.0 / t.e, p = std::pow(h, r), pn = std::pow(std::min(1.0, 32.0 / n), r),
-                     pm = std::pow(std::min(1.0, 32.0 / m), r);
-        const double F = std::min({1.0, t.u * h, std::pow(p + pn, t.e)});
+struct SparseTime {
+    const SparseCost& t;
+    const bool both_sides;
+    const double N, M, r, pn, pm;
+    SparseTime(const SparseCost& cost, SparseUse use, double n, double m)
+        : t(cost), both_sides(use == SparseUse::coef), N(n), M(m), r(1.0 / cost.e),
+          pn(std::pow(std::min(1.0, 32.0 / n), r)), pm(std::pow(std::min(1.0, 32.0 / m), r))
+    {
+    }
+    double block(double h, double p_st, double m) const   // C(h)
+    {
+        const double p = std::pow(h, r);
+        const double F = std::min({1.0, t.u * h, std::pow(p + p_st, t.e)});
         const double G = std::min(1.0, t.x * std::pow(p + pn + pm, t.e));
         return m * (F + t.y * G);
-    };
-    double all = N * block(f, N, M), one = t.b > 0 ? block(g, N, M) : 0.0;
-    if (use == SparseUse::coef) {
-        all += M * block(f, M, N);
-        one = std::max(one, block(g, M, N));
     }
-    return t.s0 + t.sn * (N + M) + std::hypot(t.a * all, t.b * one);
-}
+    double at(double f, double g) const
+    {
+        double all = N * block(f, pn, M), one = t.b > 0 ? block(g, pn, M) : 0.0;
+        if (both_sides) {
+            all += M * block(f, pm, N);
+            one = std::max(one, block(g, pm, N));
+        }
+        return t.s0 + t.sn * (N + M) + std::hypot(t.a * all, t.b * one);
+    }
+};
 
 double sparse_sigma(const Context& c, SparseUse use)
 {
@@ -187,17 +197,18 @@ double sparse_sigma(const Context& c, SparseUse use)
     if (line >= 0) return line;
     const SparseCost& t = sparse_cost(use, c.D);
     const double limit = t.margin * (t.t0 + t.tp * N * M + t.tn * (N + M));
+    const SparseTime time(t, use, N, M);
     auto sparse_at = [&](double x) {
         double f, g;
         reach_shares(c, x, &f, &g);
-        return sparse_time(t, use, f, g, N, M) < limit;
+        return time.at(f, g) < limit;
     };
     double lo = kReachExp - 127 + 1.0, hi = lo + kReachBins - 2.0;   // log2 of q; the time grows with it
     if (!sparse_at(lo)) return line = 0.0;
     if (sparse_at(hi)) {
         lo = hi;
     } else {
-        for (int k = 0; k < 18; ++k) {
+        for (int k = 0; k < 13; ++k) {   // (to 1 %)
             const double x = 0.5 * (lo + hi);
             (sparse_at(x) ? lo : hi) = x;
         }
