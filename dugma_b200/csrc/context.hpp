@@ -215,10 +215,10 @@ struct TimingHold {
 // The REF energy or adjoint over the pairs above the FP32 flush (sparse.cu), from the records of the
 // packed kernels' prologue: the same sums as the all-pairs kernel with tiles of tile_rec and chunks of
 // chunk_rec records.  go (nullable, device): nothing is done unless it is set.
-// Pairs from which a pass may be sparse where the device decides (both ways enqueued: the one that does not run
-// costs a dense EM step 2.5 us); the coefficients also where the host does, so that a call and an EM step go
-// the same way; and a batch's problems.
-constexpr double kSparseMinPairsAuto = 256e6, kSparseCoefMinPairs = 24e6, kSparseBatchMinPairs = 4e5;
+// Pairs from which a pass may be sparse (at 2000 x 2000 a gradient's best is 1 us of 36); where the device decides
+// (both ways enqueued: the one that does not run costs a dense EM step 2.5 us); the coefficients also where
+// the host does, so that a call and an EM step go the same way; a batch's problems.
+constexpr double kSparseMinPairs = 4e6, kSparseMinPairsAuto = 256e6, kSparseCoefMinPairs = 24e6, kSparseBatchMinPairs = 4e5;
 constexpr int kSparseMaxTargets = 1 << 20;
 constexpr int kRowBlocks = 256;
 int reduce_rows(Context& c, int nv, double* out_dev, cudaStream_t s, double* host_out, const int* go);

@@ -191,6 +191,7 @@ double sparse_sigma(const Context& c, SparseUse use)
     if (c.x_indef > 0 || c.y_indef > 0 || !c.ux || !c.xpt || c.no_alloc || c.all_pairs || c.M > kSparseMaxTargets)
         return 0.0;
     const double N = c.N, M = c.M;
+    if (use != SparseUse::batch && N * M < kSparseMinPairs) return 0.0;
     if (use == SparseUse::coef && (N * M < kSparseCoefMinPairs || c.N > kSparseMaxTargets)) return 0.0;
     if (use == SparseUse::batch && N * M < kSparseBatchMinPairs) return 0.0;
     double& line = c.sparse_line[(int)use];
